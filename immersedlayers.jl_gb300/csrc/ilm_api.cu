@@ -964,37 +964,26 @@ static int cached_schur(ilm_cache_s* c, int which, DevBuf& S64, DevBuf& S32, boo
 static int schur_cg(ilm_cache_s* c, const DevBuf& S64, const DevBuf& S32, const double* rhs, double* x, double tol,
                     int maxiter, ilm_solve_info_t* info, cudaStream_t st) {
   const int N = c->npts;
-  void* pb;
-  ILM_TRY(pscr(c, 7, &pb));
-  // layout in scratch 7: CGParams | iters (int) | relres (double)
-  unsigned char* base = static_cast<unsigned char*>(pb);
-  int* d_it = reinterpret_cast<int*>(base + 256);
-  double* d_rr = reinterpret_cast<double*>(base + 264);
-  if ((size_t)N * 4 * sizeof(double) < 512) {
-    ILM_TRY(c->p_scr[7].alloc(512));
-    base = static_cast<unsigned char*>(c->p_scr[7].p);
-    d_it = reinterpret_cast<int*>(base + 256);
-    d_rr = reinterpret_cast<double*>(base + 264);
-  }
-  CGParams P;
-  P.A64 = S64.as<double>();
-  P.A32 = nullptr;
+  ILM_TRY(c->p_scr[7].alloc(cg64_scratch_bytes(N)));
   (void)S32;
+  CG64Problem P;
+  P.A = S64.as<double>();
   P.b = rhs;
   P.x = x;
   P.w = c->ds64.as<double>();
   P.n = N;
   P.maxiter = maxiter;
   P.tol = tol;
-  P.iters = d_it;
-  P.relres = d_rr;
-  ILM_CHECK_CUDA(cudaMemcpyAsync(base, &P, sizeof(P), cudaMemcpyHostToDevice, st));
-  ILM_TRY(launch_cg_batched(reinterpret_cast<CGParams*>(base), 1, N, st));
-  int it = 0;
-  double rr = 0.0;
-  ILM_CHECK_CUDA(cudaMemcpyAsync(&it, d_it, sizeof(int), cudaMemcpyDeviceToHost, st));
-  ILM_CHECK_CUDA(cudaMemcpyAsync(&rr, d_rr, sizeof(double), cudaMemcpyDeviceToHost, st));
+  ILM_TRY(launch_cg64(P, c->p_scr[7].p, st));
+  CG64State res;
+  ILM_CHECK_CUDA(cudaMemcpyAsync(&res, c->p_scr[7].p, sizeof(res), cudaMemcpyDeviceToHost, st));
   ILM_CHECK_CUDA(cudaStreamSynchronize(st));
+  if (res.timeout) {
+    set_error("Schur CG: the wait for the other CTAs ran out");
+    return ILM_ERR_TIMEOUT;
+  }
+  const int it = res.iters;
+  const double rr = res.relres;
   if (info) {
     info->iterations = it;
     info->rel_residual = rr;

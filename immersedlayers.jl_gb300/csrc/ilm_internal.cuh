@@ -645,19 +645,38 @@ int schur_build(ilm_cache_s* c, int which, double scale, double* A, cudaStream_t
 // an FP64 cache of the same points as c (c itself when it is FP64), built on
 // first use and dropped when the points move
 int ensure_twin(ilm_cache_s* c, ilm_cache_s** out);
-struct CGParams {
-  const double* A64;   // n x n column-major
-  const float* A32;    // n x n column-major
-  const double* b;     // rhs
-  double* x;           // solution
-  const double* w;     // inner-product weights (ds)
-  int n;
-  int maxiter;
-  double tol;
-  int* iters;          // device out
-  double* relres;      // device out
+// FP64 CG of one problem (ilm_cg64.cu): S dense (A column-major) or CSR with
+// float-float values, in the w-weighted inner product (S = M diag(w), M
+// symmetric; w null: ones).  Converged when the true residual ||b - S x||_2
+// <= tol ||b||_2; it is formed when the recursive one says so, every
+// `refresh` iterations and at maxiter.  stall > 0: the best true-residual
+// iterate is kept and the solve stops after `stall` refreshes without gain.
+struct CG64Problem {
+  const double* A = nullptr;       // dense n x n, or
+  const int* rowptr = nullptr;     // CSR
+  const int* colidx = nullptr;
+  const float* vhi = nullptr;
+  const float* vlo = nullptr;
+  int max_row_nnz = 0;             // CSR: bound on a row's entries (sizes the shared-memory slab)
+  const double* b = nullptr;
+  const double* w = nullptr;
+  const double* x0 = nullptr;      // initial guess (may be x); null: zero
+  double* x = nullptr;
+  int n = 0, maxiter = 0, refresh = 100, stall = 0;
+  double tol = 0.0;
+  int* iters = nullptr;            // results (null: in the scratch's CG64State)
+  double* relres = nullptr;
 };
-int launch_cg_batched(const CGParams* probs_dev, int nprob, int max_n, cudaStream_t st);
+struct CG64State {                 // head of the scratch: results and the grid variant's barrier
+  int iters, timeout;
+  double relres;
+  unsigned arrived, pad;
+};
+size_t cg64_scratch_bytes(int n);
+bool cg64_fits(int n);  // the vectors of n unknowns fit a CTA's shared memory
+inline int cg64_csr_slab(const CG64Problem& P, int rows) { return P.max_row_nnz * rows; }
+// variant: 0 by size, 1 one cluster, 2 cooperative grid
+int launch_cg64(const CG64Problem& P, void* scratch, cudaStream_t st, int variant = 0);
 
 // batched Schur builds (one launch over all problems of a batch)
 // Row stride (floats) of a batched n x n Schur complement: n rounded up to a

@@ -17,9 +17,9 @@
 // O(N * P^2 log P), and gives the same matrix (up to FP64 rounding) provided
 // every stencil stays clear of the grid's ghost layer.
 //
-// The solve is CG in the ds-weighted inner product (the matrices are M*diag(w)
-// with M symmetric), one CTA per problem, in FP64: an FP32 matvec loses the
-// Krylov convergence on these ill-conditioned (cond ~ 1e4-1e5) and, for the
+// The solve (ilm_cg64.cu) is CG in the ds-weighted inner product (the matrices
+// are M*diag(w) with M symmetric) in FP64: an FP32 matvec loses the Krylov
+// convergence on these ill-conditioned (cond ~ 1e4-1e5) and, for the
 // Dirichlet problem, indefinite (one negative eigenvalue) systems.
 // Convergence is declared on the FP64 residual ||b - A x||_2 <= tol ||b||_2.
 #include <math.h>
@@ -245,135 +245,6 @@ int schur_build(ilm_cache_s* c, int which, double scale, double* A, cudaStream_t
   k_schur_pairs<<<grd, blk, 0, st>>>(N, F.as<Functional>(), W.as<double>(), G, ld, ld - 1, sgn, A);
   ILM_CHECK_LAUNCH();
   ILM_CHECK_CUDA(cudaStreamSynchronize(st));
-  return ILM_OK;
-}
-
-// ---------------------------------------------------------------------------
-// batched CG, one CTA per problem
-// ---------------------------------------------------------------------------
-constexpr int CG_THREADS = 512;
-
-__device__ double block_sum(double v, double* red) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  __syncthreads();
-  if (lane == 0) red[wid] = v;
-  __syncthreads();
-  double s = 0.0;
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) s += red[i];
-    red[32] = s;
-  }
-  __syncthreads();
-  return red[32];
-}
-
-// y = A x (A column-major n x n, FP64), rows distributed over the block
-__device__ __forceinline__ void gemv64(const double* __restrict__ A, const double* __restrict__ x,
-                                       double* __restrict__ y, int n) {
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const double* __restrict__ col = A + i;
-    double a0 = 0.0, a1 = 0.0;
-    int j = 0;
-    for (; j + 1 < n; j += 2) {
-      a0 = fma(__ldg(col + (size_t)j * n), x[j], a0);
-      a1 = fma(__ldg(col + (size_t)(j + 1) * n), x[j + 1], a1);
-    }
-    if (j < n) a0 = fma(__ldg(col + (size_t)j * n), x[j], a0);
-    y[i] = a0 + a1;
-  }
-}
-
-// CG in the w-weighted inner product (A = M diag(w), M symmetric), FP64.
-// The recursive residual decides when to check; convergence is declared on
-// the true residual ||b - A x||_2 <= tol ||b||_2, which is also recomputed
-// (and substituted) every 100 iterations.  Bounded by maxiter: no waits.
-__global__ void __launch_bounds__(CG_THREADS) k_cg(const CGParams* __restrict__ P) {
-  const CGParams pr = P[blockIdx.x];
-  const int n = pr.n;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  double* red = reinterpret_cast<double*>(smraw);  // 40 doubles
-  double* x = red + 40;
-  double* r = x + n;
-  double* p = r + n;
-  double* q = p + n;
-  double* w = q + n;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    x[i] = 0.0;
-    r[i] = pr.b[i];
-    p[i] = r[i];
-    w[i] = pr.w ? pr.w[i] : 1.0;
-  }
-  __syncthreads();
-  double bb = 0.0, rz = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    bb += r[i] * r[i];
-    rz += w[i] * r[i] * r[i];
-  }
-  bb = block_sum(bb, red);
-  rz = block_sum(rz, red);
-  const double bnorm = sqrt(bb);
-  const double thr = pr.tol * bnorm;
-  int it = 0;
-  double relres = bnorm > 0 ? 1.0 : 0.0;
-  bool done = bnorm == 0.0;
-  while (!done && it < pr.maxiter) {
-    gemv64(pr.A64, p, q, n);
-    __syncthreads();
-    double pq = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) pq += w[i] * p[i] * q[i];
-    pq = block_sum(pq, red);
-    if (pq == 0.0) break;
-    const double alpha = rz / pq;
-    double rr = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      x[i] += alpha * p[i];
-      r[i] -= alpha * q[i];
-      rr += r[i] * r[i];
-    }
-    rr = block_sum(rr, red);
-    ++it;
-    relres = bnorm > 0 ? sqrt(rr) / bnorm : 0.0;
-    if (sqrt(rr) <= thr || (it % 100) == 0 || it == pr.maxiter) {
-      gemv64(pr.A64, x, q, n);
-      __syncthreads();
-      double tr = 0.0;
-      for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        r[i] = pr.b[i] - q[i];
-        tr += r[i] * r[i];
-      }
-      tr = block_sum(tr, red);
-      relres = bnorm > 0 ? sqrt(tr) / bnorm : 0.0;
-      if (sqrt(tr) <= thr) {
-        done = true;
-        break;
-      }
-    }
-    double rzn = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) rzn += w[i] * r[i] * r[i];
-    rzn = block_sum(rzn, red);
-    const double beta = rzn / rz;
-    rz = rzn;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) p[i] = r[i] + beta * p[i];
-    __syncthreads();
-  }
-  for (int i = threadIdx.x; i < n; i += blockDim.x) pr.x[i] = x[i];
-  if (threadIdx.x == 0) {
-    if (pr.iters) *pr.iters = it;
-    if (pr.relres) *pr.relres = relres;
-  }
-}
-
-int launch_cg_batched(const CGParams* probs_dev, int nprob, int max_n, cudaStream_t st) {
-  const size_t smem = 40 * sizeof(double) + (size_t)max_n * 5 * sizeof(double) + 64;
-  if (smem > 227 * 1024) {
-    set_error("CG: problem of %d unknowns exceeds the shared-memory solver", max_n);
-    return ILM_ERR_SIZE_LIMIT;
-  }
-  ILM_CHECK_CUDA(cudaFuncSetAttribute(k_cg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k_cg<<<nprob, CG_THREADS, smem, st>>>(probs_dev);
-  ILM_CHECK_LAUNCH();
   return ILM_OK;
 }
 
