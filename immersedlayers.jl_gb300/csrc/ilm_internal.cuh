@@ -311,12 +311,28 @@ int fill_zero(void* out, size_t bytes, cudaStream_t st);
 // ---------------------------------------------------------------------------
 // FFT convolution (inverse Laplacian)
 // ---------------------------------------------------------------------------
+// Sine-transform solver of one field size (ilm_sine.cu)
+struct SinePlan {
+  int n1 = 0, n2 = 0, N = 0, MB = 0, L = 0, ldg = 0;
+  const void* tw = nullptr;      // twiddles of length 2 N
+  const double* tab = nullptr;   // per-mode constants (shared, library-owned)
+  const double* s2 = nullptr;    // 2 sin(pi m / N), 0 <= m < 2 N
+  const double* lgf = nullptr;   // G(m, n), row stride ldg (shared, library-owned)
+  DevBuf work;                   // modes (n2 x N) and the ring's sources and potentials
+};
+bool sine_supported(int n1, int n2);
+int sine_plan_init(SinePlan* p, int n1, int n2, const void* tw, cudaStream_t st);
+// out = inv_factor * G * in, FP64, in and out n1 x n2 (x fastest, may alias)
+int sine_apply(SinePlan* p, const double* in, double* out, double inv_factor, cudaStream_t st);
+
 struct ConvPlan {
   int n1 = 0, n2 = 0, P1 = 0, P2 = 0, dtype = ILM_F64;
   const void* spec = nullptr;   // (P1/2+1) x (P2/2+1) real, scaled, device (shared)
   const void* tw1 = nullptr;    // twiddles length P1 (device, shared)
   const void* tw2 = nullptr;    // twiddles length P2
   DevBuf work;                  // n2 x (P1/2+1) complex
+  bool use_sine = false;        // FP64 fields: the sine-transform solver instead
+  SinePlan sine;
 };
 
 struct ConvJobDev {
@@ -387,11 +403,18 @@ __device__ __forceinline__ void pdl_begin() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
+// The wait alone: the next launch is scheduled when this grid is done.  For
+// kernels bound by FP64 issue or latency, whose next grid's waiting CTAs only
+// take room (the six launches of an FP64 inverse Laplacian of 405^2: 148 us
+// with launch_dependents at their start, 105 us without programmatic launch,
+// 91 us with the wait alone).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <typename... P, typename... A>
-cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, A... args) {
+cudaError_t launch_pdl_smem(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -399,6 +422,10 @@ cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t
   cfg.attrs = at;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+template <typename... P, typename... A>
+cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, A... args) {
+  return launch_pdl_smem(kernel, grid, block, 0, st, args...);
 }
 
 struct FF {
