@@ -94,11 +94,6 @@ struct CGFFParams {
   const int* boff;     // offset of each block's inverse (row-major bsize^2)
   const float* binv_hi;  // block inverses as float-float pairs
   const float* binv_lo;
-  // optional sparse matrix (CSR over rows; Shi/Slo hold the nnz values)
-  const int* rowptr;
-  const int* colidx;
-  // optional initial guess (warm start)
-  const double* x0;
   // optional learned banded preconditioner M r = W^-1 C^T C r: C has
   // 2 band_k + 1 coefficients per row (row-major), circular within each
   // body; seg_start / seg_len give each point's body (local indices)
@@ -140,35 +135,6 @@ __device__ __forceinline__ unsigned sm_id() {
   unsigned r;
   asm volatile("mov.u32 %0, %%smid;" : "=r"(r));
   return r;
-}
-
-// y[i - r0] = (S v)_i for a CSR matrix (float-float values), one warp per row
-__device__ void ff_spmv_rows(const CGFFParams& pr, int r0, int r1, const float* __restrict__ vhi,
-                             const float* __restrict__ vlo, double* __restrict__ y) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int i = r0 + warp; i < r1; i += CGC_WARPS) {
-    const int e0 = pr.rowptr[i], e1 = pr.rowptr[i + 1];
-    FF a0{0.f, 0.f}, a1{0.f, 0.f};
-    int e = e0 + lane;
-    for (; e + 32 < e1; e += 64) {
-      const int c0 = __ldg(pr.colidx + e), c1 = __ldg(pr.colidx + e + 32);
-      ff_fma(a0, __ldg(pr.Shi + e), __ldg(pr.Slo + e), vhi[c0], vlo[c0]);
-      ff_fma(a1, __ldg(pr.Shi + e + 32), __ldg(pr.Slo + e + 32), vhi[c1], vlo[c1]);
-    }
-    if (e < e1) {
-      const int c0 = __ldg(pr.colidx + e);
-      ff_fma(a0, __ldg(pr.Shi + e), __ldg(pr.Slo + e), vhi[c0], vlo[c0]);
-    }
-    FF acc = ff_add(a0, a1);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      FF other;
-      other.hi = __shfl_down_sync(0xffffffffu, acc.hi, o);
-      other.lo = __shfl_down_sync(0xffffffffu, acc.lo, o);
-      acc = ff_add(acc, other);
-    }
-    if (lane == 0) y[i - r0] = (double)acc.hi + (double)acc.lo;
-  }
 }
 
 // z[i - r0] = (M r)_i for rows i in [r0, r1): float-float block-Jacobi (the
@@ -272,8 +238,7 @@ __device__ void ff_gemv_rows_v4(const float* __restrict__ Shi, const float* __re
 // rows [r0, r1) of S v into y (full-length indexing)
 __device__ __forceinline__ void matvec_rows_full(const CGFFParams& pr, int n, int r0, int r1, const float* vhi,
                                                  const float* vlo, double* y) {
-  if (pr.rowptr) ff_spmv_rows(pr, r0, r1, vhi, vlo, y + r0);
-  else ff_gemv_rows_v4(pr.Shi, pr.Slo, n, r0, r1, vhi, vlo, y);
+  ff_gemv_rows_v4(pr.Shi, pr.Slo, n, r0, r1, vhi, vlo, y);
 }
 
 // neighbour of point j at band offset t within its body [s, s + L) (circular)
@@ -415,18 +380,11 @@ __global__ void __cluster_dims__(CG_CLUSTER, 1, 1) __launch_bounds__(CGR_THREADS
     const int rows = (n + CG_CLUSTER - 1) / CG_CLUSTER;
     const int r0 = min(n, rank * rows), r1 = min(n, r0 + rows);
     for (int j = threadIdx.x; j < n; j += blockDim.x) {
-      x[j] = pr.x0 ? pr.x0[j] : 0.0;
+      x[j] = 0.0;
       w[j] = pr.w ? pr.w[j] : 1.0;
     }
     __syncthreads();
-    if (pr.x0) {  // warm start: r = b - S x0
-      split_full(x, n, ld, S.vhi, S.vlo);
-      __syncthreads();
-      const double* t = exchange_matvec(cl, pr, S, xsel, n, rows, rank, r0, r1);
-      for (int j = threadIdx.x; j < n; j += blockDim.x) r[j] = pr.b[j] - t[j];
-    } else {
-      for (int j = threadIdx.x; j < n; j += blockDim.x) r[j] = pr.b[j];
-    }
+    for (int j = threadIdx.x; j < n; j += blockDim.x) r[j] = pr.b[j];
     __syncthreads();
     const double* sz = pr.sz;  // deflation (as k_cg_cluster): S 1, whole vector
     const double inv_e = sz ? __ldg(pr.inv_e) : 0.0;
@@ -575,33 +533,11 @@ __global__ void __cluster_dims__(CG_CLUSTER, 1, 1) __launch_bounds__(CGR_THREADS
 // may still be copying.
 // ---------------------------------------------------------------------------
 
-// rows [r0, r1) of S v as float-float pairs yh/yl[i - r0] (dense rows with
-// 16-byte alignment, or CSR)
+// rows [r0, r1) of S v as float-float pairs yh/yl[i - r0] (rows with 16-byte
+// alignment)
 __device__ void matvec_rows_ff(const CGFFParams& pr, int n, int r0, int r1, const float* __restrict__ vhi,
                                const float* __restrict__ vlo, float* __restrict__ yh, float* __restrict__ yl) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  if (pr.rowptr) {
-    for (int i = r0 + warp; i < r1; i += nwarps) {
-      const int e0 = pr.rowptr[i], e1 = pr.rowptr[i + 1];
-      FF a{0.f, 0.f};
-      for (int e = e0 + lane; e < e1; e += 32) {
-        const int c = __ldg(pr.colidx + e);
-        ff_fma(a, __ldg(pr.Shi + e), __ldg(pr.Slo + e), vhi[c], vlo[c]);
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        FF oa;
-        oa.hi = __shfl_down_sync(0xffffffffu, a.hi, o);
-        oa.lo = __shfl_down_sync(0xffffffffu, a.lo, o);
-        a = ff_add(a, oa);
-      }
-      if (lane == 0) {
-        yh[i - r0] = a.hi;
-        yl[i - r0] = a.lo;
-      }
-    }
-    return;
-  }
   const int ld = schur_ld(n), nq = ld >> 2;
   const float4* vh4 = reinterpret_cast<const float4*>(vhi);
   const float4* vl4 = reinterpret_cast<const float4*>(vlo);
@@ -987,7 +923,7 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(NT, MINB)
     // 1 / E (deflation) is read by thread 0 where it forms the scalars
     const bool pre = pr.blk != nullptr || pr.band != nullptr;
     for (int i = threadIdx.x; i < nr; i += blockDim.x) {
-      xs[i] = pr.x0 ? pr.x0[r0 + i] : 0.0;
+      xs[i] = 0.0;
       bs[i] = pr.b[r0 + i];
       ws[i] = pr.w ? pr.w[r0 + i] : 1.0;
     }
@@ -995,19 +931,8 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(NT, MINB)
       ph[j] = pl[j] = bh[j] = bl[j] = 0.f;
     }
     __syncthreads();
-    if (pr.x0) {  // warm start: r = b - S x0 (x through buffer B)
-      double v[1] = {0.0};
-      publish_slice(xs, r0, nr, bh, bl);
-      csum_t0<1, CS>(cl, v, nr, red, pub, slot);  // the barrier that publishes x
-      gather_parts(cl, bh, bl, n, rows, rank);
-      matvec_rows_ff(pr, n, r0, r1, bh, bl, yh, yl);
-      __syncthreads();
-      for (int i = threadIdx.x; i < nr; i += blockDim.x) rs[i] = bs[i] - ((double)yh[i] + (double)yl[i]);
-      __syncthreads();
-    } else {
-      for (int i = threadIdx.x; i < nr; i += blockDim.x) rs[i] = bs[i];
-      __syncthreads();
-    }
+    for (int i = threadIdx.x; i < nr; i += blockDim.x) rs[i] = bs[i];
+    __syncthreads();
     if (sz) {  // deflation: x += c 1, r -= c S 1, c = 1^T W r / E (then 1^T W r = 0)
       double v[1] = {0.0};
       for (int i = threadIdx.x; i < nr; i += blockDim.x) v[0] += ws[i] * rs[i];
@@ -1405,14 +1330,6 @@ void cgff_params_fill(void* dst, const float* Shi, const float* Slo, const doubl
   *static_cast<CGFFParams*>(dst) = p;
 }
 
-void cgff_params_fill_csr(void* dst, const float* vhi, const float* vlo, const int* rowptr, const int* colidx,
-                          const double* b, double* x, const double* x0, const double* w, int n, int maxiter,
-                          double tol, int* iters, double* relres) {
-  CGFFParams p{vhi, vlo, b, x, w, n, maxiter, tol, iters, relres,
-               nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, rowptr, colidx, x0};
-  *static_cast<CGFFParams*>(dst) = p;
-}
-
 void cgff_params_set_deflation(void* dst, const double* sz, const double* inv_e) {
   CGFFParams* p = static_cast<CGFFParams*>(dst);
   p->sz = sz;
@@ -1422,8 +1339,6 @@ void cgff_params_set_deflation(void* dst, const double* sz, const double* inv_e)
 void cgff_params_set_timing(void* dst, unsigned long long* tspan) {
   static_cast<CGFFParams*>(dst)->tspan = tspan;
 }
-
-void cgff_params_set_x0(void* dst, const double* x0) { static_cast<CGFFParams*>(dst)->x0 = x0; }
 
 void cgff_params_set_coarse(void* dst, int nb, const int* starts, const double* Einv) {
   CGFFParams* p = static_cast<CGFFParams*>(dst);

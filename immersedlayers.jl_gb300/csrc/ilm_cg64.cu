@@ -116,7 +116,6 @@ __global__ void __launch_bounds__(C64_T, 1) k_cg64(const CG64Args A) {
   unsigned bar = 0;      // grid barriers passed
   bool ok = true;
 
-  if (!GRID && rank == 0 && t == 0) A.state->timeout = 0;
   int e0 = 0;
   if (CSR) e0 = P.rowptr[r0];
   if (A.resident) {
@@ -215,7 +214,7 @@ __global__ void __launch_bounds__(C64_T, 1) k_cg64(const CG64Args A) {
           asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&A.state->arrived) : "memory");
         } while (seen < goal && ++k < C64_SPIN);
         s_ok = seen >= goal;
-        if (seen < goal) atomicExch(&A.state->timeout, 1);
+        if (seen < goal) atomicExch(P.timeout, 1);
       }
       __syncthreads();
       ok = s_ok != 0;
@@ -427,6 +426,8 @@ int launch_cg64(const CG64Problem& P, void* scratch, cudaStream_t st, int varian
   A.gq = reinterpret_cast<double*>(A.state + 1);
   if (!A.p.iters) A.p.iters = &A.state->iters;
   if (!A.p.relres) A.p.relres = &A.state->relres;
+  ILM_CHECK_CUDA(cudaMemsetAsync(A.state, 0, sizeof(CG64State), st));
+  if (!A.p.timeout) A.p.timeout = &A.state->timeout;
   const long long entries = (long long)n * (csr ? std::min(P.max_row_nnz, n) : n);
   size_t smem = plan(P, false, C64_CLUSTER, &A);
   if ((variant == 1 || (variant == 0 && entries <= C64_CLUSTER_ENTRIES)) && smem <= (size_t)C64_MAX_SMEM &&
@@ -441,7 +442,6 @@ int launch_cg64(const CG64Problem& P, void* scratch, cudaStream_t st, int varian
   }
   smem = plan(P, true, std::min(sms, n), &A);
   ILM_CHECK_CUDA((csr ? kernel_attributes<true, true>() : kernel_attributes<false, true>()));
-  ILM_CHECK_CUDA(cudaMemsetAsync(A.state, 0, sizeof(CG64State), st));
   const int G = (n + A.R - 1) / A.R;
   return csr ? run_grid<true>(A, G, smem, st) : run_grid<false>(A, G, smem, st);
 }

@@ -162,6 +162,8 @@ __global__ void k_heat_combine(size_t n, const T* __restrict__ a, double cb, con
 
 using namespace ilm;
 
+constexpr int HEAT_MAX_POINTS = 4688;  // unknowns of a stage solve
+
 struct ilm_heat_s {
   ilm_cache_s* c = nullptr;
   double kappa = 1.0, dt = 0.0;
@@ -181,7 +183,8 @@ struct ilm_heat_s {
   DevBuf e[4], avg64, cfield;
   DevBuf g1, g3, rhs, q1, q2, sig[3], sig_t;
   DevBuf tmp[4];
-  DevBuf cgp, order, counter, iters, relres;
+  DevBuf cgs, iters, relres;
+  int max_row[4] = {0, 0, 0, 0};  // most entries of a row
   long long total_iters = 0;
   int last_iters[3] = {0, 0, 0};
 };
@@ -270,6 +273,7 @@ int build_sparse_schur(ilm_heat_s* H, const std::vector<double>& taps, int slot)
     rp[k + 1] = (int)ci.size();
   }
   H->nnz[slot] = ci.size();
+  for (int k = 0; k < N; ++k) H->max_row[slot] = std::max(H->max_row[slot], rp[k + 1] - rp[k]);
   ILM_TRY(upd(H->rowptr[slot], rp.data(), rp.size() * sizeof(int)));
   ILM_TRY(upd(H->colidx[slot], ci.data(), ci.size() * sizeof(int)));
   ILM_TRY(upd(H->vhi[slot], vh.data(), vh.size() * sizeof(float)));
@@ -303,10 +307,34 @@ int build_gather_windows(ilm_heat_s* H, const std::vector<double>& taps, int set
   return ILM_OK;
 }
 
-int run_cg(ilm_heat_s* H, int which_params, cudaStream_t st) {
-  ILM_TRY(launch_cg_cluster(static_cast<unsigned char*>(H->cgp.p) + (size_t)which_params * cgff_params_size(),
-                            H->order.as<int>(), 1, H->counter.as<int>() + which_params, H->c->npts, 1, st));
-  return ILM_OK;
+// S sigma = rhs of stage s (0: a/3, 1: 2a/3, 2: the final update), from the
+// last step's sigma
+int run_cg(ilm_heat_s* H, int s, cudaStream_t st) {
+  constexpr int slot[3] = {0, 1, 3};
+  const int m = slot[s], N = H->c->npts;
+  if (N > HEAT_MAX_POINTS) {
+    set_error("heat: %d points exceed the stage solver's limit of %d", N, HEAT_MAX_POINTS);
+    return ILM_ERR_SIZE_LIMIT;
+  }
+  CG64Problem P;
+  P.rowptr = H->rowptr[m].as<int>();
+  P.colidx = H->colidx[m].as<int>();
+  P.vhi = H->vhi[m].as<float>();
+  P.vlo = H->vlo[m].as<float>();
+  P.max_row_nnz = H->max_row[m];
+  P.b = H->rhs.as<double>() + (size_t)s * N;
+  P.w = H->c->ds64.as<double>();
+  P.x = H->sig[s].as<double>();
+  P.x0 = H->sig[s].as<double>();
+  P.n = N;
+  P.maxiter = H->maxiter;
+  P.tol = H->tol;
+  P.refresh = 50;
+  P.stall = 8;
+  P.iters = H->iters.as<int>() + s;
+  P.relres = H->relres.as<double>() + s;
+  P.timeout = H->iters.as<int>() + 3;
+  return launch_cg64(P, H->cgs.p, st);
 }
 
 }  // namespace
@@ -393,21 +421,10 @@ int ilm_heat_create(ilm_cache_t c, double kappa, double dt, const double* tb_plu
     ILM_CHECK_CUDA(cudaMemset(H->sig[s].p, 0, (size_t)N * 8));
   }
   ILM_TRY(H->sig_t.alloc((size_t)N * es));
-  ILM_TRY(H->iters.alloc(3 * sizeof(int)));
+  ILM_TRY(H->iters.alloc(4 * sizeof(int)));  // and the solver's time-out flag
+  ILM_CHECK_CUDA(cudaMemset(H->iters.p, 0, 4 * sizeof(int)));
   ILM_TRY(H->relres.alloc(3 * sizeof(double)));
-  ILM_TRY(H->counter.alloc(3 * sizeof(int)));
-  int zero = 0;
-  ILM_TRY(upd(H->order, &zero, sizeof(int)));
-  std::vector<unsigned char> prm(3 * cgff_params_size());
-  const int mslot[3] = {0, 1, 3};
-  for (int s = 0; s < 3; ++s) {
-    cgff_params_fill_csr(prm.data() + s * cgff_params_size(), H->vhi[mslot[s]].as<float>(),
-                         H->vlo[mslot[s]].as<float>(), H->rowptr[mslot[s]].as<int>(), H->colidx[mslot[s]].as<int>(),
-                         H->rhs.as<double>() + (size_t)s * N, H->sig[s].as<double>(), H->sig[s].as<double>(),
-                         c->ds64.as<double>(), N, maxiter, tol, H->iters.as<int>() + s,
-                         H->relres.as<double>() + s);
-  }
-  ILM_TRY(upd(H->cgp, prm.data(), prm.size()));
+  ILM_TRY(H->cgs.alloc(cg64_scratch_bytes(N)));
   ILM_CHECK_CUDA(cudaDeviceSynchronize());
   *out = guard.release();
   return ILM_OK;
@@ -489,9 +506,14 @@ int ilm_heat_advance(ilm_heat_t H, void* T, void* sigma_out, int nsteps, ilm_str
     ILM_TRY(st_affine(N, c->dtype, -1.0, sigma_out, 0.0, sigma_out, st));
   }
   if (nsteps > 0) {
-    int it[3];
-    ILM_CHECK_CUDA(cudaMemcpyAsync(it, H->iters.p, 3 * sizeof(int), cudaMemcpyDeviceToHost, st));
+    int it[4];
+    ILM_CHECK_CUDA(cudaMemcpyAsync(it, H->iters.p, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
     ILM_CHECK_CUDA(cudaStreamSynchronize(st));
+    if (it[3]) {
+      ILM_CHECK_CUDA(cudaMemset(H->iters.as<int>() + 3, 0, sizeof(int)));
+      set_error("heat: a stage solve's wait for the other CTAs ran out");
+      return ILM_ERR_TIMEOUT;
+    }
     for (int s = 0; s < 3; ++s) H->last_iters[s] = it[s];
   }
   return ILM_OK;
