@@ -949,23 +949,37 @@ int ilm_schur_build(ilm_cache_t c, int which, double scale, double* A_dev, ilm_s
 
 namespace ilm {
 
-// S (FP64 and FP32 copies) cached in the cache
-static int cached_schur(ilm_cache_s* c, int which, DevBuf& S64, DevBuf& S32, bool& ready, cudaStream_t st) {
+// S of problem `which` (and the FP32 inverse its solves refine), kept until
+// the points move
+static int cached_schur(ilm_cache_s* c, int which, cudaStream_t st) {
+  const bool dir = which == ILM_SCHUR_RTLINVR;
+  bool& ready = dir ? c->S_dir_ready : c->S_neu_ready;
   if (ready) return ILM_OK;
+  DevBuf& S64 = dir ? c->S_dir64 : c->S_neu64;
   const size_t nn = (size_t)c->npts * c->npts;
-  (void)S32;
   ILM_TRY(S64.alloc(std::max<size_t>(nn, 1) * sizeof(double)));
   ILM_TRY(schur_build(c, which, 1.0, S64.as<double>(), st));
+  CG64Inverse& inv = dir ? c->inv_dir : c->inv_neu;
+  inv.ready = false;
+  if (cg64_fits(c->npts)) {
+    CG64Problem P;
+    P.A = S64.as<double>();
+    P.w = c->ds64.as<double>();
+    P.n = c->npts;
+    ILM_TRY(cg64_inverse(&inv, P, st));
+  }
   ready = true;
   return ILM_OK;
 }
 
-// Solve S x = rhs (rhs, x FP64 device) by CG on the device.
-static int schur_cg(ilm_cache_s* c, const DevBuf& S64, const DevBuf& S32, const double* rhs, double* x, double tol,
-                    int maxiter, ilm_solve_info_t* info, cudaStream_t st) {
+// Solve S x = rhs (rhs, x FP64 device) on the device, S of problem `which`.
+static int schur_cg(ilm_cache_s* c, int which, const double* rhs, double* x, double tol, int maxiter,
+                    ilm_solve_info_t* info, cudaStream_t st) {
+  const bool dir = which == ILM_SCHUR_RTLINVR;
+  const DevBuf& S64 = dir ? c->S_dir64 : c->S_neu64;
+  const CG64Inverse& inv = dir ? c->inv_dir : c->inv_neu;
   const int N = c->npts;
   ILM_TRY(c->p_scr[7].alloc(cg64_scratch_bytes(N)));
-  (void)S32;
   CG64Problem P;
   P.A = S64.as<double>();
   P.b = rhs;
@@ -974,6 +988,7 @@ static int schur_cg(ilm_cache_s* c, const DevBuf& S64, const DevBuf& S32, const 
   P.n = N;
   P.maxiter = maxiter;
   P.tol = tol;
+  if (inv.ready) inv.attach(&P);
   ILM_TRY(launch_cg64(P, c->p_scr[7].p, st));
   CG64State res;
   ILM_CHECK_CUDA(cudaMemcpyAsync(&res, c->p_scr[7].p, sizeof(res), cudaMemcpyDeviceToHost, st));
@@ -1033,8 +1048,8 @@ int ilm_solve_dirichlet(ilm_cache_t c, const void* fplus, const void* fminus, vo
   ILM_TRY(launch_gather(c, &t, 1, g, false, 1.0, st));
   ILM_TRY(st_axpby(N, c->dtype, 1.0, g, -1.0, avg, g, st));
   ILM_TRY(st_convert(N, c->dtype, g, ILM_F64, rhs64, st));
-  ILM_TRY(cached_schur(c, ILM_SCHUR_RTLINVR, c->S_dir64, c->S_dir32, c->S_dir_ready, st));
-  const int cg = schur_cg(c, c->S_dir64, c->S_dir32, static_cast<double*>(rhs64), static_cast<double*>(x64), tol,
+  ILM_TRY(cached_schur(c, ILM_SCHUR_RTLINVR, st));
+  const int cg = schur_cg(c, ILM_SCHUR_RTLINVR, static_cast<double*>(rhs64), static_cast<double*>(x64), tol,
                           maxiter, info, st);
   if (cg != ILM_OK && cg != ILM_ERR_NOT_CONVERGED) return cg;
   ILM_TRY(st_convert(N, ILM_F64, x64, c->dtype, s_out, st));
@@ -1084,8 +1099,8 @@ int ilm_solve_neumann_full(ilm_cache_t c, const void* vplus, const void* vminus,
   ILM_TRY(ilm_surface_grad(c, fstar, g, stream));
   ILM_TRY(st_axpby(N, c->dtype, 1.0, g, -1.0, avg, g, st));
   ILM_TRY(st_convert(N, c->dtype, g, ILM_F64, rhs64, st));
-  ILM_TRY(cached_schur(c, ILM_SCHUR_CLINVCT, c->S_neu64, c->S_neu32, c->S_neu_ready, st));
-  const int cg = schur_cg(c, c->S_neu64, c->S_neu32, static_cast<double*>(rhs64), static_cast<double*>(x64), tol,
+  ILM_TRY(cached_schur(c, ILM_SCHUR_CLINVCT, st));
+  const int cg = schur_cg(c, ILM_SCHUR_CLINVCT, static_cast<double*>(rhs64), static_cast<double*>(x64), tol,
                           maxiter, info, st);
   if (cg != ILM_OK && cg != ILM_ERR_NOT_CONVERGED) return cg;
   ILM_TRY(st_convert(N, ILM_F64, x64, c->dtype, df_out, st));
@@ -1098,7 +1113,7 @@ int ilm_solve_neumann_full(ilm_cache_t c, const void* vplus, const void* vminus,
   ilm_solve_info_t info2{0, 1, 0.0};
   ILM_TRY(ilm_surface_grad_cross(c, fstar, g, stream));
   ILM_TRY(st_convert(N, c->dtype, g, ILM_F64, rhs64, st));
-  const int cg2 = schur_cg(c, c->S_neu64, c->S_neu32, static_cast<double*>(rhs64), static_cast<double*>(x64), tol,
+  const int cg2 = schur_cg(c, ILM_SCHUR_CLINVCT, static_cast<double*>(rhs64), static_cast<double*>(x64), tol,
                            maxiter, &info2, st);
   if (cg2 != ILM_OK && cg2 != ILM_ERR_NOT_CONVERGED) return cg2;
   ILM_TRY(st_convert(N, ILM_F64, x64, c->dtype, ds_out, st));
@@ -1246,9 +1261,9 @@ static int solve_refined(ilm_cache_s* c, bool neumann, const double* fplus, cons
   // the FP64 Schur complement (the same pair sums for every dtype)
   DevBuf& S64 = neumann ? c->S_neu64 : c->S_dir64;
   if (neumann)
-    ILM_TRY(cached_schur(c, ILM_SCHUR_CLINVCT, c->S_neu64, c->S_neu32, c->S_neu_ready, st));
+    ILM_TRY(cached_schur(c, ILM_SCHUR_CLINVCT, st));
   else
-    ILM_TRY(cached_schur(c, ILM_SCHUR_RTLINVR, c->S_dir64, c->S_dir32, c->S_dir_ready, st));
+    ILM_TRY(cached_schur(c, ILM_SCHUR_RTLINVR, st));
   double rel = 0.0;
   for (int k = 0;; ++k) {
     k_dense_matvec64<<<(N + 127) / 128, 128, 0, st>>>(N, S64.as<double>(), c->ref_x.as<double>(),
@@ -1264,8 +1279,8 @@ static int solve_refined(ilm_cache_s* c, bool neumann, const double* fplus, cons
     if (rel <= tol || k >= max_refine) break;
     // correction: S d = r by the FP64 CG, x += d
     ilm_solve_info_t ci{0, 0, 0.0};
-    const int rc = schur_cg(c, S64, S64, c->ref_r.as<double>(), c->ref_y.as<double>(), kRefineInnerTol, maxiter, &ci,
-                            st);
+    const int rc = schur_cg(c, neumann ? ILM_SCHUR_CLINVCT : ILM_SCHUR_RTLINVR, c->ref_r.as<double>(),
+                            c->ref_y.as<double>(), kRefineInnerTol, maxiter, &ci, st);
     if (rc != ILM_OK && rc != ILM_ERR_NOT_CONVERGED) return rc;
     total_its += ci.iterations;
     ILM_TRY(st_axpby(N, ILM_F64, 1.0, c->ref_x.p, 1.0, c->ref_y.p, c->ref_x.p, st));

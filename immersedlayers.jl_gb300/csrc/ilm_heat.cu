@@ -184,6 +184,7 @@ struct ilm_heat_s {
   DevBuf g1, g3, rhs, q1, q2, sig[3], sig_t;
   DevBuf tmp[4];
   DevBuf cgs, iters, relres;
+  CG64Inverse inv[3];             // FP32 inverses of the three stage systems
   int max_row[4] = {0, 0, 0, 0};  // most entries of a row
   long long total_iters = 0;
   int last_iters[3] = {0, 0, 0};
@@ -307,33 +308,39 @@ int build_gather_windows(ilm_heat_s* H, const std::vector<double>& taps, int set
   return ILM_OK;
 }
 
-// S sigma = rhs of stage s (0: a/3, 1: 2a/3, 2: the final update), from the
-// last step's sigma
-int run_cg(ilm_heat_s* H, int s, cudaStream_t st) {
+// the system S sigma = rhs of stage s (0: a/3, 1: 2a/3, 2: the final update)
+CG64Problem stage_problem(ilm_heat_s* H, int s) {
   constexpr int slot[3] = {0, 1, 3};
   const int m = slot[s], N = H->c->npts;
-  if (N > HEAT_MAX_POINTS) {
-    set_error("heat: %d points exceed the stage solver's limit of %d", N, HEAT_MAX_POINTS);
-    return ILM_ERR_SIZE_LIMIT;
-  }
   CG64Problem P;
   P.rowptr = H->rowptr[m].as<int>();
   P.colidx = H->colidx[m].as<int>();
   P.vhi = H->vhi[m].as<float>();
   P.vlo = H->vlo[m].as<float>();
   P.max_row_nnz = H->max_row[m];
-  P.b = H->rhs.as<double>() + (size_t)s * N;
   P.w = H->c->ds64.as<double>();
-  P.x = H->sig[s].as<double>();
-  P.x0 = H->sig[s].as<double>();
   P.n = N;
   P.maxiter = H->maxiter;
   P.tol = H->tol;
   P.refresh = 50;
   P.stall = 8;
+  return P;
+}
+
+// from the last step's sigma
+int run_cg(ilm_heat_s* H, int s, cudaStream_t st) {
+  CG64Problem P = stage_problem(H, s);
+  if (P.n > HEAT_MAX_POINTS) {
+    set_error("heat: %d points exceed the stage solver's limit of %d", P.n, HEAT_MAX_POINTS);
+    return ILM_ERR_SIZE_LIMIT;
+  }
+  P.b = H->rhs.as<double>() + (size_t)s * P.n;
+  P.x = H->sig[s].as<double>();
+  P.x0 = H->sig[s].as<double>();
   P.iters = H->iters.as<int>() + s;
   P.relres = H->relres.as<double>() + s;
   P.timeout = H->iters.as<int>() + 3;
+  if (H->inv[s].ready) H->inv[s].attach(&P);
   return launch_cg64(P, H->cgs.p, st);
 }
 
@@ -425,6 +432,8 @@ int ilm_heat_create(ilm_cache_t c, double kappa, double dt, const double* tb_plu
   ILM_CHECK_CUDA(cudaMemset(H->iters.p, 0, 4 * sizeof(int)));
   ILM_TRY(H->relres.alloc(3 * sizeof(double)));
   ILM_TRY(H->cgs.alloc(cg64_scratch_bytes(N)));
+  if (N <= HEAT_MAX_POINTS)
+    for (int s = 0; s < 3; ++s) ILM_TRY(cg64_inverse(&H->inv[s], stage_problem(H, s), nullptr));
   ILM_CHECK_CUDA(cudaDeviceSynchronize());
   *out = guard.release();
   return ILM_OK;

@@ -486,6 +486,59 @@ struct GatherTerm {
   int coef;           // Coef code
 };
 
+// FP64 CG of one problem (ilm_cg64.cu): S dense (A column-major) or CSR with
+// float-float values, in the w-weighted inner product (S = M diag(w), M
+// symmetric; w null: ones).  Converged when the true residual ||b - S x||_2
+// <= tol ||b||_2; it is formed when the recursive one says so, every
+// `refresh` iterations and at maxiter.  stall > 0: the best true-residual
+// iterate is kept and the solve stops after `stall` refreshes without gain.
+struct CG64Problem {
+  const double* A = nullptr;       // dense n x n, or
+  const int* rowptr = nullptr;     // CSR
+  const int* colidx = nullptr;
+  const float* vhi = nullptr;
+  const float* vlo = nullptr;
+  int max_row_nnz = 0;             // CSR: bound on a row's entries (sizes the shared-memory slab)
+  const double* b = nullptr;
+  const double* w = nullptr;
+  const double* x0 = nullptr;      // initial guess (may be x); null: zero
+  double* x = nullptr;
+  int n = 0, maxiter = 0, refresh = 100, stall = 0;
+  double tol = 0.0;
+  int* iters = nullptr;            // results (null: in the scratch's CG64State)
+  double* relres = nullptr;
+  int* timeout = nullptr;          // set to 1 if the grid variant's wait ran out (null: in CG64State)
+  // optional FP32 inverse of W S (cg64_inverse): refined with FP64 residuals
+  // before, and usually instead of, the CG
+  const float* inv = nullptr;      // row stride ldi; column ldi - 32 holds the shift's vector
+  const float* invs = nullptr;     // its scalars
+  int ldi = 0;
+};
+// FP32 inverse of W S for CG64Problem::inv, formed on the device without a
+// host wait; unusable ones (S far from definite) are marked and skipped.
+struct CG64Inverse {
+  DevBuf a, b, s;
+  int n = 0, ld = 0;
+  bool ready = false;              // formed for the current S
+  const float* inv = nullptr;
+  void attach(CG64Problem* P) const {
+    P->inv = inv;
+    P->invs = s.as<float>();
+    P->ldi = ld;
+  }
+};
+int cg64_inverse(CG64Inverse* I, const CG64Problem& P, cudaStream_t st);
+struct CG64State {                 // head of the scratch: results and the grid variant's barrier
+  int iters, timeout;
+  double relres;
+  unsigned arrived, pad;
+};
+size_t cg64_scratch_bytes(int n);
+bool cg64_fits(int n);  // the vectors of n unknowns fit a CTA's shared memory
+inline int cg64_csr_slab(const CG64Problem& P, int rows) { return P.max_row_nnz * rows; }
+// variant: 0 by size, 1 one cluster, 2 cooperative grid
+int launch_cg64(const CG64Problem& P, void* scratch, cudaStream_t st, int variant = 0);
+
 }  // namespace ilm
 
 struct ilm_cache_s {
@@ -513,8 +566,9 @@ struct ilm_cache_s {
   ilm::DevBuf g_scr[6];
   // scratch point buffers (FP64 and cache dtype)
   ilm::DevBuf p_scr[8];
-  // cached Schur complements for the problem solves (FP64 and FP32 copies)
-  ilm::DevBuf S_dir64, S_dir32, S_neu64, S_neu32;
+  // cached Schur complements for the problem solves, and their FP32 inverses
+  ilm::DevBuf S_dir64, S_neu64;
+  ilm::CG64Inverse inv_dir, inv_neu;
   bool S_dir_ready = false, S_neu_ready = false;
   // surface filter: W = E R 1 (cache dtype) and a grid buffer of the cache's class
   ilm::DevBuf filt_diag, filt_grid;
@@ -672,40 +726,6 @@ int schur_build(ilm_cache_s* c, int which, double scale, double* A, cudaStream_t
 // an FP64 cache of the same points as c (c itself when it is FP64), built on
 // first use and dropped when the points move
 int ensure_twin(ilm_cache_s* c, ilm_cache_s** out);
-// FP64 CG of one problem (ilm_cg64.cu): S dense (A column-major) or CSR with
-// float-float values, in the w-weighted inner product (S = M diag(w), M
-// symmetric; w null: ones).  Converged when the true residual ||b - S x||_2
-// <= tol ||b||_2; it is formed when the recursive one says so, every
-// `refresh` iterations and at maxiter.  stall > 0: the best true-residual
-// iterate is kept and the solve stops after `stall` refreshes without gain.
-struct CG64Problem {
-  const double* A = nullptr;       // dense n x n, or
-  const int* rowptr = nullptr;     // CSR
-  const int* colidx = nullptr;
-  const float* vhi = nullptr;
-  const float* vlo = nullptr;
-  int max_row_nnz = 0;             // CSR: bound on a row's entries (sizes the shared-memory slab)
-  const double* b = nullptr;
-  const double* w = nullptr;
-  const double* x0 = nullptr;      // initial guess (may be x); null: zero
-  double* x = nullptr;
-  int n = 0, maxiter = 0, refresh = 100, stall = 0;
-  double tol = 0.0;
-  int* iters = nullptr;            // results (null: in the scratch's CG64State)
-  double* relres = nullptr;
-  int* timeout = nullptr;          // set to 1 if the grid variant's wait ran out (null: in CG64State)
-};
-struct CG64State {                 // head of the scratch: results and the grid variant's barrier
-  int iters, timeout;
-  double relres;
-  unsigned arrived, pad;
-};
-size_t cg64_scratch_bytes(int n);
-bool cg64_fits(int n);  // the vectors of n unknowns fit a CTA's shared memory
-inline int cg64_csr_slab(const CG64Problem& P, int rows) { return P.max_row_nnz * rows; }
-// variant: 0 by size, 1 one cluster, 2 cooperative grid
-int launch_cg64(const CG64Problem& P, void* scratch, cudaStream_t st, int variant = 0);
-
 // batched Schur builds (one launch over all problems of a batch)
 // Row stride (floats) of a batched n x n Schur complement: n rounded up to a
 // multiple of 4, so that every row starts on a 16-byte boundary (vector
