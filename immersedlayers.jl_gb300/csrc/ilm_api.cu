@@ -951,14 +951,14 @@ namespace ilm {
 
 // S of problem `which` (and the FP32 inverse its solves refine), kept until
 // the points move
-static int cached_schur(ilm_cache_s* c, int which, cudaStream_t st) {
+int cached_schur(ilm_cache_s* c, int which, cudaStream_t st) {
   const bool dir = which == ILM_SCHUR_RTLINVR;
   bool& ready = dir ? c->S_dir_ready : c->S_neu_ready;
   if (ready) return ILM_OK;
   DevBuf& S64 = dir ? c->S_dir64 : c->S_neu64;
   const size_t nn = (size_t)c->npts * c->npts;
   ILM_TRY(S64.alloc(std::max<size_t>(nn, 1) * sizeof(double)));
-  ILM_TRY(schur_build(c, which, 1.0, S64.as<double>(), st));
+  ILM_TRY(schur_build(c, which, 1.0, S64.as<double>(), st, true));
   CG64Inverse& inv = dir ? c->inv_dir : c->inv_neu;
   inv.ready = false;
   if (cg64_fits(c->npts)) {
@@ -973,7 +973,7 @@ static int cached_schur(ilm_cache_s* c, int which, cudaStream_t st) {
 }
 
 // Solve S x = rhs (rhs, x FP64 device) on the device, S of problem `which`.
-static int schur_cg(ilm_cache_s* c, int which, const double* rhs, double* x, double tol, int maxiter,
+int schur_cg(ilm_cache_s* c, int which, const double* rhs, double* x, double tol, int maxiter,
                     ilm_solve_info_t* info, cudaStream_t st) {
   const bool dir = which == ILM_SCHUR_RTLINVR;
   const DevBuf& S64 = dir ? c->S_dir64 : c->S_neu64;

@@ -723,6 +723,11 @@ int st_point_dot(int n, int dtype, const void* a, const void* b, const double* w
 // Schur (ilm_schur.cu)
 // any_cache: also on vector caches (their Nodes{Primal} / Nodes{Dual} windows)
 int schur_build(ilm_cache_s* c, int which, double scale, double* A, cudaStream_t st, bool any_cache = false);
+// the dense S of kind `which` (RTLINVR or CLINVCT) kept in the cache, and S x =
+// rhs (FP64 device vectors) on the device (ilm_api.cu)
+int cached_schur(ilm_cache_s* c, int which, cudaStream_t st);
+int schur_cg(ilm_cache_s* c, int which, const double* rhs, double* x, double tol, int maxiter, ilm_solve_info_t* info,
+             cudaStream_t st);
 // an FP64 cache of the same points as c (c itself when it is FP64), built on
 // first use and dropped when the points move
 int ensure_twin(ilm_cache_s* c, ilm_cache_s** out);

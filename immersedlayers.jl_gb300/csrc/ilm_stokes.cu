@@ -123,6 +123,35 @@ __global__ void __launch_bounds__(256) k_gemm_rows(int n, int k, int t, const do
   }
 }
 
+// Z_comp = T R_comp for both velocity components of up to 8 right-hand sides
+// (T symmetric N x N; columns of R and Z 2N apart).  A warp per row of T and
+// component: one thread per row (the kernel above) left 2 CTAs of the chip
+// busy with a chain of N FMAs, 300 us at N = 428 where this takes 7.
+__global__ void __launch_bounds__(256) k_pc_apply(int N, int t, const double* __restrict__ T,
+                                                  const double* __restrict__ R, double* __restrict__ Z) {
+  const int id = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (id >= 2 * N) return;
+  const int comp = id >= N, i = id - comp * N;
+  const double* row = T + (size_t)i * N;
+  const double* r = R + (size_t)comp * N;
+  double acc[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) acc[q] = 0.0;
+  for (int j = lane; j < N; j += 32) {
+    const double a = __ldg(row + j);
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (q < t) acc[q] = fma(a, __ldg(r + j + (size_t)q * 2 * N), acc[q]);
+  }
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    if (q >= t) break;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+    if (lane == 0) Z[(size_t)comp * N + i + (size_t)q * 2 * N] = acc[q];
+  }
+}
+
 // T = sym(Sp diag(1/ds)) + shift (N x N)
 __global__ void k_pc_form(int N, const double* __restrict__ Sp, const double* __restrict__ ds, double shift,
                           double* __restrict__ T) {
@@ -305,6 +334,178 @@ int gemm(int n, int k, int t, const double* A, const double* B, double alpha, do
   return ILM_OK;
 }
 
+// Scalars of cg_single on the device: [0] |b|^2, [1] p.q, [2] |r|^2 of the last
+// step, [3] the smallest |r|^2 so far (that of Ybest)
+__device__ __forceinline__ double cta_sum(double v, double* red) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  __syncthreads();
+  if (lane == 0) red[warp] = v;
+  __syncthreads();
+  double s = lane < (int)(blockDim.x >> 5) ? red[lane] : 0.0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
+__global__ void __launch_bounds__(1024) k_cg1_start(int n, const double* __restrict__ b, double* __restrict__ y,
+                                                    double* __restrict__ r, double* __restrict__ sc) {
+  __shared__ double red[32];
+  double a = 0.0;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    r[i] = b[i];
+    y[i] = 0.0;
+    a = fma(b[i], b[i], a);
+  }
+  a = cta_sum(a, red);
+  if (threadIdx.x == 0) sc[0] = sc[2] = sc[3] = a;
+}
+
+// alpha = p.r / p.q; y += alpha p; r -= alpha q; the best y kept
+__global__ void __launch_bounds__(1024) k_cg1_step(int n, const double* __restrict__ p, const double* __restrict__ q,
+                                                   double* __restrict__ y, double* __restrict__ r,
+                                                   double* __restrict__ ybest, double* __restrict__ sc) {
+  __shared__ double red[32];
+  double pq = 0.0, pr = 0.0;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    pq = fma(p[i], q[i], pq);
+    pr = fma(p[i], r[i], pr);
+  }
+  pq = cta_sum(pq, red);
+  pr = cta_sum(pr, red);
+  const double alpha = pq > 0.0 ? pr / pq : 0.0;
+  double rr = 0.0;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    y[i] = fma(alpha, p[i], y[i]);
+    const double ri = fma(-alpha, q[i], r[i]);
+    r[i] = ri;
+    rr = fma(ri, ri, rr);
+  }
+  rr = cta_sum(rr, red);
+  const double best = sc[3];
+  __syncthreads();
+  if (rr < best)
+    for (int i = threadIdx.x; i < n; i += blockDim.x) ybest[i] = y[i];
+  if (threadIdx.x == 0) {
+    sc[1] = pq;
+    sc[2] = rr;
+    if (rr < best) sc[3] = rr;
+  }
+}
+
+// p = z - (q.z / p.q) p
+__global__ void __launch_bounds__(1024) k_cg1_dir(int n, const double* __restrict__ q, const double* __restrict__ z,
+                                                  double* __restrict__ p, const double* __restrict__ sc) {
+  __shared__ double red[32];
+  double qz = 0.0;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) qz = fma(q[i], z[i], qz);
+  qz = cta_sum(qz, red);
+  const double beta = -qz / sc[1];
+  for (int i = threadIdx.x; i < n; i += blockDim.x) p[i] = fma(beta, p[i], z[i]);
+}
+
+// r = b - q and its squared norm
+__global__ void __launch_bounds__(1024) k_cg1_residual(int n, const double* __restrict__ b,
+                                                       const double* __restrict__ q, double* __restrict__ r,
+                                                       double* __restrict__ sc) {
+  __shared__ double red[32];
+  double rr = 0.0;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const double ri = b[i] - q[i];
+    r[i] = ri;
+    rr = fma(ri, ri, rr);
+  }
+  rr = cta_sum(rr, red);
+  if (threadIdx.x == 0) sc[2] = rr;
+}
+
+// Block CG of one right-hand side: the same recurrence and rules (best iterate
+// kept, true residual before convergence is declared, divergence and stall
+// windows), its scalars and vector updates in one CTA's kernels, one host
+// wait per iteration.
+int cg_single(int n, const BlockApply& A, const BlockPrec* M, const double* b, double* Y, double tol, int maxiter,
+              int* iters, double* relres, cudaStream_t st, int stall) {
+  DevBuf w;
+  ILM_TRY(w.alloc(((size_t)5 * std::max(n, 1) + 4) * sizeof(double)));
+  double* sc = w.as<double>();
+  double *R = sc + 4, *Z = R + n, *P = Z + n, *Q = P + n, *Yb = Q + n;
+  const int T = std::min(1024, std::max(32, (n + 31) / 32 * 32));
+  double h[4];
+  auto read = [&]() -> int {
+    ILM_CHECK_CUDA(cudaMemcpyAsync(h, sc, sizeof(h), cudaMemcpyDeviceToHost, st));
+    ILM_CHECK_CUDA(cudaStreamSynchronize(st));
+    return ILM_OK;
+  };
+  auto precond = [&](double* z) -> int {
+    if (M) return (*M)(R, z, 1);
+    ILM_CHECK_CUDA(cudaMemcpyAsync(z, R, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, st));
+    return ILM_OK;
+  };
+  // the true residual of Y
+  auto residual = [&](double* rel) -> int {
+    ILM_TRY(A(Y, Q, 1));
+    k_cg1_residual<<<1, T, 0, st>>>(n, b, Q, R, sc);
+    ILM_CHECK_LAUNCH();
+    ILM_TRY(read());
+    *rel = sqrt(std::max(h[2], 0.0) / h[0]);
+    return ILM_OK;
+  };
+  *iters = 0;
+  *relres = 0.0;
+  if (n == 0) return ILM_OK;
+  k_cg1_start<<<1, T, 0, st>>>(n, b, Y, R, sc);
+  ILM_CHECK_LAUNCH();
+  ILM_CHECK_CUDA(cudaMemsetAsync(Yb, 0, (size_t)n * sizeof(double), st));
+  ILM_TRY(precond(P));
+  ILM_TRY(read());
+  if (!(h[0] > 0.0)) return ILM_OK;
+  *relres = 1.0;
+  double best = 1.0;
+  int it = 0, last_gain = 0;
+  while (it < maxiter) {
+    ILM_TRY(A(P, Q, 1));
+    k_cg1_step<<<1, T, 0, st>>>(n, P, Q, Y, R, Yb, sc);
+    ILM_CHECK_LAUNCH();
+    ILM_TRY(precond(Z));
+    ILM_TRY(read());
+    if (!(h[1] > 0.0)) break;  // no direction left (stagnation)
+    ++it;
+    const double rel = sqrt(std::max(h[2], 0.0) / h[0]);
+    *relres = rel;
+    if (rel < 0.9 * best) last_gain = it;  // a 10% gain restarts the stall window
+    if (rel < best) best = rel;
+    if (!(rel <= 1e3 * best) || (stall > 0 && it - last_gain >= stall)) {  // back to the best iterate
+      ILM_CHECK_CUDA(cudaMemcpyAsync(Y, Yb, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, st));
+      ILM_TRY(residual(relres));
+      break;
+    }
+    if (rel <= tol || it == maxiter) {
+      ILM_TRY(residual(relres));
+      if (*relres <= tol) break;
+      if (it == maxiter) {
+        if (*relres > best) {  // the kept iterate, if better
+          const double last = *relres;
+          ILM_CHECK_CUDA(cudaMemcpyAsync(P, Y, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, st));
+          ILM_CHECK_CUDA(cudaMemcpyAsync(Y, Yb, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, st));
+          ILM_TRY(residual(relres));
+          if (!(*relres < last)) {
+            ILM_CHECK_CUDA(cudaMemcpyAsync(Y, P, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, st));
+            *relres = last;
+          }
+        }
+        break;
+      }
+      ILM_TRY(precond(Z));  // R is the true residual now
+      ILM_TRY(A(P, Q, 1));  // and Q held S Y
+    }
+    k_cg1_dir<<<1, T, 0, st>>>(n, Q, Z, P, sc);
+    ILM_CHECK_LAUNCH();
+  }
+  *iters = it;
+  return ILM_OK;
+}
+
 // Block CG on B Y = Bb (n x s, FP64 device, column-major); Y = 0 at start.
 // relres[j] = ||Bb_j - B Y_j|| / ||Bb_j|| (recomputed from B Y at the end).
 // `drop`: directions whose A-norm^2 falls below drop x the largest are
@@ -316,6 +517,7 @@ int gemm(int n, int k, int t, const double* A, const double* B, double alpha, do
 // kept one.
 int block_cg(int n, int s, const BlockApply& A, const BlockPrec* M, const double* Bb, double* Y, double tol,
              int maxiter, double drop, int* iters, double* relres, cudaStream_t st, int stall = 0) {
+  if (s == 1) return cg_single(n, A, M, Bb, Y, tol, maxiter, iters, relres, st, stall);
   const size_t nb = (size_t)n * s * sizeof(double);
   BlockCG w;
   DevBuf Ybest;
@@ -560,14 +762,11 @@ struct StokesWork {
   }
   // each velocity component: Z_comp = P^-1 R_comp (leading dimension 2N)
   int applyM(const double* Rb, double* Zb, int s, cudaStream_t st) const {
-    const double* Ti = c->stokes_pc.as<double>();
-    for (int comp = 0; comp < 2; ++comp)
-      for (int j0 = 0; j0 < s; j0 += 8) {
-        const int t = std::min(8, s - j0);
-        k_gemm_rows<<<(N + 255) / 256, 256, 0, st>>>(N, N, t, Ti, N, Rb + comp * N + n2 * j0, (int)n2, 1.0, 0.0,
-                                                     Zb + comp * N + n2 * j0, (int)n2);
-        ILM_CHECK_LAUNCH();
-      }
+    for (int j0 = 0; j0 < s; j0 += 8) {
+      k_pc_apply<<<(2 * N * 32 + 255) / 256, 256, 0, st>>>(N, std::min(8, s - j0), c->stokes_pc.as<double>(),
+                                                           Rb + n2 * j0, Zb + n2 * j0);
+      ILM_CHECK_LAUNCH();
+    }
     return ILM_OK;
   }
 
@@ -594,6 +793,26 @@ struct StokesWork {
     return ilm_surface_filter(c, 2, sig, sig, stream);
   }
 };
+
+// The scalar Schur complement Ss = -C_s L^-1 C_s^T of a vector cache is that
+// of create_CLinvCT: one inverse Laplacian, translation invariant, so the
+// point-pair sums give it exactly where no regularization window meets the
+// ghost layer (where curl! writes zeros).
+bool dense_scalar_schur(ilm_cache_s* c) {
+  if (c->npts == 0 || !cg64_fits(c->npts) || cache_sync_host(c) != ILM_OK) return false;
+  for (int k = 0; k < c->npts; ++k)
+    for (int d = 0; d < 2; ++d)
+      if (c->hbx[d][k] < 1 || c->hbx[d][k] + NTAP > c->grid.nx - 2 || c->hby[d][k] < 1 ||
+          c->hby[d][k] + NTAP > c->grid.ny - 2)
+        return false;
+  return true;
+}
+
+// y[i] = ds[i] x[i]
+__global__ void k_times_ds(int n, const double* x, const double* __restrict__ ds, double* y) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) y[i] = ds[i] * x[i];
+}
 
 int stokes_check(ilm_cache_s* c, int nrhs, double tol, int maxiter) {
   ILM_REQUIRE(c, "null cache");
@@ -648,8 +867,22 @@ int ilm_solve_stokes_multi(ilm_cache_t c, int nrhs, const void* vplus, const voi
   for (int r = 0; r < nrhs; ++r)
     ILM_TRY(w.fields(Y.as<double>() + n2 * r, w.at(sigma_out, n2, r), w.at(v_out, ne, r), w.at(s_out, nd, r), st));
   // Ss d = G^x_s phi in y = W d: (Ss W^-1) y = rhs
-  ILM_TRY(block_cg(N, nrhs, applyBs, nullptr, Bs.as<double>(), Ys.as<double>(), tol, maxiter, drop, &it2, rr2.data(),
-                   st));
+  if (dense_scalar_schur(c)) {
+    ILM_TRY(cached_schur(c, ILM_SCHUR_CLINVCT, st));
+    for (int r = 0; r < nrhs; ++r) {
+      double* y = Ys.as<double>() + (size_t)N * r;
+      ilm_solve_info_t one{0, 1, 0.0};
+      const int rc = schur_cg(c, ILM_SCHUR_CLINVCT, Bs.as<double>() + (size_t)N * r, y, tol, maxiter, &one, st);
+      if (rc != ILM_OK && rc != ILM_ERR_NOT_CONVERGED) return rc;
+      it2 = std::max(it2, one.iterations);
+      rr2[r] = one.rel_residual;
+      k_times_ds<<<(N + 255) / 256, 256, 0, st>>>(N, y, c->ds64.as<double>(), y);
+      ILM_CHECK_LAUNCH();
+    }
+  } else {
+    ILM_TRY(block_cg(N, nrhs, applyBs, nullptr, Bs.as<double>(), Ys.as<double>(), tol, maxiter, drop, &it2,
+                     rr2.data(), st));
+  }
   for (int r = 0; r < nrhs; ++r)
     ILM_TRY(w.finish(Ys.as<double>() + (size_t)N * r, w.at(sigma_out, n2, r), w.at(s_out, nd, r), st));
   ILM_CHECK_CUDA(cudaStreamSynchronize(st));
