@@ -329,164 +329,7 @@ int twiddle_table(int L, int dtype, const void** out) {
 // conflicts); element n = n1 N2 + n2 is at n1 (N2 + 1) + n2, in natural order
 // before and after the transform.
 // ---------------------------------------------------------------------------
-// exp(-2 pi i k / N) for N = 32 and 24 as literals: in the unrolled register
-// DFTs k is a compile-time constant, so the switch folds to an immediate and
-// the multiplications by the trivial factors (0, +-1, +-1/2) simplify
-__device__ __forceinline__ float2 tw32(int k) {
-  switch (k) {
-    case 0: return make_float2(1.000000000e+00f, 0.000000000e+00f);
-    case 1: return make_float2(9.807852804e-01f, -1.950903220e-01f);
-    case 2: return make_float2(9.238795325e-01f, -3.826834324e-01f);
-    case 3: return make_float2(8.314696123e-01f, -5.555702330e-01f);
-    case 4: return make_float2(7.071067812e-01f, -7.071067812e-01f);
-    case 5: return make_float2(5.555702330e-01f, -8.314696123e-01f);
-    case 6: return make_float2(3.826834324e-01f, -9.238795325e-01f);
-    case 7: return make_float2(1.950903220e-01f, -9.807852804e-01f);
-    case 8: return make_float2(0.000000000e+00f, -1.000000000e+00f);
-    case 9: return make_float2(-1.950903220e-01f, -9.807852804e-01f);
-    case 10: return make_float2(-3.826834324e-01f, -9.238795325e-01f);
-    case 11: return make_float2(-5.555702330e-01f, -8.314696123e-01f);
-    case 12: return make_float2(-7.071067812e-01f, -7.071067812e-01f);
-    case 13: return make_float2(-8.314696123e-01f, -5.555702330e-01f);
-    case 14: return make_float2(-9.238795325e-01f, -3.826834324e-01f);
-    case 15: return make_float2(-9.807852804e-01f, -1.950903220e-01f);
-    case 16: return make_float2(-1.000000000e+00f, 0.000000000e+00f);
-    case 17: return make_float2(-9.807852804e-01f, 1.950903220e-01f);
-    case 18: return make_float2(-9.238795325e-01f, 3.826834324e-01f);
-    case 19: return make_float2(-8.314696123e-01f, 5.555702330e-01f);
-    case 20: return make_float2(-7.071067812e-01f, 7.071067812e-01f);
-    case 21: return make_float2(-5.555702330e-01f, 8.314696123e-01f);
-    case 22: return make_float2(-3.826834324e-01f, 9.238795325e-01f);
-    case 23: return make_float2(-1.950903220e-01f, 9.807852804e-01f);
-    case 24: return make_float2(0.000000000e+00f, 1.000000000e+00f);
-    case 25: return make_float2(1.950903220e-01f, 9.807852804e-01f);
-    case 26: return make_float2(3.826834324e-01f, 9.238795325e-01f);
-    case 27: return make_float2(5.555702330e-01f, 8.314696123e-01f);
-    case 28: return make_float2(7.071067812e-01f, 7.071067812e-01f);
-    case 29: return make_float2(8.314696123e-01f, 5.555702330e-01f);
-    case 30: return make_float2(9.238795325e-01f, 3.826834324e-01f);
-    case 31: return make_float2(9.807852804e-01f, 1.950903220e-01f);
-    default: return make_float2(1.f, 0.f);
-  }
-}
-__device__ __forceinline__ float2 tw24(int k) {
-  switch (k) {
-    case 0: return make_float2(1.000000000e+00f, 0.000000000e+00f);
-    case 1: return make_float2(9.659258263e-01f, -2.588190451e-01f);
-    case 2: return make_float2(8.660254038e-01f, -5.000000000e-01f);
-    case 3: return make_float2(7.071067812e-01f, -7.071067812e-01f);
-    case 4: return make_float2(5.000000000e-01f, -8.660254038e-01f);
-    case 5: return make_float2(2.588190451e-01f, -9.659258263e-01f);
-    case 6: return make_float2(0.000000000e+00f, -1.000000000e+00f);
-    case 7: return make_float2(-2.588190451e-01f, -9.659258263e-01f);
-    case 8: return make_float2(-5.000000000e-01f, -8.660254038e-01f);
-    case 9: return make_float2(-7.071067812e-01f, -7.071067812e-01f);
-    case 10: return make_float2(-8.660254038e-01f, -5.000000000e-01f);
-    case 11: return make_float2(-9.659258263e-01f, -2.588190451e-01f);
-    case 12: return make_float2(-1.000000000e+00f, 0.000000000e+00f);
-    case 13: return make_float2(-9.659258263e-01f, 2.588190451e-01f);
-    case 14: return make_float2(-8.660254038e-01f, 5.000000000e-01f);
-    case 15: return make_float2(-7.071067812e-01f, 7.071067812e-01f);
-    case 16: return make_float2(-5.000000000e-01f, 8.660254038e-01f);
-    case 17: return make_float2(-2.588190451e-01f, 9.659258263e-01f);
-    case 18: return make_float2(0.000000000e+00f, 1.000000000e+00f);
-    case 19: return make_float2(2.588190451e-01f, 9.659258263e-01f);
-    case 20: return make_float2(5.000000000e-01f, 8.660254038e-01f);
-    case 21: return make_float2(7.071067812e-01f, 7.071067812e-01f);
-    case 22: return make_float2(8.660254038e-01f, 5.000000000e-01f);
-    case 23: return make_float2(9.659258263e-01f, 2.588190451e-01f);
-    default: return make_float2(1.f, 0.f);
-  }
-}
-
 constexpr int FAST_THREADS = 256;
-
-__host__ __device__ constexpr int bitrev_c(int i, int bits) {
-  int r = 0;
-  for (int b = 0; b < bits; ++b) r |= ((i >> b) & 1) << (bits - 1 - b);
-  return r;
-}
-__host__ __device__ constexpr int ilog2_c(int n) { return n <= 1 ? 0 : 1 + ilog2_c(n / 2); }
-
-// w_N^j (forward sign) for N dividing 32 or 24; conjugated for SIGN > 0
-template <int N, int SIGN>
-__device__ __forceinline__ float2 twr(int j) {
-  float2 w;
-  if (32 % N == 0) w = tw32(j * (32 / N));
-  else w = tw24(j * (24 / N));
-  if (SIGN > 0) w.y = -w.y;
-  return w;
-}
-
-// in-register radix-2 DIT DFT, N a power of two
-template <int N, int SIGN>
-__device__ __forceinline__ void dft_pow2(float2 (&a)[N]) {
-  constexpr int B = ilog2_c(N);
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    const int j = bitrev_c(i, B);
-    if (j > i) {
-      const float2 t = a[i];
-      a[i] = a[j];
-      a[j] = t;
-    }
-  }
-#pragma unroll
-  for (int half = 1; half < N; half *= 2) {
-#pragma unroll
-    for (int k = 0; k < N; k += 2 * half) {
-#pragma unroll
-      for (int j = 0; j < half; ++j) {
-        float2 t = a[k + j + half];
-        if (j != 0) t = cmul(twr<N, SIGN>(j * (N / (2 * half))), t);
-        a[k + j + half] = csub(a[k + j], t);
-        a[k + j] = cadd(a[k + j], t);
-      }
-    }
-  }
-}
-
-// N = 3 M: three interleaved DFTs of length M and a radix-3 combination
-template <int M, int SIGN>
-__device__ __forceinline__ void dft_3m(float2 (&a)[3 * M]) {
-  constexpr int N = 3 * M;
-  float2 b0[M], b1[M], b2[M];
-#pragma unroll
-  for (int m = 0; m < M; ++m) {
-    b0[m] = a[3 * m];
-    b1[m] = a[3 * m + 1];
-    b2[m] = a[3 * m + 2];
-  }
-  dft_pow2<M, SIGN>(b0);
-  dft_pow2<M, SIGN>(b1);
-  dft_pow2<M, SIGN>(b2);
-  const float s3 = 0.86602540378443864676f * (float)SIGN;
-#pragma unroll
-  for (int k = 0; k < M; ++k) {
-    float2 t1 = b1[k], t2 = b2[k];
-    if (k != 0) {
-      t1 = cmul(twr<N, SIGN>(k), t1);
-      t2 = cmul(twr<N, SIGN>(2 * k), t2);
-    }
-    const float2 s = cadd(t1, t2), d = csub(t1, t2);
-    float2 m;
-    m.x = b0[k].x - 0.5f * s.x;
-    m.y = b0[k].y - 0.5f * s.y;
-    float2 id;  // i * SIGN * sqrt(3)/2 * d
-    id.x = -s3 * d.y;
-    id.y = s3 * d.x;
-    a[k] = cadd(b0[k], s);
-    a[k + M] = cadd(m, id);
-    a[k + 2 * M] = csub(m, id);
-  }
-}
-
-template <int N, int SIGN>
-__device__ __forceinline__ void dft_reg(float2 (&a)[N]) {
-  if constexpr (N == 12) dft_3m<4, SIGN>(a);
-  else if constexpr (N == 24) dft_3m<8, SIGN>(a);
-  else dft_pow2<N, SIGN>(a);
-}
 
 // One transform of length N1 N2 on the padded matrix x, by the G threads
 // g = 0..G-1 of a group (act: this group has a transform).  twL[j * tws] =
@@ -1080,7 +923,7 @@ int conv_plan_init(ConvPlan* plan, int n1, int n2, int dtype, cudaStream_t st) {
   plan->dtype = dtype;
   plan->P1 = good_fft_size(2 * n1 - 1);
   plan->P2 = good_fft_size(2 * n2 - 1);
-  if (plan->P1 > 8192 || plan->P2 > 8192) {
+  if (plan->P1 > 8192 || plan->P2 > 6144) {
     set_error("grid too large for the FFT convolution (P=%d x %d)", plan->P1, plan->P2);
     return ILM_ERR_SIZE_LIMIT;
   }
@@ -1107,6 +950,8 @@ int conv_plan_init(ConvPlan* plan, int n1, int n2, int dtype, cudaStream_t st) {
 int conv_apply(ConvPlan* plan, const void* in, void* out, double inv_factor, cudaStream_t st) {
   if (plan->use_sine)
     return sine_apply(&plan->sine, static_cast<const double*>(in), static_cast<double*>(out), inv_factor, st);
+  if (plan->dtype == ILM_F32 && field_conv_supported(plan->P1, plan->P2))
+    return field_conv_apply(plan, static_cast<const float*>(in), static_cast<float*>(out), inv_factor, st);
   ConvJobDev J;
   memset(&J, 0, sizeof(J));
   J.in = in;

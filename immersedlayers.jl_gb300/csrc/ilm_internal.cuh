@@ -360,6 +360,9 @@ struct ConvJobDev {
   // prepared job table write into a caller's buffer)
   size_t out_off;
 };
+// FP32 convolution of one field (ilm_fft_field.cu)
+bool field_conv_supported(int P1, int P2);
+int field_conv_apply(ConvPlan* plan, const float* in, float* out, double scale, cudaStream_t st);
 struct ConvLaunch {
   int rows = 0, cols = 0, CW = 1, maxP1 = 0, maxP2 = 0;
   int fast = 0, frows = 0, firows = 0;  // register four-step FFT path (FP32): forward / inverse row CTAs

@@ -116,8 +116,9 @@ __device__ __forceinline__ Radix stage_radix(int x, int y, int s) {
 }
 constexpr int SR_T = 256;        // threads of k_sine_rows
 constexpr int SR_SPLIT_N = 256;  // largest N of the split stages (two outputs per thread)
+constexpr int SR_FOLD_N = 1024;  // largest N of the split folds
 
-template <bool SPLIT>
+template <bool SPLIT, bool FOLD>
 __global__ void __launch_bounds__(SR_T) k_sine_rows(int N, int lx, int ly, int nrows, const double* __restrict__ in,
                                                     int ldin, int nin, int jin, double* __restrict__ out, int ldout,
                                                     int nout, int kout, double scale, const double2* __restrict__ tw) {
@@ -137,7 +138,7 @@ __global__ void __launch_bounds__(SR_T) k_sine_rows(int N, int lx, int ly, int n
     B[j] = make_double2(ok ? xa[j] : 0.0, ok && two ? xb[j] : 0.0);
   }
   __syncthreads();
-  if (SPLIT) {
+  if (FOLD) {
     // folds: level l leaves p_j at N_l - j and hands z_j - z_{N_l - j} at j to the next
     for (int l = 0; l < lx; ++l) {
       const int Nl = N >> l, H = Nl >> 1;
@@ -320,9 +321,10 @@ __device__ __forceinline__ double mode_sum(double v, double* red) {
   for (int o = 16; o >= MB; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   if ((t & 31) < MB) red[(t >> 5) * MB + m] = v;
   __syncthreads();
-  double s = 0.0;
+  // lane (w, m) takes warp w's sum (lanes beyond the warps: none)
+  double s = (t & 31) < SM_WARPS * MB ? red[t & 31] : 0.0;
 #pragma unroll
-  for (int w = 0; w < SM_WARPS; ++w) s += red[w * MB + m];
+  for (int o = 16; o >= MB; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   __syncthreads();
   return s;
 }
@@ -677,7 +679,7 @@ int sine_apply(SinePlan* p, const double* in, double* out, double inv_factor, cu
   const int ly = (N >> lx) == 3 ? 1 : 0;
   const size_t smr = 2 * (size_t)N * sizeof(double2);
   const int rb = (n2 + N + 7) / 8;
-  auto rows = N <= SR_SPLIT_N ? k_sine_rows<true> : k_sine_rows<false>;
+  auto rows = N <= SR_SPLIT_N ? k_sine_rows<true, true> : N <= SR_FOLD_N ? k_sine_rows<false, true> : k_sine_rows<false, false>;
   ILM_CHECK_CUDA(cudaFuncSetAttribute(rows, cudaFuncAttributeMaxDynamicSharedMemorySize, SM_MAX_SMEM));
   auto modes = [&](bool second) -> int {
     using K = void (*)(int, int, int, double*, const double*, const double*, const double*, const double*,
