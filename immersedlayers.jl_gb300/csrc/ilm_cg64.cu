@@ -175,17 +175,24 @@ __global__ void __launch_bounds__(C64_T, 1) k_cg64(const CG64Args A) {
     const int lane = t & 31, warp = t >> 5;
     for (int i = warp; i < nr; i += C64_T / 32) {
       const float* row = P.inv + (size_t)(r0 + i) * P.ldi;
-      float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+      float a[4] = {0.f, 0.f, 0.f, 0.f};
       int j = lane;
-      for (; j + 96 < n; j += 128) {
-        const float m0 = __ldg(row + j), m1 = __ldg(row + j + 32), m2 = __ldg(row + j + 64), m3 = __ldg(row + j + 96);
-        a0 = fmaf(m0, v[j], a0);
-        a1 = fmaf(m1, v[j + 32], a1);
-        a2 = fmaf(m2, v[j + 64], a2);
-        a3 = fmaf(m3, v[j + 96], a3);
+      for (; j + 7 * 32 < n; j += 8 * 32) {  // eight loads from L2 in flight
+        float m[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) m[q] = __ldg(row + j + 32 * q);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) a[q & 3] = fmaf(m[q], v[j + 32 * q], a[q & 3]);
       }
-      for (; j < n; j += 32) a0 = fmaf(__ldg(row + j), v[j], a0);
-      a0 = (a0 + a1) + (a2 + a3);
+      {
+        float m[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) m[q] = j + 32 * q < n ? __ldg(row + j + 32 * q) : 0.f;
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          if (j + 32 * q < n) a[q & 3] = fmaf(m[q], v[j + 32 * q], a[q & 3]);
+      }
+      float a0 = (a[0] + a[1]) + (a[2] + a[3]);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) a0 += __shfl_xor_sync(0xffffffffu, a0, o);
       const double u = (double)fmaf(shift, __ldg(row + P.ldi - 32), a0);

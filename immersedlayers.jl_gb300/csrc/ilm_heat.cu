@@ -54,34 +54,182 @@ std::vector<double> heat_kernel_taps(double a, double tol = 1e-17, int rmax = 40
   return k;  // one side, k[0] at the centre
 }
 
-// one thread per output; x pass: out[j][i] = sum_m k[|m|] in[j][i+m] (zero outside)
-template <typename T>
-__global__ void k_if_x(int n1, int n2, const double* __restrict__ k, int R, const T* __restrict__ in,
-                       T* __restrict__ out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y;
-  if (i >= n1) return;
-  const T* row = in + (size_t)j * n1;
-  double acc = k[0] * (double)row[i];
-  for (int m = 1; m <= R; ++m) {
-    const double km = k[m];
-    if (i - m >= 0) acc += km * (double)row[i - m];
-    if (i + m < n1) acc += km * (double)row[i + m];
+// ---------------------------------------------------------------------------
+// Integrating-factor passes: out = sum_m k[|m|] in[. + m] along x, then along y
+// (zero outside).  All taps in FP64 are 2 R + 1 ~ 27 operations per value on a
+// unit that issues 1.7 per clock and SM: 50 us per pass of a 1023^2 field.  The
+// taps |m| >= m0, whose sum is at most 2% (at 0.5 h^2 / kappa per step: |m| >=
+// 3), are taken in float-float on the FP32 pipes instead: 2^-48 of 2% is below
+// the rounding of the FP64 sum.  The values are split and put together again
+// with integer operations (a conversion costs as much as an FP64 FMA).  A tile
+// whose values leave FP32's exponent range takes every tap in FP64; a tile of
+// zeros (most of R sigma) is skipped.  A 1023^2 step (the field,
+// the sparse second one and the final sum): 32 us along x and 40 us along y; four
+// FP64 passes and the sum took 4 x 51 + 10.
+// ---------------------------------------------------------------------------
+struct IFTaps {
+  const double* k;    // R + 1
+  const float2* kf;   // the same as (hi, lo)
+  int R, m0;
+};
+
+__device__ __forceinline__ float2 split64(double v) {
+  const unsigned h = (unsigned)__double2hiint(v), l = (unsigned)__double2loint(v);
+  const int e = (int)(h >> 20 & 0x7ffu);
+  const unsigned sg = h & 0x80000000u;
+  float2 r = make_float2(0.f, 0.f);
+  if (e > 896) {
+    r.x = __uint_as_float(sg | (unsigned)(e - 896) << 23 | (h & 0xfffffu) << 3 | l >> 29);
+    if (e > 948)  // the 29 bits below, in units of 2^(e - 1075)
+      r.y = (float)(int)(l & 0x1fffffffu) * __uint_as_float(sg | (unsigned)(e - 948) << 23);
   }
-  out[(size_t)j * n1 + i] = (T)acc;
+  return r;
+}
+__device__ __forceinline__ float2 split64(float v) { return make_float2(v, 0.f); }
+
+__device__ __forceinline__ double widen(float x) {
+  const unsigned b = __float_as_uint(x), e = b >> 23 & 0xffu;
+  return e == 0u ? 0.0 : __hiloint2double((int)((b & 0x80000000u) | (e + 896u) << 20 | (b & 0x7fffffu) >> 3), (int)(b << 29));
 }
 
-template <typename T>
-__global__ void k_if_y(int n1, int n2, const double* __restrict__ k, int R, const T* __restrict__ in,
-                       T* __restrict__ out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y;
-  if (i >= n1) return;
-  double acc = k[0] * (double)in[(size_t)j * n1 + i];
-  for (int m = 1; m <= R; ++m) {
-    const double km = k[m];
-    if (j - m >= 0) acc += km * (double)in[(size_t)(j - m) * n1 + i];
-    if (j + m < n2) acc += km * (double)in[(size_t)(j + m) * n1 + i];
+// stages one value; returns its magnitude bits for the tile's range
+__device__ __forceinline__ unsigned stage_value(double v, float2 f, double* d, float2* s) {
+  *d = v;
+  *s = f;
+  return (unsigned)__double2hiint(v) & 0x7fffffffu;
+}
+
+// what the tile's largest magnitude allows
+enum { IF_ZERO = 0, IF_SPLIT = 1, IF_FP64 = 2 };
+__device__ __forceinline__ int tile_mode(unsigned mag, unsigned low, unsigned* red) {
+  if (threadIdx.x == 0) red[0] = red[1] = 0u;
+  __syncthreads();
+  mag = __reduce_max_sync(0xffffffffu, mag);
+  low = __reduce_max_sync(0xffffffffu, low);
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(red, mag);
+    atomicMax(red + 1, low);
   }
-  out[(size_t)j * n1 + i] = (T)acc;
+  __syncthreads();
+  const unsigned top = red[0] >> 20, any = red[0] | red[1];
+  return any == 0u ? IF_ZERO : top >= 963u && top <= 1143u ? IF_SPLIT : IF_FP64;
+}
+
+// one output: centre index at, tap distance step
+__device__ __forceinline__ double if_value(const double* d, const float2* f, int at, int step, const double* k,
+                                           const float2* kf, int R, int m0, int mode) {
+  double acc = k[0] * d[at];
+  const int near = mode == IF_SPLIT ? min(m0 - 1, R) : R;
+  for (int m = 1; m <= near; ++m) {
+    acc = fma(k[m], d[at - m * step], acc);
+    acc = fma(k[m], d[at + m * step], acc);
+  }
+  if (mode != IF_SPLIT) return acc;
+  FF a{0.f, 0.f}, b{0.f, 0.f};
+#pragma unroll 4
+  for (int m = m0; m <= R; ++m) {
+    const float2 c = kf[m], u = f[at - m * step], v = f[at + m * step];
+    ff_fma(a, c.x, c.y, u.x, u.y);
+    ff_fma(b, c.x, c.y, v.x, v.y);
+  }
+  a = ff_add(a, b);
+  return acc + (widen(a.hi) + widen(a.lo));
+}
+
+constexpr int IF_T = 256;
+constexpr int IFX_C = 128, IFX_R = 8;   // x pass: columns and rows of a tile
+constexpr int IFY_C = 32, IFY_R = 32;   // y pass
+constexpr int IF_RMAX = 40;
+
+// taps into shared memory behind the tile
+__device__ __forceinline__ void stage_taps(const IFTaps& t, double* k, float2* kf) {
+  for (int m = threadIdx.x; m <= t.R; m += IF_T) {
+    k[m] = t.k[m];
+    kf[m] = t.kf[m];
+  }
+}
+
+// x pass of up to two fields (blockIdx.z)
+template <typename T>
+__global__ void __launch_bounds__(IF_T) k_if_x(int n1, int n2, IFTaps t0, const T* __restrict__ in0, T* __restrict__ out0,
+                                               IFTaps t1, const T* __restrict__ in1, T* __restrict__ out1) {
+  extern __shared__ __align__(16) double if_sm[];
+  __shared__ unsigned red[2];
+  __shared__ double k[IF_RMAX + 1];
+  __shared__ float2 kf[IF_RMAX + 1];
+  const IFTaps t = blockIdx.z ? t1 : t0;
+  const T* __restrict__ in = blockIdx.z ? in1 : in0;
+  T* __restrict__ out = blockIdx.z ? out1 : out0;
+  const int W = IFX_C + 2 * t.R, x0 = blockIdx.x * IFX_C, y0 = blockIdx.y * IFX_R;
+  double* d = if_sm;
+  float2* f = reinterpret_cast<float2*>(d + W * IFX_R);
+  stage_taps(t, k, kf);
+  unsigned mag = 0u, low = 0u;
+  for (int q = threadIdx.x; q < W * IFX_R; q += IF_T) {
+    const int r = q / W, i = x0 + q - r * W - t.R, j = y0 + r;
+    const T v = i >= 0 && i < n1 && j < n2 ? in[(size_t)j * n1 + i] : (T)0;
+    mag = max(mag, stage_value((double)v, split64(v), d + q, f + q));
+    low |= (unsigned)__double2loint((double)v);
+  }
+  const int mode = tile_mode(mag, low, red);
+  const int c = threadIdx.x % IFX_C, i = x0 + c;
+  if (i >= n1) return;
+  for (int r = threadIdx.x / IFX_C; r < IFX_R && y0 + r < n2; r += IF_T / IFX_C)
+    out[(size_t)(y0 + r) * n1 + i] =
+        mode == IF_ZERO ? (T)0 : (T)if_value(d, f, r * W + c + t.R, 1, k, kf, t.R, t.m0, mode);
+}
+
+// y pass: out = IFy_0 in0 (+ c1 IFy_1 in1 + c2 add2 + add3, where given)
+template <typename T>
+__global__ void __launch_bounds__(IF_T) k_if_y(int n1, int n2, IFTaps t0, const T* __restrict__ in0, IFTaps t1, double c1,
+                                               const T* __restrict__ in1, double c2, const T* __restrict__ add2,
+                                               const T* __restrict__ add3, T* __restrict__ out) {
+  extern __shared__ __align__(16) double if_sm[];
+  __shared__ unsigned red[2];
+  __shared__ double k[IF_RMAX + 1];
+  __shared__ float2 kf[IF_RMAX + 1];
+  constexpr int PER = IFY_R * IFY_C / IF_T;
+  const int x0 = blockIdx.x * IFY_C, y0 = blockIdx.y * IFY_R, c = threadIdx.x % IFY_C, r0 = threadIdx.x / IFY_C;
+  const int i = x0 + c;
+  double acc[PER];
+#pragma unroll
+  for (int q = 0; q < PER; ++q) acc[q] = 0.0;
+  for (int fld = 0; fld < (in1 ? 2 : 1); ++fld) {
+    const IFTaps t = fld ? t1 : t0;
+    const T* __restrict__ in = fld ? in1 : in0;
+    const int rows = IFY_R + 2 * t.R;
+    double* d = if_sm;
+    float2* f = reinterpret_cast<float2*>(d + rows * IFY_C);
+    stage_taps(t, k, kf);
+    unsigned mag = 0u, low = 0u;
+    for (int q = threadIdx.x; q < rows * IFY_C; q += IF_T) {
+      const int j = y0 + q / IFY_C - t.R;
+      const T v = i < n1 && j >= 0 && j < n2 ? in[(size_t)j * n1 + i] : (T)0;
+      mag = max(mag, stage_value((double)v, split64(v), d + q, f + q));
+      low |= (unsigned)__double2loint((double)v);
+    }
+    const int mode = tile_mode(mag, low, red);
+    if (mode != IF_ZERO && i < n1) {
+#pragma unroll
+      for (int q = 0; q < PER; ++q) {
+        const int r = r0 + q * (IF_T / IFY_C);
+        if (y0 + r >= n2) continue;
+        const double v = if_value(d, f, (r + t.R) * IFY_C + c, IFY_C, k, kf, t.R, t.m0, mode);
+        acc[q] = fld ? fma(c1, v, acc[q]) : v;
+      }
+    }
+    __syncthreads();
+  }
+  if (i >= n1) return;
+#pragma unroll
+  for (int q = 0; q < PER; ++q) {
+    const int j = y0 + r0 + q * (IF_T / IFY_C);
+    if (j >= n2) continue;
+    const size_t at = (size_t)j * n1 + i;
+    double v = acc[q];
+    if (add2) v = fma(c2, (double)add2[at], v) + (double)add3[at];
+    out[at] = (T)v;
+  }
 }
 
 // smeared-window gather: out_k = sum_{jj,ii} wy[k][jj] wx[k][ii] T[by+jj][bx+ii]
@@ -103,16 +251,19 @@ __global__ void k_conv_gather2(int N, int n1, int n2, const T* __restrict__ f, i
   const int e0 = set ? by1[k] : by0[k];
   const double* wx = (set ? wx1 : wx0) + (size_t)k * L;
   const double* wy = (set ? wy1 : wy0) + (size_t)k * L;
+  // a lane keeps its columns (one, or three at most: L <= 84) and sums over the
+  // rows, eight rows' loads in flight; the column weight comes last
   double acc = 0.0;
-  for (int jj = 0; jj < L; ++jj) {
-    const int j = e0 + jj;
-    if ((unsigned)j >= (unsigned)n2) continue;
-    double racc = 0.0;
-    for (int ii = lane; ii < L; ii += 32) {
-      const int i = b0 + ii;
-      if ((unsigned)i < (unsigned)n1) racc += wx[ii] * (double)f[(size_t)j * n1 + i];
+  for (int ii = lane; ii < L; ii += 32) {
+    const int i = b0 + ii;
+    if ((unsigned)i >= (unsigned)n1) continue;
+    double col = 0.0;
+#pragma unroll 8
+    for (int jj = 0; jj < L; ++jj) {
+      const int j = e0 + jj;
+      if ((unsigned)j < (unsigned)n2) col = fma(wy[jj], (double)f[(size_t)j * n1 + i], col);
     }
-    acc += wy[jj] * racc;
+    acc = fma(wx[ii], col, acc);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
@@ -149,13 +300,6 @@ __global__ void k_stage_rhs(int n, const double* __restrict__ avg, const double*
   rhs[k] = (avg[k] - s) * inv_denom;
 }
 
-template <typename T>
-__global__ void k_heat_combine(size_t n, const T* __restrict__ a, double cb, const T* __restrict__ b, double cc,
-                               const T* __restrict__ c, const T* __restrict__ d, T* __restrict__ out) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    out[i] = (T)((double)a[i] + cb * (double)b[i] + cc * (double)c[i] + (double)d[i]);
-}
-
 }  // namespace
 
 }  // namespace ilm
@@ -173,7 +317,8 @@ struct ilm_heat_s {
   int n1 = 0, n2 = 0;
   // integrating-factor taps for a * (1/3, 2/3, 1)
   int R[3] = {0, 0, 0};
-  DevBuf kt[3];
+  DevBuf kt[3], ktf[3];
+  int m0[3] = {1, 1, 1};
   // smeared gather windows for a/3 (set 0) and a (set 1)
   int L[2] = {0, 0};
   DevBuf gbx[2], gby[2], gwx[2], gwy[2];
@@ -198,17 +343,26 @@ int upd(DevBuf& b, const void* h, size_t bytes) {
   return ILM_OK;
 }
 
-int apply_if_dev(ilm_heat_s* H, int which, const void* in, void* tmp, void* out, cudaStream_t st) {
-  const int R = H->R[which];
-  const double* k = H->kt[which].as<double>();
-  dim3 blk(256), grd((H->n1 + 255) / 256, H->n2);
-  if (H->c->dtype == ILM_F64) {
-    k_if_x<double><<<grd, blk, 0, st>>>(H->n1, H->n2, k, R, static_cast<const double*>(in), static_cast<double*>(tmp));
-    k_if_y<double><<<grd, blk, 0, st>>>(H->n1, H->n2, k, R, static_cast<const double*>(tmp), static_cast<double*>(out));
-  } else {
-    k_if_x<float><<<grd, blk, 0, st>>>(H->n1, H->n2, k, R, static_cast<const float*>(in), static_cast<float*>(tmp));
-    k_if_y<float><<<grd, blk, 0, st>>>(H->n1, H->n2, k, R, static_cast<const float*>(tmp), static_cast<float*>(out));
-  }
+IFTaps taps_of(const ilm_heat_s* H, int which) {
+  return IFTaps{H->kt[which].as<double>(), H->ktf[which].as<float2>(), H->R[which], H->m0[which]};
+}
+
+// out = exp(a_0 L) in0 (+ c1 exp(a_1 L) in1 + c2 add2 + add3); tmp0, tmp1: the fields after their x pass
+template <typename T>
+int apply_if(const ilm_heat_s* H, int w0, const void* in0, void* tmp0, int w1, double c1, const void* in1, void* tmp1,
+             double c2, const void* add2, const void* add3, void* out, cudaStream_t st) {
+  const IFTaps t0 = taps_of(H, w0), t1 = in1 ? taps_of(H, w1) : t0;
+  const int R = std::max(t0.R, t1.R), n1 = H->n1, n2 = H->n2;
+  const size_t sx = (size_t)(IFX_C + 2 * R) * IFX_R * 16, sy = (size_t)(IFY_R + 2 * R) * IFY_C * 16;
+  ILM_CHECK_CUDA(cudaFuncSetAttribute(k_if_x<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
+  ILM_CHECK_CUDA(cudaFuncSetAttribute(k_if_y<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
+  k_if_x<T><<<dim3((n1 + IFX_C - 1) / IFX_C, (n2 + IFX_R - 1) / IFX_R, in1 ? 2 : 1), IF_T, sx, st>>>(
+      n1, n2, t0, static_cast<const T*>(in0), static_cast<T*>(tmp0), t1, static_cast<const T*>(in1),
+      static_cast<T*>(tmp1));
+  ILM_CHECK_LAUNCH();
+  k_if_y<T><<<dim3((n1 + IFY_C - 1) / IFY_C, (n2 + IFY_R - 1) / IFY_R), IF_T, sy, st>>>(
+      n1, n2, t0, static_cast<const T*>(tmp0), t1, c1, static_cast<const T*>(in1 ? tmp1 : nullptr), c2,
+      static_cast<const T*>(add2), static_cast<const T*>(add3), static_cast<T*>(out));
   ILM_CHECK_LAUNCH();
   return ILM_OK;
 }
@@ -378,6 +532,16 @@ int ilm_heat_create(ilm_cache_t c, double kappa, double dt, const double* tb_plu
     taps[w] = heat_kernel_taps(af * frac[w]);
     H->R[w] = (int)taps[w].size() - 1;
     ILM_TRY(upd(H->kt[w], taps[w].data(), taps[w].size() * sizeof(double)));
+    std::vector<float> tf(2 * taps[w].size());
+    double far = 0.0;
+    H->m0[w] = H->R[w] + 1;  // the taps from m0 on add up to at most 2% (both sides)
+    for (int m = H->R[w]; m >= 0; --m) {
+      tf[2 * m] = (float)taps[w][m];
+      tf[2 * m + 1] = (float)(taps[w][m] - (double)tf[2 * m]);
+      far += 2.0 * taps[w][m];
+      if (m > 0 && far <= 0.02) H->m0[w] = m;
+    }
+    ILM_TRY(upd(H->ktf[w], tf.data(), tf.size() * sizeof(float)));
   }
   ILM_TRY(build_gather_windows(H, taps[0], 0));
   ILM_TRY(build_gather_windows(H, taps[2], 1));
@@ -408,7 +572,8 @@ int ilm_heat_create(ilm_cache_t c, double kappa, double dt, const double* tb_plu
   ILM_TRY(H->cfield.alloc(np * es));
   for (int t = 0; t < 4; ++t) ILM_TRY(H->e[t].alloc((size_t)N * 8));
   for (int w = 0; w < 3; ++w) {
-    ILM_TRY(apply_if_dev(H, w, r1, H->tmp[1].p, H->tmp[2].p, nullptr));
+    ILM_TRY((c->dtype == ILM_F64 ? apply_if<double> : apply_if<float>)(H, w, r1, H->tmp[1].p, 0, 0.0, nullptr, nullptr,
+                                                                       0.0, nullptr, nullptr, H->tmp[2].p, nullptr));
     ILM_TRY(ilm_interpolate(c, ILM_NODES_PRIMAL, H->tmp[2].p, pt.p, nullptr));
     ILM_TRY(st_convert(N, c->dtype, pt.p, ILM_F64, H->e[w].p, nullptr));
     if (w == 1) {  // cfield = dt b2 exp(2a/3 L) r1 + dt b3 r1   (b1 = 0)
@@ -449,7 +614,6 @@ int ilm_heat_advance(ilm_heat_t H, void* T, void* sigma_out, int nsteps, ilm_str
   ilm_cache_s* c = H->c;
   cudaStream_t st = as_stream(stream);
   const int N = c->npts;
-  const size_t np = (size_t)H->n1 * H->n2;
   const double dt = H->dt;
   const int wb = (2 * N * 32 + 255) / 256;
   const int pb = (N + 255) / 256;
@@ -494,21 +658,13 @@ int ilm_heat_advance(ilm_heat_t H, void* T, void* sigma_out, int nsteps, ilm_str
     ILM_CHECK_LAUNCH();
     ILM_TRY(run_cg(H, 2, st));
     // grid: T <- exp(aL) T + dt b2 exp(2a/3 L) R sigma2 + dt b3 R sigma3 + cfield
-    ILM_TRY(apply_if_dev(H, 2, T, H->tmp[0].p, H->tmp[1].p, st));
     ILM_TRY(st_convert(N, ILM_F64, H->sig[1].p, c->dtype, H->sig_t.p, st));
     ILM_TRY(ilm_regularize(c, ILM_NODES_PRIMAL, H->sig_t.p, H->tmp[2].p, st));
-    ILM_TRY(apply_if_dev(H, 1, H->tmp[2].p, H->tmp[0].p, H->tmp[3].p, st));
     ILM_TRY(st_convert(N, ILM_F64, H->sig[2].p, c->dtype, H->sig_t.p, st));
-    ILM_TRY(ilm_regularize(c, ILM_NODES_PRIMAL, H->sig_t.p, H->tmp[2].p, st));
-    if (c->dtype == ILM_F64)
-      k_heat_combine<double><<<1024, 256, 0, st>>>(np, H->tmp[1].as<double>(), dt * H->b2, H->tmp[3].as<double>(),
-                                                    dt * H->b3, H->tmp[2].as<double>(), H->cfield.as<double>(),
-                                                    static_cast<double*>(T));
-    else
-      k_heat_combine<float><<<1024, 256, 0, st>>>(np, H->tmp[1].as<float>(), dt * H->b2, H->tmp[3].as<float>(),
-                                                   dt * H->b3, H->tmp[2].as<float>(), H->cfield.as<float>(),
-                                                   static_cast<float*>(T));
-    ILM_CHECK_LAUNCH();
+    ILM_TRY(ilm_regularize(c, ILM_NODES_PRIMAL, H->sig_t.p, H->tmp[3].p, st));
+    ILM_TRY((c->dtype == ILM_F64 ? apply_if<double> : apply_if<float>)(H, 2, T, H->tmp[0].p, 1, dt * H->b2, H->tmp[2].p,
+                                                                       H->tmp[1].p, dt * H->b3, H->tmp[3].p,
+                                                                       H->cfield.p, T, st));
   }
   if (sigma_out) {  // the reference's constraint force enters as -R sigma
     ILM_TRY(st_convert(N, ILM_F64, H->sig[2].p, c->dtype, sigma_out, st));

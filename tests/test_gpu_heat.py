@@ -133,3 +133,37 @@ def test_heat_rejects_index_scaling_and_large_steps(cuda):
         sys = il.construct_system(prob)
         with pytest.raises((ValueError, il._lib.ILMError)):
             il.init(il.init_sol(sys), (0.0, 1.0), sys)
+
+
+@pytest.mark.parametrize("scale", [1.0, 2.0 ** -100])
+@pytest.mark.parametrize("fourier", [0.05, 0.5, 4.0])
+def test_heat_integrating_factor_tiles(cuda, fourier, scale):
+    """The integrating-factor passes over ragged tiles (133 nodes a side, radii
+    from 8 to 29, a block of zeros) where no surface term reaches: one step is
+    there exp(Fo L) T with zeros outside.  The scaled field leaves the range of
+    the float-float taps, so every tap of it is taken in FP64.  Two passes of at
+    most 59 rounded FP64 taps, whose own values agree to some 1e-14: 1e-13."""
+    import torch
+    import immersedlayers as il
+    og, b = heat_case(ds_factor=1.4)
+    n = [len(c) for c in og.coords(O.NODES_PRIMAL)]
+    T0 = scale * np.random.default_rng(5).standard_normal(n)
+    T0[30:, 90:] = 0.0
+    zero = lambda t, x, c, p, m: il.zeros_surface(c)
+    prob = il.DirichletHeatConductionProblem(
+        il.PhysicalGrid((-1.28, 1.28), (-1.28, 1.28), og.h), b, dtype=torch.float64,
+        phys_params={"diffusivity": 1.0, "Fourier": fourier}, bc={"exterior": zero, "interior": zero},
+        timestep_func=il.timestep_fourier)
+    sys = il.construct_system(prob)
+    u0 = il.init_sol(sys)
+    u0.state.set_numpy(T0)
+    integ = il.init(u0, (0.0, 1.0), sys, tol=1e-12, maxiter=500)
+    integ.advance(1)
+    torch.cuda.synchronize()
+    T = il.temperature(integ).numpy_components()
+    ref = O.apply_if(T0, fourier)
+    x, y = og.coords(O.NODES_PRIMAL)
+    reach = 0.4 + (3 + O.heat_kernel_1d(fourier).size // 2) * og.h
+    free = np.maximum(np.abs(x)[:, None], np.abs(y)[None, :]) > reach
+    assert free.sum() > 300
+    assert np.abs(T - ref)[free].max() < 1e-13 * np.abs(ref).max()
