@@ -43,11 +43,17 @@ namespace {
 
 constexpr int C64_T = 256;             // threads per CTA
 constexpr int C64_CLUSTER = 16;        // CTAs of the cluster variant
-constexpr int C64_MAX_SMEM = 227 * 1024 - 256;  // dynamic shared memory beside the static scalars
+// dynamic shared memory beside the static scalars
+constexpr int C64_MAX_CLUSTER = 227 * 1024 - 512, C64_MAX_GRID = 227 * 1024 - 256;
 // matrix entries up to which the cluster variant is used: an iteration of a
 // dense n takes 4.8 / 5.4 / 6.9 / 8.2 us with the cluster and 5.5 / 5.8 / 6.8 /
 // 6.9 us with the grid at n = 157 / 224 / 300 / 400
 constexpr long long C64_CLUSTER_ENTRIES = 256 * 256;
+// unknowns up to which it is used with an FP32 inverse, whose rows 16 SMs read
+// from L2 (us per solve, cluster and grid): dense n = 157 25 / 33, 300 39.6 /
+// 41.2, 400 41.6 / 34.9; 19 entries a row, n = 157 29 / 39, 560 39.1 / 39.8,
+// 696 43.3 / 41.3
+constexpr int C64_CLUSTER_DENSE = 320, C64_CLUSTER_CSR = 560;
 constexpr unsigned C64_SPIN = 1u << 22;  // polls of the grid barrier before it gives up (seconds)
 
 struct CG64Args {
@@ -57,7 +63,8 @@ struct CG64Args {
   int resident;     // the CTA's rows of S are kept in shared memory
   int ld;           // row stride of the resident dense slab (doubles)
   int slab_nnz;     // CSR: entries of the largest slab
-  double* gq;       // grid variant: two exchange buffers of n doubles
+  int nv;           // stride of the shared-memory vectors (n rounded up to 4)
+  double* gq;       // grid variant: exchange (two vectors of n doubles, two sums per CTA)
   CG64State* state;
 };
 
@@ -72,6 +79,7 @@ struct Scal {
   double part[16];
   float part32[8];
   double a, b, c;   // first sum, second sum, derived scalar
+  unsigned top;     // refinement: largest magnitude bits of b
   int flag;
 };
 
@@ -111,14 +119,15 @@ __global__ void __launch_bounds__(C64_T, 1) k_cg64(const CG64Args A) {
   const int r0 = min(n, rank * A.R), nr = min(A.R, n - r0);
   extern __shared__ __align__(16) double sm[];
   double* x = sm;
-  double* r = x + n;
-  double* p = r + n;
-  double* w = p + n;
-  double* qb = w + n;                          // cluster: two buffers; grid: one
-  double* slab = qb + (GRID ? 1 : 2) * (size_t)n;
+  double* r = x + A.nv;
+  double* p = r + A.nv;
+  double* w = p + A.nv;
+  double* qb = w + A.nv;                       // cluster: two buffers; grid: one
+  double* slab = qb + (GRID ? 1 : 2) * (size_t)A.nv;
   int* scol = reinterpret_cast<int*>(slab + A.slab_nnz);
   __shared__ Scal s;
   __shared__ int s_ok;
+  __shared__ double tot[GRID ? 1 : 2 * C64_CLUSTER];  // refinement: the CTAs' parts of |r|^2 and |b|^2
   int par = 0;           // exchange buffer
   unsigned bar = 0;      // grid barriers passed
   bool ok = true;
@@ -129,7 +138,7 @@ __global__ void __launch_bounds__(C64_T, 1) k_cg64(const CG64Args A) {
     if (CSR) {
       const int e1 = P.rowptr[r0 + nr];
       for (int e = e0 + t; e < e1; e += C64_T) {
-        slab[e - e0] = (double)P.vhi[e] + (double)P.vlo[e];
+        slab[e - e0] = widen(P.vhi[e]) + widen(P.vlo[e]);
         scol[e - e0] = P.colidx[e];
       }
     } else {
@@ -140,8 +149,8 @@ __global__ void __launch_bounds__(C64_T, 1) k_cg64(const CG64Args A) {
     }
   }
 
-  // the CTAs' rows of one vector become visible to all
-  auto publish = [&](double* q) {
+  // what the CTAs sent becomes visible to all
+  auto barrier = [&]() {
     if (GRID) {
       // counter barrier: every CTA of the cooperative launch is resident; the
       // wait is bounded all the same
@@ -160,60 +169,27 @@ __global__ void __launch_bounds__(C64_T, 1) k_cg64(const CG64Args A) {
       }
       __syncthreads();
       ok = s_ok != 0;
-      for (int j = t; j < n; j += C64_T) q[j] = __ldcg(A.gq + (size_t)par * n + j);
-      // no CTA barrier here: each thread reads back the entries it stored
     } else {
       cg::this_cluster().sync();
     }
+  };
+
+  // the CTAs' rows of one vector become visible to all
+  auto publish = [&](double* q) {
+    barrier();
+    if (GRID)
+      for (int j = t; j < n; j += C64_T) q[j] = __ldcg(A.gq + (size_t)par * n + j);
+    // no CTA barrier here: each thread reads back the entries it stored
     par ^= 1;
   };
 
-  // rows r0 .. r0 + nr of P v for the FP32 inverse (v in shared memory, FP32),
-  // each row a warp's, sent to every CTA
-  auto product32 = [&](const float* v, float shift) -> double* {
-    double* q = GRID ? qb : qb + (size_t)par * n;
-    const int lane = t & 31, warp = t >> 5;
-    for (int i = warp; i < nr; i += C64_T / 32) {
-      const float* row = P.inv + (size_t)(r0 + i) * P.ldi;
-      float a[4] = {0.f, 0.f, 0.f, 0.f};
-      int j = lane;
-      for (; j + 7 * 32 < n; j += 8 * 32) {  // eight loads from L2 in flight
-        float m[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) m[q] = __ldg(row + j + 32 * q);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) a[q & 3] = fmaf(m[q], v[j + 32 * q], a[q & 3]);
-      }
-      {
-        float m[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) m[q] = j + 32 * q < n ? __ldg(row + j + 32 * q) : 0.f;
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-          if (j + 32 * q < n) a[q & 3] = fmaf(m[q], v[j + 32 * q], a[q & 3]);
-      }
-      float a0 = (a[0] + a[1]) + (a[2] + a[3]);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) a0 += __shfl_xor_sync(0xffffffffu, a0, o);
-      const double u = (double)fmaf(shift, __ldg(row + P.ldi - 32), a0);
-      if (GRID) {
-        if (lane == 0) __stcg(A.gq + (size_t)par * n + r0 + i, u);
-      } else if (lane < G) {
-        cg::this_cluster().map_shared_rank(q, lane)[r0 + i] = u;
-      }
-    }
-    publish(q);
-    return q;
-  };
-
-  // rows r0 .. r0 + nr of S v, sent to every CTA; returns the whole product
-  // (cluster: the buffer the other CTAs wrote; grid: the CTA's own copy)
-  auto product = [&](const double* v) -> double* {
+  // rows r0 .. r0 + nr of S v; emit(i, value, c, L) with row i's value in each
+  // of its L lanes (c: the lane)
+  auto rows_of = [&](const double* v, auto emit) {
     const int L = A.lpr, c = t & (L - 1), rows = C64_T / L;
-    double* q = GRID ? qb : qb + (size_t)par * n;
     if (!CSR && GRID && !A.resident) {
       // S streamed from L2: consecutive threads take consecutive rows of one
-      // column, partial sums meet in q (free between products; n > C64_T here)
+      // column, partial sums meet in qb (free between products; n > C64_T here)
       for (int b0 = 0; b0 < nr; b0 += C64_T) {
         const int m = min(C64_T, nr - b0), nc = C64_T / m, k = t / m, i = t - k * m;
         if (k < nc) {
@@ -229,13 +205,13 @@ __global__ void __launch_bounds__(C64_T, 1) k_cg64(const CG64Args A) {
             a1 = fma(s3, v[j + 3 * nc], a1);
           }
           for (; j < n; j += nc) a0 = fma(__ldg(col + (size_t)j * n), v[j], a0);
-          q[t] = a0 + a1;
+          qb[t] = a0 + a1;
         }
         __syncthreads();
         if (t < m) {
-          double a = q[t];
-          for (int u = 1; u < nc; ++u) a += q[u * m + t];
-          __stcg(A.gq + (size_t)par * n + r0 + b0 + t, a);
+          double a = qb[t];
+          for (int u = 1; u < nc; ++u) a += qb[u * m + t];
+          emit(b0 + t, a, 0, 1);
         }
         __syncthreads();
       }
@@ -250,7 +226,7 @@ __global__ void __launch_bounds__(C64_T, 1) k_cg64(const CG64Args A) {
               for (int k = b + c; k < e; k += L) a0 = fma(slab[k - e0], v[scol[k - e0]], a0);
             else
               for (int k = b + c; k < e; k += L)
-                a0 = fma((double)__ldg(P.vhi + k) + (double)__ldg(P.vlo + k), v[__ldg(P.colidx + k)], a0);
+                a0 = fma(widen(__ldg(P.vhi + k)) + widen(__ldg(P.vlo + k)), v[__ldg(P.colidx + k)], a0);
           } else {
             const double* row = slab + (size_t)i * A.ld;
             int j = c;
@@ -263,16 +239,24 @@ __global__ void __launch_bounds__(C64_T, 1) k_cg64(const CG64Args A) {
         }
         a0 += a1;
         for (int o = L >> 1; o > 0; o >>= 1) a0 += __shfl_xor_sync(0xffffffffu, a0, o);
-        if (i < nr) {
-          if (GRID) {
-            if (c == 0) __stcg(A.gq + (size_t)par * n + r0 + i, a0);
-          } else {
-            cg::cluster_group cl = cg::this_cluster();
-            for (int d = c; d < G; d += L) cl.map_shared_rank(q, d)[r0 + i] = a0;
-          }
-        }
+        if (i < nr) emit(i, a0, c, L);
       }
     }
+  };
+
+  // entry k (of this CTA's rows, or any) of an exchanged vector, to every CTA
+  auto send = [&](double* local, double* global, int k, double v, int c, int L) {
+    if (GRID) {
+      if (c == 0) __stcg(global + k, v);
+    } else {
+      for (int d = c; d < G; d += L) cg::this_cluster().map_shared_rank(local, d)[k] = v;
+    }
+  };
+
+  // S v in all CTAs (cluster: the buffer the other CTAs wrote; grid: the CTA's own copy)
+  auto product = [&](const double* v) -> double* {
+    double* q = GRID ? qb : qb + (size_t)par * A.nv;
+    rows_of(v, [&](int i, double a, int c, int L) { send(q, A.gq + (size_t)par * n, r0 + i, a, c, L); });
     publish(q);
     return q;
   };
@@ -283,86 +267,202 @@ __global__ void __launch_bounds__(C64_T, 1) k_cg64(const CG64Args A) {
   }
   if (!GRID) cg::this_cluster().sync();  // every CTA of the cluster runs before its shared memory is written
   __syncthreads();
-  if (P.x0) {  // warm start: r = b - S x0 (x0 may be the output: all CTAs have read it at the barrier)
-    const double* q = product(x);
-    for (int j = t; j < n; j += C64_T) r[j] = P.b[j] - q[j];
-  } else {
-    for (int j = t; j < n; j += C64_T) r[j] = P.b[j];
-  }
-  double bb = 0.0, rr = 0.0;
-  for (int j = t; j < n; j += C64_T) {
-    bb += P.b[j] * P.b[j];
-    rr += r[j] * r[j];
-  }
-  block_sums(bb, rr, true, n, s, [](double, double) {});
-  bb = s.a;
-  rr = s.b;
-  const double bnorm = sqrt(bb), thr = P.tol * bnorm, thr2 = thr * thr;
+  double bb = 0.0, rr = 0.0, bnorm = 0.0, thr2 = 0.0, thr = 0.0, last = 0.0;
+  auto set_norm = [&]() {
+    bnorm = sqrt(bb);
+    thr = P.tol * bnorm;
+    thr2 = thr * thr;
+    last = bb;
+  };
   // squared norms are compared, except where they are about to underflow
   auto below = [&](double v) { return v <= thr2 || v < 1e-280; };
   auto converged = [&](double v) { return thr2 > 1e-280 ? v <= thr2 : sqrt(v) <= thr; };
+  // r = b - S x0, or b (x0 may be the output: all CTAs have read it at the barrier)
+  auto start = [&]() {
+    const double* q = P.x0 ? product(x) : nullptr;
+    for (int j = t; j < n; j += C64_T) r[j] = P.x0 ? P.b[j] - q[j] : P.b[j];
+  };
   int it = 0;
-  bool done = bnorm == 0.0;
-  double last = bb;
-  if (P.inv && P.invs[0] != 0.f && !done) {
-    float* v = reinterpret_cast<float*>(p);  // W r scaled into FP32's range
+  bool done = false;
+  const bool refine = P.inv && P.invs[0] != 0.f;
+  if (refine) {
+    // Steps x += P r, r = b - S x.  A CTA forms r and the update of x for its own
+    // rows only (a pass of FP64 operations over all n costs n / 1.7 clocks) and
+    // sends W r, in FP32, and x: two barriers per step.  The norm of a residual is
+    // summed beside the product with P and judged beside the next residual's, by
+    // the last warp, off the chain of the others: so the correction after the
+    // residual that passes is always taken.  It is wanted: that residual is rich in
+    // the modes that P gets least right, the slow ones, and x is further off for it
+    // than a CG iterate of that residual (steps gained a factor of four so far).
+    float* v = reinterpret_cast<float*>(p);               // W r scaled into FP32's range
+    float* gv = reinterpret_cast<float*>(A.gq + n);       // grid: its exchange
+    double* gs = A.gq + 2 * (size_t)n;                    // grid: the CTAs' sums
+    const int lane = t & 31, warp = t >> 5;
     const float kappa = P.invs[1];
-    // x += P r, r the residual of squared norm rho
-    auto correct = [&](double rho) {
-      const int e = (__double2hiint(rho) >> 20 & 0x7ff) - 1023;  // rho ~ 2^e
-      const double down = __hiloint2double((1023 - e / 2) << 20, 0), up = __hiloint2double((1023 + e / 2) << 20, 0);
-      float g = 0.f, shift = 0.f;
-      for (int j = t; j < n; j += C64_T) {
-        const float vj = (float)(w[j] * (r[j] * down));
-        v[j] = vj;
-        if (kappa != 0.f) g = fmaf(__ldg(P.inv + (size_t)j * P.ldi + P.ldi - 32), vj, g);
+    if (t == 0) s.top = 0u;
+    __syncthreads();
+    unsigned top = 0u;
+    for (int j = t; j < n; j += C64_T) top = max(top, (unsigned)__double2hiint(P.b[j]) & 0x7fffffffu);
+    top = __reduce_max_sync(0xffffffffu, top);
+    if (lane == 0) atomicMax(&s.top, top);
+    for (int j = n + t; j < A.nv; j += C64_T) v[j] = 0.f;
+    __syncthreads();
+    const int e = min(max((int)(s.top >> 20) - 1023, -1000), 1000);  // max |b| ~ 2^e
+    const double down = __hiloint2double((1023 - e) << 20, 0), up = __hiloint2double((1023 + e) << 20, 0);
+    auto residual = [&](int i, double y, int c, int L) {
+      const double ri = P.b[r0 + i] - y;
+      const float vi = (float)(w[r0 + i] * (ri * down));
+      if (c == 0) r[r0 + i] = ri;
+      if (GRID) {
+        if (c == 0) __stcg(gv + r0 + i, vi);
+      } else {
+        for (int d = c; d < G; d += L) cg::this_cluster().map_shared_rank(v, d)[r0 + i] = vi;
       }
+    };
+    auto gather_x = [&]() {
+      if (GRID)
+        for (int j = t; j < n; j += C64_T) x[j] = __ldcg(A.gq + j);
+      __syncthreads();
+    };
+    constexpr int LAST = C64_T / 32 - 1;
+    enum { DONE = 1, UNDO = 2, RESET = 4 };
+    double* old = p + A.nv / 2;  // the CTA's rows of x before the last correction (behind v)
+    int flags = 0;
+    if (!P.x0)
+      for (int i = t; i < nr; i += C64_T) residual(i, 0.0, 0, 1);
+    for (int round = 0;; ++round) {
+      if (round || P.x0) rows_of(x, residual);
+      if (round && warp == LAST) {  // judge the residual of the round before
+        double a = 0.0, b = 0.0;
+        for (int k = lane; k < G; k += 32) {
+          a += GRID ? __ldcg(gs + 2 * k) : tot[2 * k];
+          if (round == 1) b += GRID ? __ldcg(gs + 2 * k + 1) : tot[2 * k + 1];
+        }
+        const double now = warp_sum(a);
+        int f = 0;
+        if (round == 1) {
+          bb = warp_sum(b);
+          rr = now;
+          set_norm();
+          last = rr;
+          if (bnorm == 0.0 || rr == 0.0) f = DONE | UNDO;
+          else if (converged(rr)) f = DONE;
+        } else {
+          if (converged(now)) f |= DONE;
+          if (!(now <= 0.0625 * last)) f |= UNDO;                   // slow: from here on CG
+          if (f == UNDO && !(now <= rr)) f |= RESET;                // no better than the start: the CG begins there
+          last = f & RESET ? rr : now;
+        }
+        if (f == 0 && round - 1 >= P.maxiter) f = UNDO;
+        if (lane == 0) {
+          s.a = last;
+          s.b = bb;
+          s.flag = f;
+        }
+      }
+      __syncthreads();
+      if (round) {
+        it = round - 1;
+        flags = s.flag;
+        if (flags) break;
+      }
+      barrier();
+      if (!ok) break;
+      if (GRID)
+        for (int j = t; j < n; j += C64_T) v[j] = __ldcg(gv + j);
+      float shift = 0.f;
       if (kappa != 0.f) {
+        float g = 0.f;
+        for (int j = t; j < n; j += C64_T) g = fmaf(__ldg(P.invg + j), v[j], g);
         for (int o = 16; o > 0; o >>= 1) g += __shfl_xor_sync(0xffffffffu, g, o);
-        if ((t & 31) == 0) s.part32[t >> 5] = g;
-        __syncthreads();
+        if (lane == 0) s.part32[warp] = g;
+      }
+      __syncthreads();
+      if (kappa != 0.f) {
         for (int k = 0; k < C64_T / 32; ++k) shift += s.part32[k];
         shift *= kappa;
       }
-      __syncthreads();
-      const double* u = product32(v, shift);
-      for (int j = t; j < n; j += C64_T) x[j] = fma(u[j], up, x[j]);
-      __syncthreads();
-    };
-    last = rr;
-    done = converged(rr);
-    bool slow = false;
-    while (!done && !slow && ok && it < P.maxiter) {
-      correct(last);
-      if (!ok) break;
-      const double* y = product(x);
-      if (!ok) break;
-      double tr = 0.0;
-      for (int j = t; j < n; j += C64_T) {
-        const double rj = P.b[j] - y[j];
-        r[j] = rj;
-        tr = fma(rj, rj, tr);
+      // rows of P v, each a warp's (the last warp takes its CTA's part of the norms first)
+      if (warp == LAST) {
+        double a = 0.0, b = 0.0;
+        for (int i = lane; i < nr; i += 32) {
+          a = fma(r[r0 + i], r[r0 + i], a);
+          if (round == 0) b = fma(P.b[r0 + i], P.b[r0 + i], b);
+        }
+        a = warp_sum(a);
+        send(tot, gs, 2 * rank, a, lane, 32);
+        if (round == 0) {
+          b = warp_sum(b);
+          send(tot, gs, 2 * rank + 1, b, lane, 32);
+        }
       }
-      block_sums(tr, 0.0, false, n, s, [](double, double) {});
-      ++it;
-      const double now = s.a;
-      done = converged(now);
-      slow = !(now <= 0.0625 * last);
-      if (slow && !done && !(now <= rr)) {  // no better than the start: the CG begins there
-        for (int j = t; j < n; j += C64_T) x[j] = P.x0 ? P.x0[j] : 0.0;
-        __syncthreads();
-        if (P.x0) y = product(x);
-        for (int j = t; j < n; j += C64_T) r[j] = P.x0 ? P.b[j] - y[j] : P.b[j];
-        last = rr;
-      } else {
-        last = now;
+      const float4* v4 = reinterpret_cast<const float4*>(v);
+      const int n4 = A.nv / 4;
+      for (int i = warp; i < nr; i += C64_T / 32) {
+        const float4* row = reinterpret_cast<const float4*>(P.inv + (size_t)(r0 + i) * P.ldi);
+        float a[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int j0 = 0; j0 < n4; j0 += 4 * 32) {  // four 16-byte loads from L2 in flight
+          float4 m[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int j = j0 + 32 * q + lane;
+            m[q] = j < n4 ? __ldg(row + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+          }
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int j = j0 + 32 * q + lane;
+            const float4 f = j < n4 ? v4[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+            a[0] = fmaf(m[q].x, f.x, a[0]);
+            a[1] = fmaf(m[q].y, f.y, a[1]);
+            a[2] = fmaf(m[q].z, f.z, a[2]);
+            a[3] = fmaf(m[q].w, f.w, a[3]);
+          }
+        }
+        float u = (a[0] + a[1]) + (a[2] + a[3]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) u += __shfl_xor_sync(0xffffffffu, u, o);
+        u = kappa != 0.f ? fmaf(shift, __ldg(P.invg + r0 + i), u) : u;
+        const double x0 = x[r0 + i], xi = fma((double)u, up, x0);
+        __syncwarp();  // every lane has read x before it is replaced
+        if (lane == 0) old[i] = x0;
+        send(x, A.gq, r0 + i, xi, lane, 32);
       }
+      barrier();
+      if (!ok) break;
+      gather_x();
     }
-    // The residual that passed is rich in the modes that P gets least right, the
-    // slow ones, and x is further off for it than a CG iterate of that residual:
-    // one correction more (its residual is not formed; steps gained a factor
-    // of four so far)
-    if (done && !slow && last > 0.0) correct(last);
+    if (ok) {
+      done = flags & DONE;
+      last = s.a;
+      bb = s.b;
+    }
+    if (ok && flags & UNDO) {  // the last correction does not count
+      barrier();
+      for (int i = t; i < nr; i += C64_T)
+        send(x, A.gq, r0 + i, flags & RESET ? (P.x0 ? P.x0[r0 + i] : 0.0) : old[i], 0, 1);
+      barrier();
+      gather_x();
+    }
+    if (ok && !done) {
+      const double l = last;
+      set_norm();
+      last = l;
+      par = 1;  // (others may still read the first exchange buffer)
+      const double* y = product(x);
+      for (int j = t; j < n; j += C64_T) r[j] = P.b[j] - y[j];
+    }
+    if (!ok) done = true;
+  } else {
+    start();
+    for (int j = t; j < n; j += C64_T) {
+      bb += P.b[j] * P.b[j];
+      rr += r[j] * r[j];
+    }
+    block_sums(bb, rr, true, n, s, [](double, double) {});
+    bb = s.a;
+    rr = s.b;
+    set_norm();
+    done = bnorm == 0.0;
   }
   double rz = 0.0;
   if (!done) {
@@ -438,7 +538,9 @@ __global__ void __launch_bounds__(C64_T, 1) k_cg64(const CG64Args A) {
     for (int j = t; j < n; j += C64_T) p[j] = fma(beta, p[j], r[j]);
     __syncthreads();
   }
-  double relres = bnorm > 0 ? sqrt(last) / bnorm : 0.0;
+  double relres = 0.0;
+  if (guard || (rank == 0 && t == 0)) relres = bb > 0 ? sqrt(last / bb) : 0.0;
+  if (done) relres = fmin(relres, P.tol);  // (squares were compared)
   __syncthreads();
   if (guard && best < relres) relres = best;  // stopped past the best iterate: P.x holds it
   else
@@ -486,10 +588,11 @@ size_t plan(const CG64Problem& P, bool grid, int G, CG64Args* A) {
   A->R = (n + G - 1) / G;
   A->lpr = lanes_per_row(A->R);
   A->ld = slab_ld(n, A->lpr);
-  const size_t vecs = (size_t)(grid ? 5 : 6) * n * sizeof(double);
+  A->nv = (n + 3) / 4 * 4;
+  const size_t vecs = (size_t)(grid ? 5 : 6) * A->nv * sizeof(double);
   const size_t slab = csr ? (size_t)cg64_csr_slab(P, A->R) * (sizeof(double) + sizeof(int))
                           : (size_t)A->R * A->ld * sizeof(double);
-  A->resident = vecs + slab <= (size_t)C64_MAX_SMEM;
+  A->resident = vecs + slab <= (size_t)(grid ? C64_MAX_GRID : C64_MAX_CLUSTER);
   A->slab_nnz = csr && A->resident ? cg64_csr_slab(P, A->R) : 0;
   return vecs + (A->resident ? slab : 0);
 }
@@ -522,7 +625,7 @@ int run_grid(CG64Args& A, int G, size_t smem, cudaStream_t st) {
 template <bool CSR, bool GRID>
 cudaError_t kernel_attributes() {
   const cudaError_t e = cudaFuncSetAttribute(k_cg64<CSR, GRID>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             C64_MAX_SMEM);
+                                             GRID ? C64_MAX_GRID : C64_MAX_CLUSTER);
   if (e != cudaSuccess || GRID) return e;
   return cudaFuncSetAttribute(k_cg64<CSR, GRID>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
 }
@@ -538,7 +641,7 @@ cudaError_t kernel_attributes() {
 // tiles, one launch per block column (each step reads one copy of the matrix
 // and writes the other), w carried along as a right-hand side.  A pivot that
 // is not positive marks the inverse unusable.  n = 157 / 448 / 696: 5 / 14 / 22
-// launches.
+// launches, 47 / 112 / 191 us.
 // ---------------------------------------------------------------------------
 namespace {
 
@@ -620,100 +723,133 @@ __global__ void k_inv_form_csr(int n, int ld, const int* __restrict__ rowptr, co
     T[(size_t)i * ld + colidx[e]] += (float)(wi * ((double)vhi[e] + (double)vlo[e]));
 }
 
-// M <- M^-1 in place, 256 threads (thread: row t / 8, four columns)
-__device__ __forceinline__ void invert_tile(float (*M)[GJ + 1], float* __restrict__ sc) {
-  const int r = threadIdx.x >> 3, c0 = (threadIdx.x & 7) * 4;
-  for (int s = 0; s < GJ; ++s) {
-    __syncthreads();
-    float p = M[s][s];
-    if (!(p > 0.f) || !(p < 3e38f)) {
-      if (threadIdx.x == 0) sc[0] = 0.f;
-      p = 1.f;
-    }
-    const float ip = 1.f / p, f = M[r][s] * ip;
-    float v[4];
+constexpr int GJL = GJ + 4;  // row stride of a tile in shared memory (16-byte rows)
+
+// M <- M^-1 in place (M symmetric) by the first warp.  A lane holds a column in
+// registers, rotated so that the pivot's row is always the first (a rolled loop:
+// 32 unrolled steps run once each are bound by instruction fetch, 6 us); the
+// pivot column is the pivot row, negative where the pivots are done, and goes
+// through shared memory; the next pivot's row comes first, its reciprocal (with
+// one Newton step) runs beside the other rows.  3.7 us, a chain of latencies; 256
+// threads on the tile in shared memory, two CTA barriers and an IEEE division
+// per pivot, took 8 us.
+__device__ __forceinline__ void invert_tile(float (*M)[GJL], float (*col)[GJ], float* __restrict__ sc) {
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    bool bad = false;
+    float a[GJ];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int c = c0 + q;
-      const float u = c == s ? 1.f : M[s][c];
-      v[q] = r == s ? u * ip : fmaf(-f, u, c == s ? 0.f : M[r][c]);
-    }
-    __syncthreads();
+    for (int r = 0; r < GJ; ++r) a[r] = M[r][lane];
+    float p = __shfl_sync(0xffffffffu, a[0], 0);
+#pragma unroll 1
+    for (int s = 0; s < GJ; ++s) {
+      float* c = col[s & 1];
+      c[(lane - s) & 31] = lane < s ? -a[0] : a[0];
+      const bool mine = lane == s;
+      bad |= !(p > 0.f) || !(p < 3e38f);
+      float ip = __fdividef(1.f, p);
+      ip = fmaf(ip, fmaf(-p, ip, 1.f), ip);
+      const float u = mine ? ip : a[0] * ip;
+      __syncwarp();
 #pragma unroll
-    for (int q = 0; q < 4; ++q) M[r][c0 + q] = v[q];
+      for (int r = 0; r < GJ; r += 4) {
+        const float4 f = *reinterpret_cast<const float4*>(c + r);
+        if (r) a[r - 1] = fmaf(-f.x, u, mine ? 0.f : a[r]);
+        a[r] = fmaf(-f.y, u, mine ? 0.f : a[r + 1]);
+        if (r == 0) p = __shfl_sync(0xffffffffu, a[0], (s + 1) & 31);
+        a[r + 1] = fmaf(-f.z, u, mine ? 0.f : a[r + 2]);
+        a[r + 2] = fmaf(-f.w, u, mine ? 0.f : a[r + 3]);
+      }
+      a[GJ - 1] = u;
+    }
+    if (bad) sc[0] = 0.f;
+#pragma unroll
+    for (int r = 0; r < GJ; ++r) M[r][lane] = a[r];
   }
   __syncthreads();
 }
+
+// acc += sign * (row r of X) Y, four columns from c0
+__device__ __forceinline__ void tile_mm(float4& acc, float sign, const float (*X)[GJL], const float (*Y)[GJL], int r,
+                                        int c0) {
+#pragma unroll
+  for (int e = 0; e < GJ; e += 4) {
+    const float4 x4 = *reinterpret_cast<const float4*>(&X[r][e]);
+    const float x[4] = {sign * x4.x, sign * x4.y, sign * x4.z, sign * x4.w};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float4 y = *reinterpret_cast<const float4*>(&Y[e + q][c0]);
+      acc.x = fmaf(x[q], y.x, acc.x);
+      acc.y = fmaf(x[q], y.y, acc.y);
+      acc.z = fmaf(x[q], y.z, acc.z);
+      acc.w = fmaf(x[q], y.w, acc.w);
+    }
+  }
+}
+
+__device__ __forceinline__ float4& at4(float* p) { return *reinterpret_cast<float4*>(p); }
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 
 __global__ void __launch_bounds__(256) k_inv_diag(int ld, const float* __restrict__ T, float* __restrict__ D,
                                                   float* __restrict__ sc) {
-  __shared__ float M[GJ][GJ + 1];
+  __shared__ __align__(16) float M[GJ][GJL], col[2][GJ];
   const int r = threadIdx.x >> 3, c0 = (threadIdx.x & 7) * 4;
-  for (int q = 0; q < 4; ++q) M[r][c0 + q] = T[(size_t)r * ld + c0 + q];
-  invert_tile(M, sc);
-  for (int q = 0; q < 4; ++q) D[r * GJ + c0 + q] = M[r][c0 + q];
+  at4(&M[r][c0]) = ld4(T + (size_t)r * ld + c0);
+  invert_tile(M, col, sc);
+  at4(D + r * GJ + c0) = at4(&M[r][c0]);
 }
 
 // one block column: B = the matrix after eliminating block k of A (D: the
-// inverse of A's diagonal block k); the CTA of block k + 1 inverts its result
-__global__ void __launch_bounds__(256) k_inv_step(int k, int ld, const float* __restrict__ A, float* __restrict__ B,
-                                                  const float* __restrict__ D, float* __restrict__ Dn,
-                                                  float* __restrict__ sc) {
-  __shared__ float d[GJ][GJ + 1], l[GJ][GJ + 1], u[GJ][GJ + 1], m[GJ][GJ + 1];
-  const int bi = blockIdx.y, bj = blockIdx.x, r = threadIdx.x >> 3, c0 = (threadIdx.x & 7) * 4;
+// inverse of A's diagonal block k); the CTA of block k + 1 (the first, so that
+// the others run beside it) inverts its result
+__global__ void __launch_bounds__(256) k_inv_step(int k, int nt, int ld, const float* __restrict__ A,
+                                                  float* __restrict__ B, const float* __restrict__ D,
+                                                  float* __restrict__ Dn, float* __restrict__ sc) {
+  __shared__ __align__(16) float d[GJ][GJL], l[GJ][GJL], u[GJ][GJL], m[GJ][GJL], col[2][GJ];
+  const int next = k + 1 < nt ? (k + 1) * (nt + 1) + k + 1 : 0;
+  const int tile = blockIdx.x == 0 ? next : blockIdx.x == next ? 0 : blockIdx.x;
+  const int bi = tile / (nt + 1), bj = tile - bi * (nt + 1), r = threadIdx.x >> 3, c0 = (threadIdx.x & 7) * 4;
   pdl_wait();
   const size_t at = (size_t)(bi * GJ + r) * ld + bj * GJ + c0;
-  float v[4];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    d[r][c0 + q] = D[r * GJ + c0 + q];
-    l[r][c0 + q] = A[(size_t)(bi * GJ + r) * ld + k * GJ + c0 + q];
-    u[r][c0 + q] = A[(size_t)(k * GJ + r) * ld + bj * GJ + c0 + q];
-    v[q] = bi == k || bj == k ? 0.f : A[at + q];
-  }
+  const bool fresh = bi == k || bj == k;
+  const float4 dv = ld4(D + r * GJ + c0), lv = ld4(A + (size_t)(bi * GJ + r) * ld + k * GJ + c0),
+               uv = ld4(A + (size_t)(k * GJ + r) * ld + bj * GJ + c0);
+  float4 v = fresh ? make_float4(0.f, 0.f, 0.f, 0.f) : ld4(A + at);
+  at4(&d[r][c0]) = dv;
+  at4(&l[r][c0]) = lv;
+  at4(&u[r][c0]) = uv;
   __syncthreads();
   if (bj == k) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      float a = 0.f;
-      for (int e = 0; e < GJ; ++e) a = fmaf(l[r][e], d[e][c0 + q], a);
-      v[q] = bi == k ? d[r][c0 + q] : -a;
-    }
+    if (bi == k) v = dv;
+    else tile_mm(v, -1.f, l, d, r, c0);
+  } else if (bi == k) {
+    tile_mm(v, 1.f, d, u, r, c0);
   } else {
-    float x[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int e = 0; e < GJ; ++e)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) x[q] = fmaf(d[r][e], u[e][c0 + q], x[q]);
-    if (bi == k) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) v[q] = x[q];
-    } else {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) m[r][c0 + q] = x[q];
-      __syncthreads();
-      for (int e = 0; e < GJ; ++e)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) v[q] = fmaf(-l[r][e], m[e][c0 + q], v[q]);
-    }
-  }
-#pragma unroll
-  for (int q = 0; q < 4; ++q) B[at + q] = v[q];
-  if (bi == k + 1 && bj == k + 1 && (k + 2) * GJ <= ld) {
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+    tile_mm(x, 1.f, d, u, r, c0);
+    at4(&m[r][c0]) = x;
     __syncthreads();
-#pragma unroll
-    for (int q = 0; q < 4; ++q) m[r][c0 + q] = v[q];
-    invert_tile(m, sc);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) Dn[r * GJ + c0 + q] = m[r][c0 + q];
+    tile_mm(v, -1.f, l, m, r, c0);
+  }
+  at4(B + at) = v;
+  if (bi == k + 1 && bj == k + 1) {
+    at4(&u[r][c0]) = v;
+    invert_tile(u, col, sc);
+    at4(Dn + r * GJ + c0) = at4(&u[r][c0]);
   }
 }
 
-// kappa of the shift
+// kappa of the shift; g = P^-1 w as one vector
 __global__ void __launch_bounds__(1024) k_inv_kappa(int n, int ld, const float* __restrict__ T,
-                                                    const double* __restrict__ w, float* __restrict__ sc) {
+                                                    const double* __restrict__ w, float* __restrict__ sc,
+                                                    float* __restrict__ g) {
   __shared__ double ra[32];
   double a = 0.0;
-  for (int j = threadIdx.x; j < n; j += blockDim.x) a += (w ? w[j] : 1.0) * (double)T[(size_t)j * ld + ld - GJ];
+  for (int j = threadIdx.x; j < n; j += blockDim.x) {
+    g[j] = T[(size_t)j * ld + ld - GJ];
+    a += (w ? w[j] : 1.0) * (double)g[j];
+  }
   a = warp_sum(a);
   if ((threadIdx.x & 31) == 0) ra[threadIdx.x >> 5] = a;
   __syncthreads();
@@ -754,20 +890,21 @@ int cg64_inverse(CG64Inverse* I, const CG64Problem& P, cudaStream_t st) {
   k_inv_diag<<<1, 256, 0, st>>>(ld, T[0], D[0], sc);
   ILM_CHECK_LAUNCH();
   for (int k = 0; k < nt; ++k)
-    ILM_CHECK_CUDA(launch_pdl(k_inv_step, dim3(nt + 1, nt), dim3(256), st, k, ld, (const float*)T[k & 1], T[(k + 1) & 1],
+    ILM_CHECK_CUDA(launch_pdl(k_inv_step, dim3((nt + 1) * nt), dim3(256), st, k, nt, ld, (const float*)T[k & 1], T[(k + 1) & 1],
                               (const float*)D[k & 1], D[(k + 1) & 1], sc));
-  k_inv_kappa<<<1, 1024, 0, st>>>(n, ld, T[nt & 1], P.w, sc);
+  k_inv_kappa<<<1, 1024, 0, st>>>(n, ld, T[nt & 1], P.w, sc, reinterpret_cast<float*>(sums));
   ILM_CHECK_LAUNCH();
   I->n = n;
   I->ld = ld;
   I->inv = T[nt & 1];
+  I->g = reinterpret_cast<float*>(sums);
   I->ready = true;
   return ILM_OK;
 }
 
-size_t cg64_scratch_bytes(int n) { return sizeof(CG64State) + 2 * (size_t)n * sizeof(double); }
+size_t cg64_scratch_bytes(int n) { return sizeof(CG64State) + 4 * (size_t)n * sizeof(double); }
 
-bool cg64_fits(int n) { return 5 * (size_t)n * sizeof(double) + 384 <= (size_t)227 * 1024; }
+bool cg64_fits(int n) { return 5 * (size_t)((n + 3) / 4 * 4) * sizeof(double) <= (size_t)C64_MAX_GRID; }
 
 int launch_cg64(const CG64Problem& P, void* scratch, cudaStream_t st, int variant) {
   const int n = P.n;
@@ -786,7 +923,8 @@ int launch_cg64(const CG64Problem& P, void* scratch, cudaStream_t st, int varian
   if (!A.p.timeout) A.p.timeout = &A.state->timeout;
   const long long entries = (long long)n * (csr ? std::min(P.max_row_nnz, n) : n);
   size_t smem = plan(P, false, C64_CLUSTER, &A);
-  if ((variant == 1 || (variant == 0 && entries <= C64_CLUSTER_ENTRIES)) && smem <= (size_t)C64_MAX_SMEM &&
+  const bool few = P.inv ? n <= (csr ? C64_CLUSTER_CSR : C64_CLUSTER_DENSE) : entries <= C64_CLUSTER_ENTRIES;
+  if ((variant == 1 || (variant == 0 && few)) && smem <= (size_t)C64_MAX_CLUSTER &&
       (csr || A.resident)) {
     ILM_CHECK_CUDA((csr ? kernel_attributes<true, false>() : kernel_attributes<false, false>()));
     return csr ? run_cluster<true>(A, smem, st) : run_cluster<false>(A, smem, st);

@@ -87,11 +87,6 @@ __device__ __forceinline__ float2 split64(double v) {
 }
 __device__ __forceinline__ float2 split64(float v) { return make_float2(v, 0.f); }
 
-__device__ __forceinline__ double widen(float x) {
-  const unsigned b = __float_as_uint(x), e = b >> 23 & 0xffu;
-  return e == 0u ? 0.0 : __hiloint2double((int)((b & 0x80000000u) | (e + 896u) << 20 | (b & 0x7fffffu) >> 3), (int)(b << 29));
-}
-
 // stages one value; returns its magnitude bits for the tile's range
 __device__ __forceinline__ unsigned stage_value(double v, float2 f, double* d, float2* s) {
   *d = v;

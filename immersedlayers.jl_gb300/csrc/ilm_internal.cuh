@@ -441,6 +441,13 @@ __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
   e = (a - (s - v)) + (b - v);
 }
 
+// (double)x by integer operations (a conversion takes a slot of the FP64 unit);
+// finite x, those below 2^-126 go to zero
+__device__ __forceinline__ double widen(float x) {
+  const unsigned b = __float_as_uint(x), e = b >> 23 & 0xffu;
+  return e == 0u ? 0.0 : __hiloint2double((int)((b & 0x80000000u) | (e + 896u) << 20 | (b & 0x7fffffu) >> 3), (int)(b << 29));
+}
+
 // acc += S * (p_hi + p_lo) with S = s_hi + s_lo
 __device__ __forceinline__ void ff_fma(FF& acc, float s_hi, float s_lo, float p_hi, float p_lo) {
   const float ph = s_hi * p_hi;
@@ -513,7 +520,8 @@ struct CG64Problem {
   int* timeout = nullptr;          // set to 1 if the grid variant's wait ran out (null: in CG64State)
   // optional FP32 inverse of W S (cg64_inverse): refined with FP64 residuals
   // before, and usually instead of, the CG
-  const float* inv = nullptr;      // row stride ldi; column ldi - 32 holds the shift's vector
+  const float* inv = nullptr;      // row stride ldi
+  const float* invg = nullptr;     // the shift's vector
   const float* invs = nullptr;     // its scalars
   int ldi = 0;
 };
@@ -523,9 +531,10 @@ struct CG64Inverse {
   DevBuf a, b, s;
   int n = 0, ld = 0;
   bool ready = false;              // formed for the current S
-  const float* inv = nullptr;
+  const float *inv = nullptr, *g = nullptr;
   void attach(CG64Problem* P) const {
     P->inv = inv;
+    P->invg = g;
     P->invs = s.as<float>();
     P->ldi = ld;
   }
