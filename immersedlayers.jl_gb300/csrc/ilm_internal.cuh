@@ -569,7 +569,8 @@ struct ilm_cache_s {
   std::vector<double> hwx[2], hwy[2];  // host copies of the window weights
   ilm::TileList tiles[4];
   ilm::DevBuf x64, y64;                // FP64 point coordinates (device; set by a re-binning)
-  ilm::DevBuf rebin_cnt, rebin_cur;    // re-binning scratch (int per tile)
+  ilm::DevBuf rebin_cnt, rebin_cur;    // re-binning scratch (int per tile and class)
+  ilm::DevBuf schur_F;                 // functionals of the point-pair sums
   bool host_stale = false;             // host copies behind the device after ilm_cache_update_points
   // inverse Laplacian plans per position class
   ilm::ConvPlan conv[4];

@@ -12,9 +12,9 @@
 // and since L^{-1} is the exact linear convolution with G,
 //     (U L^{-1} V^T)_{kl} = (1/factor) sum_{a,b} U_k(a) G(a-b) V_l(b)
 //                         = (1/factor) sum_{dx,dy} Cx(dx) Cy(dy) G(D + (dx,dy)),
-// with Cx, Cy the 1-D correlations of the two stencils (9 values each) and D the
-// offset of the stencil bases.  This is O(N^2 * 81) FP64 work instead of
-// O(N * P^2 log P), and gives the same matrix (up to FP64 rounding) provided
+// with Cx, Cy the 1-D correlations of the two stencils (7 to 9 values each) and D
+// the offset of the stencil bases.  This is O(N^2 * 49) to O(N^2 * 288) FP64 work
+// instead of O(N * P^2 log P), and gives the same matrix (up to FP64 rounding) provided
 // every stencil stays clear of the grid's ghost layer.
 //
 // The solve (ilm_cg64.cu) is CG in the ds-weighted inner product (the matrices
@@ -23,6 +23,7 @@
 // Dirichlet problem, indefinite (one negative eigenvalue) systems.
 // Convergence is declared on the FP64 residual ||b - A x||_2 <= tol ||b||_2.
 #include <math.h>
+#include <stddef.h>
 
 #include <algorithm>
 
@@ -45,13 +46,14 @@ struct Functional {
 // FP64 subtraction, which GB300 issues at a small fraction of its FP32 rate;
 // split per point pair it was a large part of the build).  Written over the
 // Functional buffers, so it is no larger.
-struct FunctionalFF {
+struct alignas(8) FunctionalFF {
   float coef[2][2];
   float w[2];                  // the point's regularization weight ds (hi, lo)
-  short xb[2], yb[2], nterm, pad_;  // grid base indices (|index| < 32768)
+  short xb[2], yb[2], nterm, pad_[3];  // grid base indices (|index| < 32768)
   float xw[2][FW][2], yw[2][FW][2];
 };
 static_assert(sizeof(FunctionalFF) <= sizeof(Functional), "FunctionalFF overlays Functional buffers");
+static_assert(offsetof(FunctionalFF, xw) % 8 == 0 && offsetof(FunctionalFF, yw) % 8 == 0, "weight pairs are read as float2");
 
 // Build the per-point functionals for one Schur kind.  side 0 = left
 // (interpolation side, no ds weight), side 1 = right (regularization side).
@@ -121,53 +123,95 @@ __global__ void k_functionals(int N, int kind, const int* __restrict__ bxP, cons
   out[k] = F;
 }
 
-// A[k + N l] = sgn * sum_{p,q} cL_kp cR_lq w_l sum_{dx,dy} Cx Cy G(...)
-__global__ void __launch_bounds__(256) k_schur_pairs(int N, const Functional* __restrict__ F,
+// A term's weights have NTAP entries along one axis (both, for plain
+// interpolation) and FW along the other, which holds the difference.  Taken by
+// the short axis of k's term, a pair of terms is one of two shapes (G depends
+// on the distances alone, and is symmetric in them): l short on the same axis,
+// or on the other.
+__device__ __forceinline__ bool short_in_x(int kind, int p) {
+  return kind == ILM_SCHUR_GLINVD ? p == 1 : p == 0;
+}
+
+// tile (ti, tj), ti <= tj, of the upper triangle's tile t in row-major order
+__device__ __forceinline__ void triangle_tile(int t, int nt, int* ti_, int* tj_) {
+  // tile row of triangle index t (FP32 estimate, corrected exactly below)
+  const float tn = 2.0f * nt + 1.0f;
+  int ti = (int)((tn - sqrtf(fmaxf(tn * tn - 8.0f * t, 0.0f))) * 0.5f);
+  auto row0 = [nt](int i) { return i * nt - i * (i - 1) / 2; };  // first triangle tile of tile row i
+  while (ti > 0 && row0(ti) > t) --ti;
+  while (ti + 1 < nt && row0(ti + 1) <= t) ++ti;
+  *ti_ = ti;
+  *tj_ = ti + (t - row0(ti));
+}
+
+// sum_{d1,d2} C1(d1) C2(d2) G(|D1 + d1|, |D2 + d2|) with C1 the correlation of
+// k1 (K1 weights) and l1 (L1), C2 of k2 and l2
+template <int K1, int L1, int K2, int L2>
+__device__ __forceinline__ double term_sum(const double* k1, const double* l1, const double* k2, const double* l2,
+                                           int D1, int D2, const double* __restrict__ G, int ld, int M) {
+  double c1[K1 + L1 - 1], c2[K2 + L2 - 1];
+#pragma unroll
+  for (int d = 0; d < K1 + L1 - 1; ++d) c1[d] = 0.0;
+#pragma unroll
+  for (int d = 0; d < K2 + L2 - 1; ++d) c2[d] = 0.0;
+#pragma unroll
+  for (int t = 0; t < K1; ++t)
+#pragma unroll
+    for (int u = 0; u < L1; ++u) c1[t - u + L1 - 1] = fma(k1[t], l1[u], c1[t - u + L1 - 1]);
+#pragma unroll
+  for (int t = 0; t < K2; ++t)
+#pragma unroll
+    for (int u = 0; u < L2; ++u) c2[t - u + L2 - 1] = fma(k2[t], l2[u], c2[t - u + L2 - 1]);
+  D1 -= L1 - 1;
+  D2 -= L2 - 1;
+  double acc = 0.0;
+#pragma unroll
+  for (int d1 = 0; d1 < K1 + L1 - 1; ++d1) {
+    const double* row = G + (size_t)min(abs(D1 + d1), M) * ld;
+    double part = 0.0;
+#pragma unroll
+    for (int d2 = 0; d2 < K2 + L2 - 1; ++d2) part = fma(c2[d2], __ldg(row + min(abs(D2 + d2), M)), part);
+    acc = fma(c1[d1], part, acc);
+  }
+  return acc;
+}
+
+// A[k + N l] = sgn w_l T_kl, T_kl = sum_{p,q} c_kp c_lq sum_{dx,dy} Cx Cy G(...).
+// T is symmetric (both sides have the same functionals): a CTA per 16 x 16 tile
+// of its upper triangle writes both entries.  Bound by the FP64 rate: 88 FMAs
+// per pair for plain interpolation, 450 with two terms.  All pairs with 5 x 5
+// weights (140 and 560) took 148 us for 696 points, one term; this 46.
+template <bool PLAIN>
+__global__ void __launch_bounds__(256) k_schur_pairs(int N, int kind, const Functional* __restrict__ F,
                                                      const double* __restrict__ w, const double* __restrict__ G,
                                                      int ld, int M, double sgn, double* __restrict__ A) {
-  const int k = blockIdx.y * 16 + threadIdx.y;
-  const int l = blockIdx.x * 16 + threadIdx.x;
+  int ti, tj;
+  triangle_tile(blockIdx.x, (N + 15) / 16, &ti, &tj);
+  const int k = ti * 16 + threadIdx.y, l = tj * 16 + threadIdx.x;
   if (k >= N || l >= N) return;
   const Functional& Fk = F[k];
   const Functional& Fl = F[l];
   double total = 0.0;
-  for (int p = 0; p < Fk.nterm; ++p) {
-    for (int q = 0; q < Fl.nterm; ++q) {
-      double cx[2 * FW - 1], cy[2 * FW - 1];
-#pragma unroll
-      for (int d = 0; d < 2 * FW - 1; ++d) {
-        cx[d] = 0.0;
-        cy[d] = 0.0;
+  if (PLAIN) {
+    total = term_sum<NTAP, NTAP, NTAP, NTAP>(Fk.xw[0], Fl.xw[0], Fk.yw[0], Fl.yw[0], Fk.xb[0] - Fl.xb[0],
+                                             Fk.yb[0] - Fl.yb[0], G, ld, M);
+  } else {
+#pragma unroll 1
+    for (int p = 0; p < 2; ++p)
+#pragma unroll 1
+      for (int q = 0; q < 2; ++q) {
+        const bool sx = short_in_x(kind, p);
+        const double *k1 = sx ? Fk.xw[p] : Fk.yw[p], *k2 = sx ? Fk.yw[p] : Fk.xw[p];
+        const double *l1 = sx ? Fl.xw[q] : Fl.yw[q], *l2 = sx ? Fl.yw[q] : Fl.xw[q];
+        const int dx = Fk.xb[p] - Fl.xb[q], dy = Fk.yb[p] - Fl.yb[q];
+        const int D1 = sx ? dx : dy, D2 = sx ? dy : dx;
+        const double acc = p == q ? term_sum<NTAP, NTAP, FW, FW>(k1, l1, k2, l2, D1, D2, G, ld, M)
+                                  : term_sum<NTAP, FW, FW, NTAP>(k1, l1, k2, l2, D1, D2, G, ld, M);
+        total = fma(Fk.coef[p] * Fl.coef[q], acc, total);
       }
-#pragma unroll
-      for (int t = 0; t < FW; ++t) {
-#pragma unroll
-        for (int u = 0; u < FW; ++u) {
-          cx[t - u + FW - 1] += Fk.xw[p][t] * Fl.xw[q][u];
-          cy[t - u + FW - 1] += Fk.yw[p][t] * Fl.yw[q][u];
-        }
-      }
-      const int Dx = Fk.xb[p] - Fl.xb[q] - (FW - 1);
-      const int Dy = Fk.yb[p] - Fl.yb[q] - (FW - 1);
-      double acc = 0.0;
-#pragma unroll
-      for (int dy = 0; dy < 2 * FW - 1; ++dy) {
-        int my = abs(Dy + dy);
-        my = my > M ? M : my;
-        const double* Grow = G + (size_t)my;
-        double racc = 0.0;
-#pragma unroll
-        for (int dx = 0; dx < 2 * FW - 1; ++dx) {
-          int mx = abs(Dx + dx);
-          mx = mx > M ? M : mx;
-          racc += cx[dx] * __ldg(Grow + (size_t)mx * ld);
-        }
-        acc += cy[dy] * racc;
-      }
-      total += Fk.coef[p] * Fl.coef[q] * acc;
-    }
   }
-  A[(size_t)l * N + k] = sgn * w[l] * total;
+  A[(size_t)l * N + k] = sgn * (w ? w[l] : 1.0) * total;
+  if (ti != tj) A[(size_t)k * N + l] = sgn * (w ? w[k] : 1.0) * total;
 }
 
 // nRTRn: A[k + N l] = scale * w_l * (nx_k nx_l <phiU_k,phiU_l> + ny_k ny_l <phiV_k,phiV_l>)
@@ -223,28 +267,22 @@ int schur_build(ilm_cache_s* c, int which, double scale, double* A, cudaStream_t
   int ld = 0;
   const int M = std::max(g.nx, g.ny) + 16;
   ILM_TRY(lgf_table_device(M, &G, &ld, st));
-  DevBuf F, W;
-  ILM_TRY(F.alloc((size_t)N * sizeof(Functional)));
-  ILM_TRY(W.alloc((size_t)N * sizeof(double)));
+  DevBuf& F = c->schur_F;
+  if (F.bytes < (size_t)N * sizeof(Functional)) ILM_TRY(F.alloc((size_t)N * sizeof(Functional)));
   const double invh = c->scaling == ILM_GRID_SCALING ? 1.0 / g.h : 1.0;
   // w_l = regularization weight / factor : GridScaling ds_l/h^2 * h^2 = ds_l
-  const double h2 = g.h * g.h;
-  (void)h2;
   k_functionals<<<(N + 127) / 128, 128, 0, st>>>(N, which, c->bx[0].as<int>(), c->bx[1].as<int>(), c->by[0].as<int>(),
                                                  c->by[1].as<int>(), c->wx64[0].as<double>(), c->wx64[1].as<double>(),
                                                  c->wy64[0].as<double>(), c->wy64[1].as<double>(),
                                                  c->nx64.as<double>(), c->ny64.as<double>(), invh, F.as<Functional>());
   ILM_CHECK_LAUNCH();
-  if (c->scaling == ILM_GRID_SCALING) {
-    ILM_CHECK_CUDA(cudaMemcpyAsync(W.p, c->ds64.p, N * sizeof(double), cudaMemcpyDeviceToDevice, st));
-  } else {
-    ILM_TRY(st_fill(N, ILM_F64, 1.0, W.p, st));
-  }
   // RTLinvR: -scale ; CLinvCT: -scale ; GLinvD: +scale (G_s = -D_s^T)
   const double sgn = (which == ILM_SCHUR_GLINVD) ? scale : -scale;
-  k_schur_pairs<<<grd, blk, 0, st>>>(N, F.as<Functional>(), W.as<double>(), G, ld, ld - 1, sgn, A);
+  const double* w = c->scaling == ILM_GRID_SCALING ? c->ds64.as<double>() : nullptr;
+  const int nt = (N + 15) / 16;
+  (which == ILM_SCHUR_RTLINVR ? k_schur_pairs<true> : k_schur_pairs<false>)<<<nt * (nt + 1) / 2, blk, 0, st>>>(
+      N, which, F.as<Functional>(), w, G, ld, ld - 1, sgn, A);
   ILM_CHECK_LAUNCH();
-  ILM_CHECK_CUDA(cudaStreamSynchronize(st));
   return ILM_OK;
 }
 
@@ -323,7 +361,7 @@ __global__ void k_functionals_batched(int Ptot, const int* __restrict__ pt2prob,
   }
   FunctionalFF Q;
   Q.nterm = (short)F.nterm;
-  Q.pad_ = 0;
+  Q.pad_[0] = Q.pad_[1] = Q.pad_[2] = 0;
   {
     const double wk = w ? w[g] : 0.0;
     const float wh = (float)wk;
@@ -413,6 +451,109 @@ __device__ __forceinline__ FF pair_sum(const FunctionalFF& Fk, const FunctionalF
   return ff_renorm(total.hi, total.lo);
 }
 
+// The LGF as the pairs of one tile read it: the patch of distances that the
+// tile needs in shared memory where it fits (a few thousand entries for points
+// that follow a curve), else the table.  Read from the table by every pair,
+// the gathers took two thirds of the load / store pipe; with the patch, the
+// short axes' four weights and a rolled loop (the unrolled one waited for its
+// instructions) the two-term tiles of 64 problems go from 386
+// to 300 us, bound by the float-float issue rate.
+constexpr int PATCH = 5888;  // entries (46 KB: three CTAs per SM)
+constexpr int FFN = sizeof(FunctionalFF) / 4, FFW = (FFN + 3) / 4 * 4 + 2;  // words of a functional, and its stride
+static_assert(sizeof(FunctionalFF) % 4 == 0 && (FFW / 2) % 2 == 1, "16 functionals' pairs lie in distinct banks");
+constexpr size_t PAIR_SMEM = 32 * FFW * sizeof(float) + (PATCH + 256 * (2 * FW - 1)) * sizeof(float2);
+
+struct GPatch {
+  const float2* G;
+  int ld, M;
+  const float2* patch;
+  int ldp, x0, y0;
+};
+
+// as term_sum, in float-float; the first axis is x (XF) or y
+template <bool SMEM, int K1, int L1, int K2, int L2>
+__device__ __forceinline__ FF term_sum_ff(const float (*k1)[2], const float (*l1)[2], const float (*k2)[2],
+                                          const float (*l2)[2], int D1, int D2, bool xf, const GPatch& g,
+                                          float2* col) {
+  FF c1[K1 + L1 - 1], c2[K2 + L2 - 1];
+#pragma unroll
+  for (int d = 0; d < K1 + L1 - 1; ++d) c1[d] = FF{0.f, 0.f};
+#pragma unroll
+  for (int d = 0; d < K2 + L2 - 1; ++d) c2[d] = FF{0.f, 0.f};
+#pragma unroll
+  for (int u = 0; u < L1; ++u) {
+    const float2 b = *reinterpret_cast<const float2*>(l1[u]);
+#pragma unroll
+    for (int t = 0; t < K1; ++t) ff_fma(c1[t - u + L1 - 1], k1[t][0], k1[t][1], b.x, b.y);
+  }
+#pragma unroll
+  for (int u = 0; u < L2; ++u) {
+    const float2 b = *reinterpret_cast<const float2*>(l2[u]);
+#pragma unroll
+    for (int t = 0; t < K2; ++t) ff_fma(c2[t - u + L2 - 1], k2[t][0], k2[t][1], b.x, b.y);
+  }
+#pragma unroll
+  for (int d = 0; d < K1 + L1 - 1; ++d) {
+    c1[d] = ff_renorm(c1[d].hi, c1[d].lo);
+    col[d * 256] = make_float2(c1[d].hi, c1[d].lo);
+  }
+#pragma unroll
+  for (int d = 0; d < K2 + L2 - 1; ++d) c2[d] = ff_renorm(c2[d].hi, c2[d].lo);
+  D1 -= L1 - 1;
+  D2 -= L2 - 1;
+  const int st1 = SMEM ? (xf ? g.ldp : 1) : (xf ? g.ld : 1), st2 = SMEM ? (xf ? 1 : g.ldp) : (xf ? 1 : g.ld);
+  const int o1 = SMEM ? (xf ? g.x0 : g.y0) : 0, o2 = SMEM ? (xf ? g.y0 : g.x0) : 0;
+  int at2[K2 + L2 - 1];
+#pragma unroll
+  for (int d = 0; d < K2 + L2 - 1; ++d) {
+    const int m = abs(D2 + d);
+    at2[d] = ((SMEM ? m : min(m, g.M)) - o2) * st2;
+  }
+  FF acc{0.f, 0.f};
+#pragma unroll 1
+  for (int d1 = 0; d1 < K1 + L1 - 1; ++d1) {
+    const int m = abs(D1 + d1);
+    const float2 w1 = col[d1 * 256];
+    const float2* row = (SMEM ? g.patch : g.G) + ((SMEM ? m : min(m, g.M)) - o1) * st1;
+    FF part{0.f, 0.f};
+#pragma unroll
+    for (int d2 = 0; d2 < K2 + L2 - 1; ++d2) {
+      const float2 v = SMEM ? row[at2[d2]] : __ldg(row + at2[d2]);
+      ff_fma(part, v.x, v.y, c2[d2].hi, c2[d2].lo);
+    }
+    part = ff_renorm(part.hi, part.lo);
+    ff_fma(acc, w1.x, w1.y, part.hi, part.lo);
+  }
+  return ff_renorm(acc.hi, acc.lo);
+}
+
+// T_kl of one problem's kind
+template <bool SMEM>
+__device__ __forceinline__ FF schur_pair(int kind, const FunctionalFF& Fk, const FunctionalFF& Fl, const GPatch& g,
+                                         float2* col) {
+  if (kind == ILM_SCHUR_RTLINVR)
+    return term_sum_ff<SMEM, NTAP, NTAP, NTAP, NTAP>(Fk.xw[0], Fl.xw[0], Fk.yw[0], Fl.yw[0], Fk.xb[0] - Fl.xb[0],
+                                                     Fk.yb[0] - Fl.yb[0], true, g, col);
+  FF total{0.f, 0.f};
+#pragma unroll 1
+  for (int p = 0; p < 2; ++p)
+#pragma unroll 1
+    for (int q = 0; q < 2; ++q) {
+      const bool sx = short_in_x(kind, p);
+      const float(*k1)[2] = sx ? Fk.xw[p] : Fk.yw[p];
+      const float(*k2)[2] = sx ? Fk.yw[p] : Fk.xw[p];
+      const float(*l1)[2] = sx ? Fl.xw[q] : Fl.yw[q];
+      const float(*l2)[2] = sx ? Fl.yw[q] : Fl.xw[q];
+      const int dx = Fk.xb[p] - Fl.xb[q], dy = Fk.yb[p] - Fl.yb[q];
+      const int D1 = sx ? dx : dy, D2 = sx ? dy : dx;
+      const FF acc = p == q ? term_sum_ff<SMEM, NTAP, NTAP, FW, FW>(k1, l1, k2, l2, D1, D2, sx, g, col)
+                            : term_sum_ff<SMEM, NTAP, FW, FW, NTAP>(k1, l1, k2, l2, D1, D2, sx, g, col);
+      const FF cc = ff_mul(FF{Fk.coef[p][0], Fk.coef[p][1]}, FF{Fl.coef[q][0], Fl.coef[q][1]});
+      ff_fma(total, cc.hi, cc.lo, acc.hi, acc.lo);
+    }
+  return ff_renorm(total.hi, total.lo);
+}
+
 __global__ void __launch_bounds__(256) k_schur_pairs_batched(int nprob, const SchurProbDev* __restrict__ pr,
                                                              const FunctionalFF* __restrict__ F,
                                                              const double* __restrict__ w,
@@ -431,20 +572,66 @@ __global__ void __launch_bounds__(256) k_schur_pairs_batched(int nprob, const Sc
   // |a - b| only and both sides use the same functionals): one CTA per tile
   // of the upper triangle (ti <= tj) in row-major order, writing S_kl = -w_l
   // T_kl and, off the diagonal tiles, S_lk = -w_k T_kl
-  const int t = u - P.tile0;
-  // tile row of triangle index t (FP32 estimate, corrected exactly below)
-  const float tn = 2.0f * nt + 1.0f;
-  int ti = (int)((tn - sqrtf(fmaxf(tn * tn - 8.0f * t, 0.0f))) * 0.5f);
-  auto row0 = [nt](int i) { return i * nt - i * (i - 1) / 2; };  // first triangle tile of tile row i
-  while (ti > 0 && row0(ti) > t) --ti;
-  while (ti + 1 < nt && row0(ti + 1) <= t) ++ti;
-  const int tj = ti + (t - row0(ti));
+  int ti, tj;
+  triangle_tile(u - P.tile0, nt, &ti, &tj);
   const int k = ti * 16 + threadIdx.y;
   const int l = tj * 16 + threadIdx.x;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  float* sf = reinterpret_cast<float*>(smraw);  // functionals of the tile's 16 + 16 points
+  float2* patch = reinterpret_cast<float2*>(sf + 32 * FFW);
+  float2* col = patch + PATCH + threadIdx.y * 16 + threadIdx.x;  // the thread's first correlation (the loop over it is rolled)
+  __shared__ int s_lo[4], s_hi[4];  // x and y bases of the k points, then of the l points
+  {
+    const int tid = threadIdx.y * 16 + threadIdx.x;
+    if (tid < 4) {
+      s_lo[tid] = 0x7fffffff;
+      s_hi[tid] = -0x7fffffff;
+    }
+    for (int e = tid; e < 32 * FFN; e += 256) {
+      const int i = e / FFN, f = e - i * FFN, g = i < 16 ? ti * 16 + i : tj * 16 + i - 16;
+      if (g < N) sf[i * FFW + f] = reinterpret_cast<const float*>(F + P.poff + g)[f];
+    }
+    __syncthreads();
+    if (tid < 64) {  // (point, term)
+      const int i = tid >> 1, q = tid & 1, g = i < 16 ? ti * 16 + i : tj * 16 + i - 16;
+      const FunctionalFF& f = *reinterpret_cast<const FunctionalFF*>(sf + i * FFW);
+      if (g < N && q < f.nterm) {
+        const int s = i < 16 ? 0 : 2;
+        atomicMin(&s_lo[s], (int)f.xb[q]);
+        atomicMax(&s_hi[s], (int)f.xb[q]);
+        atomicMin(&s_lo[s + 1], (int)f.yb[q]);
+        atomicMax(&s_hi[s + 1], (int)f.yb[q]);
+      }
+    }
+    __syncthreads();
+  }
+  // distances of the tile: [lo, hi] per axis, FW - 1 beyond the bases' on both sides
+  GPatch gp{G, ld, M, nullptr, 0, 0, 0};
+  {
+    int lo[2], hi[2];
+    for (int a = 0; a < 2; ++a) {
+      const int d0 = s_lo[a] - s_hi[2 + a] - (FW - 1), d1 = s_hi[a] - s_lo[2 + a] + (FW - 1);
+      lo[a] = d0 <= 0 && d1 >= 0 ? 0 : min(abs(d0), abs(d1));
+      hi[a] = max(abs(d0), abs(d1));
+    }
+    // (an odd row stride: the lanes' points lie along a curve)
+    const int nx = hi[0] - lo[0] + 1, ny = hi[1] - lo[1] + 1, ldp = ny | 1;
+    if ((long long)nx * ldp <= PATCH && hi[0] <= M && hi[1] <= M) {
+      for (int e = threadIdx.y * 16 + threadIdx.x; e < nx * ny; e += 256) {
+        const int i = e / ny, j = e - i * ny;
+        patch[i * ldp + j] = __ldg(G + (size_t)(lo[0] + i) * ld + lo[1] + j);
+      }
+      gp.patch = patch;
+      gp.ldp = ldp;
+      gp.x0 = lo[0];
+      gp.y0 = lo[1];
+    }
+    __syncthreads();
+  }
   if (k >= N || l >= N) return;
-  const FunctionalFF& Fk = F[P.poff + k];
-  const FunctionalFF& Fl = F[P.poff + l];
-  const FF total = pair_sum(Fk, Fl, G, ld, M);
+  const FunctionalFF& Fk = *reinterpret_cast<const FunctionalFF*>(sf + threadIdx.y * FFW);
+  const FunctionalFF& Fl = *reinterpret_cast<const FunctionalFF*>(sf + (16 + threadIdx.x) * FFW);
+  const FF total = gp.patch ? schur_pair<true>(P.kind, Fk, Fl, gp, col) : schur_pair<false>(P.kind, Fk, Fl, gp, col);
   // row-major float-float pair: S[k][l] = hi + lo
   const FF wl{-Fl.w[0], -Fl.w[1]};
   const FF v = ff_mul(wl, total);
@@ -474,19 +661,20 @@ int schur_build_batched(int nprob, const SchurProbDev* probs_dev, int total_tile
   // (the functionals above index probs_dev by problem, so it stays in
   // problem order)
   const FunctionalFF* FF_ = reinterpret_cast<const FunctionalFF*>(F);
+  ILM_CHECK_CUDA(cudaFuncSetAttribute(k_schur_pairs_batched, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PAIR_SMEM));
   if (!order) {
     if (total_tiles > 0)
-      k_schur_pairs_batched<<<total_tiles, dim3(16, 16), 0, st>>>(nprob, probs_dev, FF_, w, G, ld, ld - 1, Shi, Slo);
+      k_schur_pairs_batched<<<total_tiles, dim3(16, 16), PAIR_SMEM, st>>>(nprob, probs_dev, FF_, w, G, ld, ld - 1, Shi, Slo);
     ILM_CHECK_LAUNCH();
     return ILM_OK;
   }
   if (tiles_first > 0)
-    k_schur_pairs_batched<<<tiles_first, dim3(16, 16), 0, st>>>(nfirst, order, FF_, w, G, ld, ld - 1, Shi, Slo);
+    k_schur_pairs_batched<<<tiles_first, dim3(16, 16), PAIR_SMEM, st>>>(nfirst, order, FF_, w, G, ld, ld - 1, Shi, Slo);
   ILM_CHECK_LAUNCH();
   if (mid) ILM_CHECK_CUDA(cudaEventRecord(mid, st));
   const int tiles_second = total_tiles - tiles_first;
   if (tiles_second > 0)
-    k_schur_pairs_batched<<<tiles_second, dim3(16, 16), 0, st>>>(nprob - nfirst, order + nfirst, FF_, w, G, ld,
+    k_schur_pairs_batched<<<tiles_second, dim3(16, 16), PAIR_SMEM, st>>>(nprob - nfirst, order + nfirst, FF_, w, G, ld,
                                                                  ld - 1, Shi, Slo);
   ILM_CHECK_LAUNCH();
   return ILM_OK;
