@@ -1366,9 +1366,11 @@ void cgff_params_set_band(void* dst, const float* band, int band_k, const int* s
 // reads free of bank conflicts), the pivot reciprocal an FP32 reciprocal and
 // one float-float Newton step (~2^-44), the row swaps undone as a column
 // permutation when the inverse is written.  The pivot search is a warp
-// argmax (ties to the lower row, deterministic).
+// argmax (ties to the lower row, deterministic).  1024 threads: a pivot's update
+// is a chain of latencies for 256 (103 blocks of up to 96 points: 310 us, 214
+// with 1024).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_block_inverse(const BJBlockTask* __restrict__ tasks, double shift) {
+__global__ void __launch_bounds__(1024) k_block_inverse(const BJBlockTask* __restrict__ tasks, double shift) {
   const BJBlockTask T = tasks[blockIdx.x];
   const int sz = T.sz;
   const int ld = sz | 1;  // odd row stride
@@ -1509,7 +1511,7 @@ int launch_block_inverse(const BJBlockTask* tasks_dev, int ntasks, int max_sz, c
     return ILM_ERR_SIZE_LIMIT;
   }
   ILM_CHECK_CUDA(cudaFuncSetAttribute(k_block_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k_block_inverse<<<ntasks, 256, smem, st>>>(tasks_dev, 1e-12);
+  k_block_inverse<<<ntasks, 1024, smem, st>>>(tasks_dev, 1e-12);
   ILM_CHECK_LAUNCH();
   return ILM_OK;
 }
