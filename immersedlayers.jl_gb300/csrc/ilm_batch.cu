@@ -356,12 +356,11 @@ struct ilm_batch_s {
   // FP64 iterative refinement (ilm_batch_solve_refined): an FP64 copy of the
   // pipeline (same problems and points, no Schur matrices of its own) for the
   // accurate Schur right-hand side and the field assembly, and FP64 vectors
-  // CG variant 6 (size split): problems above kSplitN points on the 8-CTA
-  // clusters, the others one CTA each on a second stream, joined by events
+  // CG variant 6 (size split): clusters by problem size on three streams,
+  // joined by events (ensure_split)
   bool split_ready = false;
-  int n_large = 0, n_small = 0, max_small = 0, nctas_small = 0;
-  DevBuf order_large, order_small, counter2;
-  cudaStream_t s2 = nullptr;
+  int n_big = 0, n_large = 0, n_small = 0, max_small = 0, nctas_small = 0, cs_big = 8, cs_small = 1;
+  cudaStream_t s2 = nullptr, s3 = nullptr;
   // lazy set-up of the first solve (block-Jacobi inverses, deflation
   // vectors): its own non-blocking stream, so that it overlaps the solve's
   // stage A, and its scratch allocated before stage A is issued (cudaMalloc
@@ -382,7 +381,7 @@ struct ilm_batch_s {
   cudaEvent_t band_ready = nullptr, coarse_ready = nullptr;
   bool band_check = false;
   DevBuf band_err, coarse_tasks, coarse_tprob, coarse_part, coarse_Einv;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join3 = nullptr;
   ilm_batch_s* twin = nullptr;
   DevBuf ref_in, ref_b, ref_x, ref_r, ref_y, ref_norm, dsoff;
   // host wall-clock of the set-up phases (ilm_batch_setup_times), ms
@@ -416,7 +415,9 @@ struct ilm_batch_s {
     if (gexec) cudaGraphExecDestroy(gexec);
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_join) cudaEventDestroy(ev_join);
+    if (ev_join3) cudaEventDestroy(ev_join3);
     if (s2) cudaStreamDestroy(s2);
+    if (s3) cudaStreamDestroy(s3);
     if (s_setup) cudaStreamDestroy(s_setup);
     for (cudaEvent_t e : {bj_ready, band_ready, coarse_ready})
       if (e) {
@@ -841,40 +842,45 @@ int batch_stage_a(ilm_batch_s* b, const void* fplus, const void* fminus, cudaStr
   return batch_mark(b, st);  // 5: DDF gather (Neumann: with the gradient) + Schur right-hand side
 }
 
-// CG variant 6: the two queues (largest first each), the second stream and
-// its events (built on first use)
-constexpr int kSplitN = 192;
+// CG variant 6: three queues by size (each largest first: slices of the
+// order), the other streams and their events (built on first use).  A batch
+// that leaves CTA slots free gives its largest problems clusters of 16 and the
+// small ones clusters of 4: the longest problem sets the time (64 problems of
+// 24 to 645 points: 645 points, 20 iterations of 40 us on 8 CTAs, and 161
+// points, 13 of 50 us on one).  With more problems than slots, 8 CTAs and one
+// CTA do more work per slot.
+constexpr int kSplitN = 192, kSplitBig = 384;
 int ensure_split(ilm_batch_s* b) {
   if (b->split_ready) return ILM_OK;
-  std::vector<int> ord(b->nprob), large, small;
-  for (int p = 0; p < b->nprob; ++p) ord[p] = p;
-  std::stable_sort(ord.begin(), ord.end(), [&](int a, int c) { return b->probs[a].npts > b->probs[c].npts; });
-  int max_small = 0;
-  for (int p : ord) {
-    if (b->probs[p].npts > kSplitN) {
-      large.push_back(p);
-    } else {
-      small.push_back(p);
-      max_small = std::max(max_small, b->probs[p].npts);
-    }
+  int n_big = 0, n_large = 0, max_small = 0;
+  for (int p = 0; p < b->nprob; ++p) {
+    const int n = b->probs[p].npts;
+    n_big += n > kSplitBig;
+    n_large += n > kSplitN;
+    if (n <= kSplitN) max_small = std::max(max_small, n);
   }
-  ILM_TRY(up(b->order_large, large));
-  ILM_TRY(up(b->order_small, small));
-  ILM_TRY(b->counter2.alloc(sizeof(int)));
-  if (!b->s2) ILM_CHECK_CUDA(cudaStreamCreateWithFlags(&b->s2, cudaStreamNonBlocking));
+  for (cudaStream_t* s : {&b->s2, &b->s3})
+    if (!*s) ILM_CHECK_CUDA(cudaStreamCreateWithFlags(s, cudaStreamNonBlocking));
   // timing-enabled fork / join events: with cudaEventDisableTiming the two
   // launches of the split measured as if serialised on GB300 (2.77 against
   // 2.44 ms per batched solve of the bench configuration, CUDA events around
   // whole solves; the same 2.44 ms with timing-enabled events recorded
   // between the stages, which is how the difference was found)
-  if (!b->ev_fork) ILM_CHECK_CUDA(cudaEventCreate(&b->ev_fork));
-  if (!b->ev_join) ILM_CHECK_CUDA(cudaEventCreate(&b->ev_join));
-  b->n_large = (int)large.size();
-  b->n_small = (int)small.size();
+  for (cudaEvent_t* e : {&b->ev_fork, &b->ev_join, &b->ev_join3})
+    if (!*e) ILM_CHECK_CUDA(cudaEventCreate(e));
+  const int n_small = b->nprob - n_large, n_mid = n_large - n_big;
+  const int slots = cg_cta_slots(b->maxN, 8);
+  b->cs_big = 16 * n_big + 8 * n_mid + n_small <= slots ? 16 : 8;
+  b->cs_small = b->cs_big * n_big + 8 * n_mid + 4 * n_small <= slots ? 4 : 1;
+  if (b->cs_big == 8) n_big = 0;  // one queue of clusters of 8
+  b->n_big = n_big;
+  b->n_large = n_large;
+  b->n_small = n_small;
   b->max_small = max_small;
   // the CTA slots the large problems' clusters leave free (at least 8)
-  const int slots = small.empty() ? 0 : cg_single_slots(max_small);
-  b->nctas_small = std::max(8, std::min(b->n_small, slots - 8 * cg_cluster_count(b->nprob, b->maxN, 1)));
+  b->nctas_small = b->cs_small == 4 ? n_small
+                                    : std::max(8, std::min(n_small, (n_small ? cg_single_slots(max_small) : 0) -
+                                                                        8 * std::min(n_large, b->nclusters)));
   b->split_ready = true;
   return ILM_OK;
 }
@@ -885,16 +891,31 @@ int batch_cg(ilm_batch_s* b, cudaStream_t st) {
   ILM_TRY(wait_precond(b, st));
   if (b->cg_variant == 6 || b->cg_variant == 0) {  // the default is the size split
     ILM_TRY(ensure_split(b));
-    if (b->n_small > 0 && b->n_large > 0) {
+    if ((b->n_small > 0 && b->n_large > 0) || b->n_big > 0) {
+      int* const counter = b->counter.as<int>();
+      const int* const order = b->order.as<int>();
+      const int n_mid = b->n_large - b->n_big;
       ILM_CHECK_CUDA(cudaEventRecord(b->ev_fork, st));
-      ILM_CHECK_CUDA(cudaStreamWaitEvent(b->s2, b->ev_fork, 0));
-      ILM_TRY(launch_cg_cluster(b->cgp.p, b->order_large.as<int>(), b->n_large, b->counter.as<int>(), b->maxN,
-                                b->nclusters, st, 1));
-      ILM_TRY(launch_cg_single(b->cgp.p, b->order_small.as<int>(), b->n_small, b->counter2.as<int>(), b->max_small,
-                               b->nctas_small, b->s2));
-      ILM_CHECK_CUDA(cudaEventRecord(b->ev_join, b->s2));
-      ILM_CHECK_CUDA(cudaStreamWaitEvent(st, b->ev_join, 0));
-      b->launches += 2;
+      if (b->n_big > 0) {
+        ILM_CHECK_CUDA(cudaStreamWaitEvent(b->s3, b->ev_fork, 0));
+        ILM_TRY(launch_cg_sized(b->cgp.p, order, b->n_big, counter + 2, b->maxN, b->n_big, b->cs_big, b->s3));
+        ILM_CHECK_CUDA(cudaEventRecord(b->ev_join3, b->s3));
+        b->launches++;
+      }
+      if (b->n_small > 0) {
+        ILM_CHECK_CUDA(cudaStreamWaitEvent(b->s2, b->ev_fork, 0));
+        ILM_TRY(launch_cg_sized(b->cgp.p, order + b->n_large, b->n_small, counter + 1, b->max_small, b->nctas_small,
+                                b->cs_small, b->s2));
+        ILM_CHECK_CUDA(cudaEventRecord(b->ev_join, b->s2));
+        b->launches++;
+      }
+      if (n_mid > 0) {
+        ILM_TRY(launch_cg_sized(b->cgp.p, order + b->n_big, n_mid, counter, b->maxN, std::min(n_mid, b->nclusters), 8,
+                                st));
+        b->launches++;
+      }
+      if (b->n_big > 0) ILM_CHECK_CUDA(cudaStreamWaitEvent(st, b->ev_join3, 0));
+      if (b->n_small > 0) ILM_CHECK_CUDA(cudaStreamWaitEvent(st, b->ev_join, 0));
       return batch_mark(b, st);  // 6: Schur CG
     }
   }
@@ -1215,7 +1236,7 @@ int batch_create_impl(int nprob, const ilm_batch_problem_t* probs, const double*
     }
     A.add(&B->iters, (size_t)nprob * sizeof(int));
     A.add(&B->relres, (size_t)nprob * sizeof(double));
-    A.add(&B->counter, sizeof(int));
+    A.add(&B->counter, 3 * sizeof(int));
     ILM_TRY(A.commit(B->arena_geom, sg));
     phase("upload points, allocate buffers (one arena)");
     BatchGeomDev G;
@@ -2059,7 +2080,7 @@ int ilm_batch_autotune(ilm_batch_t b, const void* fplus, const void* fminus, voi
   for (int v = 1; v <= ILM_CG_VARIANTS && rc == ILM_OK; ++v) {
     if (ms_per_variant) ms_per_variant[v - 1] = -1.f;
     if (v == 2 && cg_rep_smem(b->maxN) > 200 * 1024) continue;
-    if (v != 2 && cg_variant_smem(b->maxN, v) > 200 * 1024) continue;
+    if (!cg_variant_fits(b->maxN, v)) continue;
     if ((rc = ilm_batch_set_cg_variant(b, v)) != ILM_OK) break;
     if ((rc = ilm_batch_solve(b, fplus, fminus, f_out, s_out, tol, maxiter, stream)) != ILM_OK) {
       // a variant the device refuses to launch (cluster size, shared memory)

@@ -521,68 +521,102 @@ __global__ void __cluster_dims__(CG_CLUSTER, 1, 1) __launch_bounds__(CGR_THREADS
 // Each CTA owns rows [r0, r1) of every vector (FP64 slices of x, r, p, q, z,
 // W, b) and of the matrix.  Vectors that the whole cluster needs (p for the
 // product, r for the preconditioner, x for the true residual) are exchanged
-// as float-float splits: every CTA writes the split of its slice into its own
-// full-length buffer, a cluster barrier publishes it, and every CTA copies the
-// other CTAs' parts through distributed shared memory (FP32 loads; no FP64
-// work over the full length).  Reductions sum per-thread partials in warp 0
-// only and publish one value per CTA; the CG scalars are formed once, by
-// thread 0, and broadcast.  GB300's FP64 issue rate is a small fraction of
-// its FP32 rate, so FP64 work is kept to the owned rows.  Two exchange
-// buffers alternate; between two writes of one buffer lies the barrier of
-// an exchange through the other, so no CTA overwrites rows that another CTA
-// may still be copying.
+// as float-float splits: every CTA writes the split of its slice into every
+// CTA's full-length buffer through distributed shared memory, and the cluster
+// barrier of the reduction that follows publishes it.  Reductions send one value per CTA to
+// every CTA; the CG scalars are formed once, by thread 0, and broadcast.
+// GB300's FP64 issue rate is a small fraction of its FP32 rate, so FP64 work is
+// kept to the owned rows and values are split and joined by integer
+// operations.  Two exchange buffers alternate; between two writes of one buffer
+// lies the barrier of an exchange through the other, so no CTA overwrites rows
+// that another CTA may still be reading.
+//
+// An iteration is a chain of latencies (645 points on 16 CTAs, of 20 us: the
+// product 7, the preconditioner 3, three reductions with their barriers 7): what
+// each phase waits for is kept out of L2 (the problem's record, the blocks of the
+// owned rows, the coarse inverse) or requested together.  Rows of S copied ahead
+// into shared memory by bulk copies did not help (34 against 21 thousand clocks
+// for 81 rows of 645: the float-float products issue, they do not wait).
+// Batches of 5 / 63 / 256 problems, per solve: 616 / 1153 / 1932 us before, 357 /
+// 760 / 1518 now.
 // ---------------------------------------------------------------------------
 
+// Sums over the warp of four float-float values per lane: the halves trade two
+// values each, then one, so that a lane carries one value through the last
+// three steps (6 additions; 20 for four butterflies, as many instructions as
+// the dot products of 160 columns).  Lanes 0, 8, 16, 24 hold values 0 to 3.
+__device__ __forceinline__ FF warp_sum4(const FF (&a)[4]) {
+  const int lane = threadIdx.x & 31;
+  const bool up = lane & 16, up2 = lane & 8;
+  auto swap = [](FF keep, FF give, int o) {
+    FF w;
+    w.hi = __shfl_xor_sync(0xffffffffu, give.hi, o);
+    w.lo = __shfl_xor_sync(0xffffffffu, give.lo, o);
+    return ff_add(keep, w);
+  };
+  const FF b0 = swap(up ? a[2] : a[0], up ? a[0] : a[2], 16), b1 = swap(up ? a[3] : a[1], up ? a[1] : a[3], 16);
+  FF c = swap(up2 ? b1 : b0, up2 ? b0 : b1, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) c = swap(c, c, o);
+  return c;
+}
+
 // rows [r0, r1) of S v as float-float pairs yh/yl[i - r0] (rows with 16-byte
-// alignment)
+// alignment): consecutive rows to a warp, four at a time, 128 columns a step
 __device__ void matvec_rows_ff(const CGFFParams& pr, int n, int r0, int r1, const float* __restrict__ vhi,
                                const float* __restrict__ vlo, float* __restrict__ yh, float* __restrict__ yl) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  const int ld = schur_ld(n), nq = ld >> 2;
+  const int ld = schur_ld(n), nq = ld >> 2, nr = r1 - r0;
   const float4* vh4 = reinterpret_cast<const float4*>(vhi);
   const float4* vl4 = reinterpret_cast<const float4*>(vlo);
-  for (int i = r0 + 2 * warp; i < r1; i += 2 * nwarps) {
-    const bool two = i + 1 < r1;
-    const float4* h0 = reinterpret_cast<const float4*>(pr.Shi + (size_t)i * ld);
-    const float4* l0 = reinterpret_cast<const float4*>(pr.Slo + (size_t)i * ld);
-    const float4* h1 = reinterpret_cast<const float4*>(pr.Shi + (size_t)(two ? i + 1 : i) * ld);
-    const float4* l1 = reinterpret_cast<const float4*>(pr.Slo + (size_t)(two ? i + 1 : i) * ld);
-    FF a{0.f, 0.f}, b{0.f, 0.f};
-    int j = lane;
-    for (; j + 32 < nq; j += 64) {  // eight 16-byte loads in flight per lane
-      const float4 x0 = __ldg(h0 + j), y0 = __ldg(l0 + j), x1 = __ldg(h1 + j), y1 = __ldg(l1 + j);
-      const float4 x2 = __ldg(h0 + j + 32), y2 = __ldg(l0 + j + 32), x3 = __ldg(h1 + j + 32),
-                   y3 = __ldg(l1 + j + 32);
-      ff_fma4(a, x0, y0, vh4[j], vl4[j]);
-      ff_fma4(b, x1, y1, vh4[j], vl4[j]);
-      ff_fma4(a, x2, y2, vh4[j + 32], vl4[j + 32]);
-      ff_fma4(b, x3, y3, vh4[j + 32], vl4[j + 32]);
-    }
-    if (j < nq) {
-      const float4 x0 = __ldg(h0 + j), y0 = __ldg(l0 + j), x1 = __ldg(h1 + j), y1 = __ldg(l1 + j);
-      ff_fma4(a, x0, y0, vh4[j], vl4[j]);
-      ff_fma4(b, x1, y1, vh4[j], vl4[j]);
-    }
+  const int per = (nr + nwarps - 1) / nwarps, i1 = min(nr, (warp + 1) * per);
+  for (int i = warp * per; i < i1; i += 4) {
+    const float4* h = reinterpret_cast<const float4*>(pr.Shi + (size_t)(r0 + i) * ld);
+    const float4* l = reinterpret_cast<const float4*>(pr.Slo + (size_t)(r0 + i) * ld);
+    const int m = i1 - i;
+    FF a[4];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      FF oa, ob;
-      oa.hi = __shfl_down_sync(0xffffffffu, a.hi, o);
-      oa.lo = __shfl_down_sync(0xffffffffu, a.lo, o);
-      ob.hi = __shfl_down_sync(0xffffffffu, b.hi, o);
-      ob.lo = __shfl_down_sync(0xffffffffu, b.lo, o);
-      a = ff_add(a, oa);
-      b = ff_add(b, ob);
-    }
-    if (lane == 0) {
-      yh[i - r0] = a.hi;
-      yl[i - r0] = a.lo;
-      if (two) {
-        yh[i + 1 - r0] = b.hi;
-        yl[i + 1 - r0] = b.lo;
+    for (int u = 0; u < 4; ++u) a[u] = FF{0.f, 0.f};
+    for (int j = lane; j < nq; j += 32) {  // eight 16-byte loads in flight per lane
+      float4 x[4], y[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int o = u < m ? u * nq + j : j;
+        x[u] = __ldg(h + o);
+        y[u] = __ldg(l + o);
       }
+      const float4 p = vh4[j], q = vl4[j];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (u < m) ff_fma4(a[u], x[u], y[u], p, q);
+    }
+    const FF c = warp_sum4(a);
+    if ((lane & 7) == 0 && (lane >> 3) < m) {
+      yh[i + (lane >> 3)] = c.hi;
+      yl[i + (lane >> 3)] = c.lo;
     }
   }
 }
+
+// v = hi + lo by integer operations (a conversion takes a slot of the FP64
+// unit), outside FP32's range by conversions
+__device__ __forceinline__ FF split_ff(double v) {
+  const unsigned h = (unsigned)__double2hiint(v), l = (unsigned)__double2loint(v);
+  const unsigned e = h >> 20 & 0x7ffu, sg = h & 0x80000000u;
+  if (e < 949u || e > 1149u) {
+    if ((h << 1 | l) == 0u) return FF{0.f, 0.f};
+    const float f = (float)v;
+    return FF{f, (float)(v - (double)f)};
+  }
+  const float hi = __uint_as_float(sg | (e - 896u) << 23 | (h & 0xfffffu) << 3 | l >> 29);
+  return ff_renorm(hi, (float)(int)(l & 0x1fffffffu) * __uint_as_float(sg | (e - 948u) << 23));
+}
+__device__ __forceinline__ double widen_any(float x) {
+  const unsigned b = __float_as_uint(x), e = b >> 23 & 0xffu;
+  if (e - 1u < 254u) return widen(x);
+  return b << 1 == 0u ? 0.0 : (double)x;
+}
+__device__ __forceinline__ double join_ff(float hi, float lo) { return widen_any(hi) + widen_any(lo); }
 
 // z[i - r0] = (W^-1 C^T C r)_i for the owned rows (float-float).  u = C r is
 // formed for every point (one thread per point, coefficient rows read from
@@ -642,204 +676,180 @@ __device__ void apply_band_rows(const CGFFParams& pr, int n, int r0, int r1, con
   }
 }
 
-// zh/zl[i - r0] = (M r)_i for the owned rows, block-Jacobi in float-float:
-// one warp per four rows so that four rows' loads are in flight together
-__device__ void apply_bjacobi_rows(const CGFFParams& pr, int r0, int r1, const float* __restrict__ rhi,
-                                   const float* __restrict__ rlo, float* __restrict__ zh, float* __restrict__ zl) {
+// block of an owned row: its first point, its size and the row's place in the
+// inverses (read once per problem; looked up in every application, three
+// dependent loads came before the row's)
+struct BJRow {
+  int s, sz;
+  size_t off;
+};
+
+// zh/zl[i] = (M r) of owned row i, block-Jacobi in float-float: one warp per
+// four rows, the loads of 96 columns of the four in flight together
+__device__ void apply_bjacobi_rows(const CGFFParams& pr, const BJRow* __restrict__ rows, int nr,
+                                   const float* __restrict__ rhi, const float* __restrict__ rlo,
+                                   float* __restrict__ zh, float* __restrict__ zl) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int i0 = r0 + 4 * warp; i0 < r1; i0 += 4 * nw) {
+  const float* __restrict__ bh = pr.binv_hi;
+  const float* __restrict__ bl = pr.binv_lo;
+  for (int i0 = 4 * warp; i0 < nr; i0 += 4 * nw) {
     FF acc[4];
+    BJRow R[4];
+    int most = 0;
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       acc[u] = FF{0.f, 0.f};
-      const int i = i0 + u;
-      if (i < r1) {
-        const int b = pr.blk[i];
-        const int s = pr.bstart[b], sz = pr.bsize[b];
-        const float* __restrict__ rh = pr.binv_hi + pr.boff[b] + (size_t)(i - s) * sz;
-        const float* __restrict__ rl = pr.binv_lo + pr.boff[b] + (size_t)(i - s) * sz;
-        int t = lane;
-        for (; t + 32 < sz; t += 64) {  // two columns per lane per trip, loads first
-          const float h0 = __ldg(rh + t), l0 = __ldg(rl + t), h1 = __ldg(rh + t + 32), l1 = __ldg(rl + t + 32);
-          ff_fma(acc[u], h0, l0, rhi[s + t], rlo[s + t]);
-          ff_fma(acc[u], h1, l1, rhi[s + t + 32], rlo[s + t + 32]);
-        }
-        if (t < sz) ff_fma(acc[u], __ldg(rh + t), __ldg(rl + t), rhi[s + t], rlo[s + t]);
-      }
+      R[u] = i0 + u < nr ? rows[i0 + u] : BJRow{0, 0, 0};
+      most = max(most, R[u].sz);
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        FF other;
-        other.hi = __shfl_down_sync(0xffffffffu, acc[u].hi, o);
-        other.lo = __shfl_down_sync(0xffffffffu, acc[u].lo, o);
-        acc[u] = ff_add(acc[u], other);
-      }
-    }
-    if (lane == 0) {
+    for (int t0 = lane; t0 - lane < most; t0 += 96) {
+      float h[4][3], l[4][3];
 #pragma unroll
       for (int u = 0; u < 4; ++u)
-        if (i0 + u < r1) {
-          zh[i0 + u - r0] = acc[u].hi;
-          zl[i0 + u - r0] = acc[u].lo;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          const int t = t0 + 32 * q;
+          h[u][q] = t < R[u].sz ? __ldg(bh + R[u].off + t) : 0.f;
+          l[u][q] = t < R[u].sz ? __ldg(bl + R[u].off + t) : 0.f;
         }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          const int t = t0 + 32 * q;
+          if (t < R[u].sz) ff_fma(acc[u], h[u][q], l[u][q], rhi[R[u].s + t], rlo[R[u].s + t]);
+        }
+    }
+    const FF c = warp_sum4(acc);
+    if ((lane & 7) == 0 && i0 + (lane >> 3) < nr) {
+      zh[i0 + (lane >> 3)] = c.hi;
+      zl[i0 + (lane >> 3)] = c.lo;
     }
   }
 }
 
-// Cluster-wide sums of K <= 4 values, partials held by threads [0, nact).
-// On return the totals are in v[] of thread 0 only; thread 0 derives what
+// Cluster-wide sums of K values, partials held by threads [0, nact).
+// On return the totals are in v[] of the first warp; thread 0 derives what
 // the other threads need, stores it in the broadcast area and the caller
 // synchronises the CTA before reading it.  Each FP64 partial is split into a
-// float-float pair (hi exact, lo rounded: ~48 bits) and the sums run in FP32
-// float-float arithmetic: GB300 issues FP64 at a small fraction of the FP32
-// rate and a chain of dependent FP64 adds costs far more latency than the
-// same chain of FP32 two-sums.  `red` holds 2 K blockDim floats (K blockDim
-// doubles), `pub` 8 slots of 4 float-float values; the published slot
-// rotates over seven values so that a CTA never overwrites a slot another
-// CTA may still be reading.  K <= CG_RED_K.
+// float-float pair (~48 bits) and the sums run in FP32 float-float
+// arithmetic: GB300 issues FP64 at a small fraction of the FP32 rate and a
+// chain of dependent FP64 adds costs far more latency than the same chain of
+// FP32 two-sums.  A warp sums one value of the CTA and sends it to every CTA
+// (the totals are then formed from shared memory; fetched from the other CTAs
+// after the barrier, they cost 1.7 thousand clocks per two values).  `red`
+// holds 2 K stride floats, `pub` two slots of CS x CG_RED_K float-float values,
+// which alternate: a CTA writes a slot again only after a barrier that the
+// others reach when they have read it.  K <= CG_RED_K.
 template <int K, int CS = CG_CLUSTER>
-__device__ void csum_t0(cg::cluster_group& cl, double (&v)[K], int nact, double* red, double* pub, int& slot) {
+__device__ void csum_t0(cg::cluster_group& cl, double (&v)[K], int nact, int stride, double* red, double* pub,
+                        int& slot) {
   static_assert(K <= CG_RED_K, "too many values in one cluster reduction");
-  constexpr int PS = 2 * CG_RED_K;  // floats per published slot
-  const int t = threadIdx.x, nt = blockDim.x;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nw = blockDim.x >> 5;
   float* rf = reinterpret_cast<float*>(red);
-  float* pf = reinterpret_cast<float*>(pub);
-  nact = min(nact, nt);  // threads beyond hold zero partials (or none)
+  float2* pf = reinterpret_cast<float2*>(pub) + slot * CS * CG_RED_K;  // [value][CTA]
+  nact = min(nact, (int)blockDim.x);  // threads beyond hold zero partials (or none)
   if (t < nact)
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-      const float h = (float)v[k];
-      rf[(2 * k) * nt + t] = h;
-      rf[(2 * k + 1) * nt + t] = (float)(v[k] - (double)h);
+      const FF h = split_ff(v[k]);
+      rf[(2 * k) * stride + t] = h.hi;
+      rf[(2 * k + 1) * stride + t] = h.lo;
     }
   __syncthreads();
-  if (t < 32) {
+  const int rank = (int)cl.block_rank();
+  for (int k = warp; k < K; k += nw) {
+    FF a{0.f, 0.f};
+    for (int i = lane; i < nact; i += 32) a = ff_add(a, FF{rf[(2 * k) * stride + i], rf[(2 * k + 1) * stride + i]});
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      FF a{0.f, 0.f};
-      for (int i = t; i < nact; i += 32) a = ff_add(a, FF{rf[(2 * k) * nt + i], rf[(2 * k + 1) * nt + i]});
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        FF b;
-        b.hi = __shfl_down_sync(0xffffffffu, a.hi, o);
-        b.lo = __shfl_down_sync(0xffffffffu, a.lo, o);
-        a = ff_add(a, b);
-      }
-      if (t == 0) {
-        pf[PS * slot + 2 * k] = a.hi;
-        pf[PS * slot + 2 * k + 1] = a.lo;
-      }
+    for (int o = 16; o > 0; o >>= 1) {
+      FF b;
+      b.hi = __shfl_xor_sync(0xffffffffu, a.hi, o);
+      b.lo = __shfl_xor_sync(0xffffffffu, a.lo, o);
+      a = ff_add(a, b);
     }
+    if (lane < CS) cl.map_shared_rank(pf, lane)[k * CS + rank] = make_float2(a.hi, a.lo);
   }
   cl.sync();
-  if (t < 32) {
-    float rh[K], rl[K];
+  if (warp == 0) {
+    constexpr int PER = 32 / CS, PASS = (K + PER - 1) / PER;  // values per pass
+    FF a[PASS];
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      rh[k] = t < CS ? cl.map_shared_rank(pf, t)[PS * slot + 2 * k] : 0.f;
-      rl[k] = t < CS ? cl.map_shared_rank(pf, t)[PS * slot + 2 * k + 1] : 0.f;
+    for (int q = 0; q < PASS; ++q) {
+      const int e = q * 32 + lane;
+      const float2 w = e < K * CS ? pf[e] : make_float2(0.f, 0.f);
+      a[q] = FF{w.x, w.y};
     }
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      FF a{rh[k], rl[k]};
+    for (int o = CS / 2; o > 0; o >>= 1)
 #pragma unroll
-      for (int o = CS / 2; o > 0; o >>= 1) {
+      for (int q = 0; q < PASS; ++q) {
         FF b;
-        b.hi = __shfl_down_sync(0xffffffffu, a.hi, o);
-        b.lo = __shfl_down_sync(0xffffffffu, a.lo, o);
-        a = ff_add(a, b);
+        b.hi = __shfl_xor_sync(0xffffffffu, a[q].hi, o);
+        b.lo = __shfl_xor_sync(0xffffffffu, a[q].lo, o);
+        a[q] = ff_add(a[q], b);
       }
-      v[k] = (double)a.hi + (double)a.lo;
+#pragma unroll
+    for (int q = 0; q < PASS; ++q) {
+      const double s = join_ff(a[q].hi, a[q].lo);
+#pragma unroll
+      for (int k = q * PER; k < (q + 1) * PER && k < K; ++k) v[k] = __shfl_sync(0xffffffffu, s, (k - q * PER) * CS);
     }
   }
-  slot = slot == 7 ? 1 : slot + 1;
+  slot ^= 1;
 }
 
-// body of local point i under the coarse correction (cnb >= 1)
-__device__ __forceinline__ int coarse_body(const CGFFParams& pr, int i) {
-  int b = 0;
-#pragma unroll
-  for (int k = 1; k < CG_COARSE_MAX; ++k) b += (k < pr.cnb && i >= pr.cstart[k]) ? 1 : 0;
-  return b;
-}
-
-// csum_t0 of v[0, K0) and, with the coarse correction, of the per-body sums
-// sum_{i in body b} w_i r_i of the owned rows; thread 0 then forms the
-// coarse coefficients c = E^-1 Z^T W r into bc[16 + b] (read after the
-// caller's next CTA barrier).
+// csum_t0 of v[0, K0) and, with the coarse correction (cnb > 0), of the
+// per-body sums sum_{i in body b} w_i r_i of the owned rows (body[i]: the body
+// of owned row i); the first warp then forms the coarse coefficients c = E^-1
+// Z^T W r into bc[16 + b] (read after the caller's next CTA barrier).
 template <int K0, int CS>
-__device__ void csum_coarse(cg::cluster_group& cl, const CGFFParams& pr, double (&v)[K0], const double* ws,
-                            const double* rs, int r0, int nr, double* red, double* pub, int& slot, double* bc) {
-  if (pr.cnb <= 0) {
-    csum_t0<K0, CS>(cl, v, nr, red, pub, slot);
+__device__ void csum_coarse(cg::cluster_group& cl, int cnb, const double* Einv, const int* body, double (&v)[K0],
+                            const double* ws, const double* rs, int nr, int stride, double* red, double* pub,
+                            int& slot, double* bc) {
+  if (cnb <= 0) {
+    csum_t0<K0, CS>(cl, v, nr, stride, red, pub, slot);
     return;
   }
+  static_assert(CG_COARSE_MAX == 4, "sixteen lanes hold E^-1");
   double u[K0 + CG_COARSE_MAX];
 #pragma unroll
   for (int k = 0; k < K0; ++k) u[k] = v[k];
 #pragma unroll
   for (int b = 0; b < CG_COARSE_MAX; ++b) u[K0 + b] = 0.0;
   for (int i = threadIdx.x; i < nr; i += blockDim.x) {
-    const int bi = coarse_body(pr, r0 + i);
+    const int bi = body[i];
     const double wr = ws[i] * rs[i];
 #pragma unroll
-    for (int b = 0; b < CG_COARSE_MAX; ++b) u[K0 + b] += b == bi ? wr : 0.0;
+    for (int b = 0; b < CG_COARSE_MAX; ++b)
+      if (b == bi) u[K0 + b] = i < (int)blockDim.x ? wr : u[K0 + b] + wr;
   }
-  csum_t0<K0 + CG_COARSE_MAX, CS>(cl, u, nr, red, pub, slot);
+  csum_t0<K0 + CG_COARSE_MAX, CS>(cl, u, nr, stride, red, pub, slot);
 #pragma unroll
   for (int k = 0; k < K0; ++k) v[k] = u[k];
-  if (threadIdx.x == 0)  // entries of E^-1 beyond the bodies are zero
-#pragma unroll
-    for (int a = 0; a < CG_COARSE_MAX; ++a) {
-      double c = 0.0;
-#pragma unroll
-      for (int b = 0; b < CG_COARSE_MAX; ++b) c += pr.cEinv[a * CG_COARSE_MAX + b] * u[K0 + b];
-      bc[16 + a] = c;
-    }
+  if (threadIdx.x < 32) {  // entries of E^-1 beyond the bodies are zero; lane 4 a + b: E^-1_ab u_b
+    const int lane = threadIdx.x, b = lane & 3;
+    const double ub = b == 0 ? u[K0] : b == 1 ? u[K0 + 1] : b == 2 ? u[K0 + 2] : u[K0 + 3];
+    double c = lane < 16 ? Einv[lane] * ub : 0.0;
+    c += __shfl_xor_sync(0xffffffffu, c, 1);
+    c += __shfl_xor_sync(0xffffffffu, c, 2);
+    if (lane < 16 && b == 0) bc[16 + (lane >> 2)] = c;
+  }
 }
 
-// z_i += c[body(i)] on the owned rows (coarse coefficients in bc[16..])
-__device__ __forceinline__ void add_coarse(const CGFFParams& pr, int r0, int nr, double* zs, const double* bc) {
-  if (pr.cnb <= 0) return;
-  for (int i = threadIdx.x; i < nr; i += blockDim.x) zs[i] += bc[16 + coarse_body(pr, r0 + i)];
-}
-
-// split of the owned slice into the exchange buffer's owned part
-__device__ __forceinline__ void publish_slice(const double* s, int r0, int nr, float* eh, float* el) {
+// the split of the owned slice into every CTA's copy of an exchange buffer
+// (visible there after the next cluster barrier)
+template <int CS>
+__device__ __forceinline__ void publish_slice(cg::cluster_group& cl, const double* s, int r0, int nr, float* eh,
+                                              float* el) {
   for (int i = threadIdx.x; i < nr; i += blockDim.x) {
-    const double v = s[i];
-    const float h = (float)v;
-    eh[r0 + i] = h;
-    el[r0 + i] = (float)(v - (double)h);
-  }
-}
-
-// copy the other CTAs' parts of an exchange buffer (after the barrier that
-// published them)
-__device__ __forceinline__ void gather_parts(cg::cluster_group& cl, float* eh, float* el, int n, int rows, int rank) {
-  // four elements per thread and trip, all remote loads issued before the stores
-  const int nt = blockDim.x;
-  for (int j0 = threadIdx.x; j0 < n; j0 += 4 * nt) {
-    float h[4], l[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int j = j0 + u * nt;
-      const int c = j < n ? j / rows : rank;
-      h[u] = c != rank ? cl.map_shared_rank(eh, c)[j] : 0.f;
-      l[u] = c != rank ? cl.map_shared_rank(el, c)[j] : 0.f;
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int j = j0 + u * nt;
-      if (j < n && j / rows != rank) {
-        eh[j] = h[u];
-        el[j] = l[u];
-      }
+    const FF v = split_ff(s[i]);
+#pragma unroll 1
+    for (int d = 0; d < CS; ++d) {
+      cl.map_shared_rank(eh, d)[r0 + i] = v.hi;
+      cl.map_shared_rank(el, d)[r0 + i] = v.lo;
     }
   }
-  __syncthreads();
 }
 
 // p = v + b p in float-float (b = bh + bl); ~2^-46 relative
@@ -880,11 +890,15 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(NT, MINB)
   const int rank = (int)cl.block_rank();
   const int rmax = (max_n + CS - 1) / CS;
   const int ldm = schur_ld(max_n);
+  __shared__ CGFFParams pr;  // the problem's record
+  __shared__ double cE[CG_COARSE_MAX * CG_COARSE_MAX];
+  __shared__ double s_inv_e;
   extern __shared__ __align__(16) unsigned char smraw[];
-  double* red = reinterpret_cast<double*>(smraw);  // CG_RED_K * threads (2 K floats per thread)
-  double* bc = red + CG_RED_K * NT;                // CG_BC: scalars broadcast by thread 0
-  double* pub = bc + CG_BC;                        // 8 slots x CG_RED_K float-float: published CTA sums
-  double* work = pub + 8 * CG_RED_K;               // 4: [0] queue index taken by rank 0
+  const int stride = min(NT, (rmax + 31) & ~31);   // of the reduction's rows
+  double* red = reinterpret_cast<double*>(smraw);  // CG_RED_K * stride
+  double* bc = red + CG_RED_K * stride;            // CG_BC: scalars broadcast by thread 0
+  double* pub = bc + CG_BC;                        // 2 slots x CS x CG_RED_K float-float: the CTAs' sums
+  double* work = pub + 2 * CS * CG_RED_K;          // 4: [0] queue index taken by rank 0
   double* xs = work + 4;                           // owned slices (rmax each)
   double* rs = xs + rmax;
   double* ps = rs + rmax;
@@ -892,9 +906,12 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(NT, MINB)
   double* zs = qs + rmax;
   double* ws = zs + rmax;
   double* bs = ws + rmax;
+  double* szs = bs + rmax;
+  BJRow* bj = reinterpret_cast<BJRow*>(szs + rmax);
+  int* body = reinterpret_cast<int*>(bj + rmax);
   // float arrays, 16-byte aligned: p (whole), exchange buffers for r (A) and
   // for z / x (B), band intermediate, product rows, staged band and segments
-  float* ph = reinterpret_cast<float*>(bs + rmax + (rmax & 1));
+  float* ph = reinterpret_cast<float*>(body + ((rmax + 3) & ~3));
   float* pl = ph + ldm;
   float* ah = pl + ldm;
   float* al = ah + ldm;
@@ -904,13 +921,15 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(NT, MINB)
   float* ulo = uhi + ldm;
   float* yh = ulo + ldm;  // product rows
   float* yl = yh + rmax;
-  int slot = 1;
+  int slot = 0;
   while (true) {
     if (rank == 0 && threadIdx.x == 0) work[0] = (double)atomicAdd(counter, 1);
     cl.sync();
     const int q = (int)cl.map_shared_rank(work, 0)[0];
     if (q >= nprob) break;
-    const CGFFParams& pr = P[order[q]];  // fields read through L1 as needed
+    for (int e = threadIdx.x; e < (int)(sizeof(CGFFParams) / 4); e += NT)
+      reinterpret_cast<int*>(&pr)[e] = __ldg(reinterpret_cast<const int*>(P + order[q]) + e);
+    __syncthreads();
     if (pr.tspan && rank == 0 && threadIdx.x == 0) {
       pr.tspan[0] = global_ns();
       pr.tspan[2] = sm_id();
@@ -922,10 +941,27 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(NT, MINB)
     const bool sz = pr.sz != nullptr;  // deflation: S 1 read from pr.sz (owned rows from r0)
     // 1 / E (deflation) is read by thread 0 where it forms the scalars
     const bool pre = pr.blk != nullptr || pr.band != nullptr;
+    auto add_coarse = [&]() {  // z_i += c[body(i)] on the owned rows
+      if (pr.cnb > 0)
+        for (int i = threadIdx.x; i < nr; i += blockDim.x) zs[i] += bc[16 + body[i]];
+    };
+    if (pr.cnb > 0 && threadIdx.x < CG_COARSE_MAX * CG_COARSE_MAX) cE[threadIdx.x] = pr.cEinv[threadIdx.x];
+    if (sz && threadIdx.x == 0) s_inv_e = *pr.inv_e;
     for (int i = threadIdx.x; i < nr; i += blockDim.x) {
       xs[i] = 0.0;
       bs[i] = pr.b[r0 + i];
       ws[i] = pr.w ? pr.w[r0 + i] : 1.0;
+      if (sz) szs[i] = pr.sz[r0 + i];
+      if (pr.blk) {
+        const int g = r0 + i, b = pr.blk[g];
+        bj[i].s = pr.bstart[b];
+        bj[i].sz = pr.bsize[b];
+        bj[i].off = (size_t)pr.boff[b] + (size_t)(g - bj[i].s) * bj[i].sz;
+      }
+      int bi = 0;
+#pragma unroll
+      for (int c = 1; c < CG_COARSE_MAX; ++c) bi += c < pr.cnb && r0 + i >= pr.cstart[c] ? 1 : 0;
+      body[i] = bi;
     }
     for (int j = n + threadIdx.x; j < ld; j += blockDim.x) {  // padding of the product's vectors
       ph[j] = pl[j] = bh[j] = bl[j] = 0.f;
@@ -936,13 +972,13 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(NT, MINB)
     if (sz) {  // deflation: x += c 1, r -= c S 1, c = 1^T W r / E (then 1^T W r = 0)
       double v[1] = {0.0};
       for (int i = threadIdx.x; i < nr; i += blockDim.x) v[0] += ws[i] * rs[i];
-      csum_t0<1, CS>(cl, v, nr, red, pub, slot);
-      if (threadIdx.x == 0) bc[0] = v[0] * __ldg(pr.inv_e);
+      csum_t0<1, CS>(cl, v, nr, stride, red, pub, slot);
+      if (threadIdx.x == 0) bc[0] = v[0] * s_inv_e;
       __syncthreads();
       const double c = bc[0];
       for (int i = threadIdx.x; i < nr; i += blockDim.x) {
         xs[i] += c;
-        rs[i] -= c * __ldg(pr.sz + r0 + i);
+        rs[i] -= c * szs[i];
       }
       __syncthreads();
     }
@@ -954,16 +990,16 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(NT, MINB)
       for (int i = threadIdx.x; i < nr; i += blockDim.x) {
         v[0] += bs[i] * bs[i];
         v[1] += ws[i] * rs[i] * rs[i];
-        if (sz) v[2] += ws[i] * __ldg(pr.sz + r0 + i) * rs[i];
+        if (sz) v[2] += ws[i] * szs[i] * rs[i];
       }
-      publish_slice(rs, r0, nr, ah, al);
-      csum_coarse<3, CS>(cl, pr, v, ws, rs, r0, nr, red, pub, slot, bc);
+      publish_slice<CS>(cl, rs, r0, nr, ah, al);
+      csum_coarse<3, CS>(cl, pr.cnb, cE, body, v, ws, rs, nr, stride, red, pub, slot, bc);
       if (threadIdx.x == 0) {
         bc[0] = sqrt(v[0]);
         bc[1] = v[1];
-        bc[2] = sz ? v[2] * __ldg(pr.inv_e) : 0.0;
+        bc[2] = sz ? v[2] * s_inv_e : 0.0;
       }
-      gather_parts(cl, ah, al, n, rows, rank);
+      __syncthreads();
       bnorm = bc[0];
       rz = bc[1];
       mu = bc[2];
@@ -972,19 +1008,19 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(NT, MINB)
       if (pr.band) {
         apply_band_rows(pr, n, r0, r1, ah, al, uhi, ulo, ws, zs);
       } else {
-        apply_bjacobi_rows(pr, r0, r1, ah, al, yh, yl);
+        apply_bjacobi_rows(pr, bj, nr, ah, al, yh, yl);
         __syncthreads();
-        for (int i = threadIdx.x; i < nr; i += blockDim.x) zs[i] = (double)yh[i] + (double)yl[i];
-        add_coarse(pr, r0, nr, zs, bc);
+        for (int i = threadIdx.x; i < nr; i += blockDim.x) zs[i] = join_ff(yh[i], yl[i]);
+        add_coarse();
       }
       __syncthreads();
       double v[1] = {0.0};
       if (sz)
-        for (int i = threadIdx.x; i < nr; i += blockDim.x) v[0] += ws[i] * __ldg(pr.sz + r0 + i) * zs[i];
-      publish_slice(zs, r0, nr, bh, bl);
-      csum_t0<1, CS>(cl, v, nr, red, pub, slot);
-      if (threadIdx.x == 0) bc[2] = sz ? v[0] * __ldg(pr.inv_e) : 0.0;
-      gather_parts(cl, bh, bl, n, rows, rank);
+        for (int i = threadIdx.x; i < nr; i += blockDim.x) v[0] += ws[i] * szs[i] * zs[i];
+      publish_slice<CS>(cl, zs, r0, nr, bh, bl);
+      csum_t0<1, CS>(cl, v, nr, stride, red, pub, slot);
+      if (threadIdx.x == 0) bc[2] = sz ? v[0] * s_inv_e : 0.0;
+      __syncthreads();
       mu = bc[2];
       const float mh = (float)mu, ml = (float)(mu - (double)mh);
       for (int j = threadIdx.x; j < n; j += blockDim.x) {
@@ -1022,14 +1058,14 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(NT, MINB)
       {
         double v[2] = {0.0, 0.0};
         for (int i = threadIdx.x; i < nr; i += blockDim.x) {
-          const double pi = (double)ph[r0 + i] + (double)pl[r0 + i];
-          const double qi = (double)yh[i] + (double)yl[i];
+          const double pi = join_ff(ph[r0 + i], pl[r0 + i]);
+          const double qi = join_ff(yh[i], yl[i]);
           ps[i] = pi;
           qs[i] = qi;
           v[0] += ws[i] * pi * qi;
           v[1] += ws[i] * pi * rs[i];
         }
-        csum_t0<2, CS>(cl, v, nr, red, pub, slot);
+        csum_t0<2, CS>(cl, v, nr, stride, red, pub, slot);
         if (threadIdx.x == 0) {
           bc[3] = v[0];
           bc[4] = v[0] != 0.0 ? fdiv(pre ? v[1] : rz, v[0]) : 0.0;
@@ -1048,14 +1084,14 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(NT, MINB)
           rs[i] = ri;
           v[0] += ri * ri;
           v[1] += ws[i] * ri * ri;
-          if (sz) v[2] += ws[i] * __ldg(pr.sz + r0 + i) * ri;
+          if (sz) v[2] += ws[i] * szs[i] * ri;
         }
-        publish_slice(rs, r0, nr, ah, al);
-        csum_coarse<3, CS>(cl, pr, v, ws, rs, r0, nr, red, pub, slot, bc);
+        publish_slice<CS>(cl, rs, r0, nr, ah, al);
+        csum_coarse<3, CS>(cl, pr.cnb, cE, body, v, ws, rs, nr, stride, red, pub, slot, bc);
         if (threadIdx.x == 0) {
           bc[5] = v[0];
           bc[6] = v[1];
-          bc[7] = sz ? v[2] * __ldg(pr.inv_e) : 0.0;
+          bc[7] = sz ? v[2] * s_inv_e : 0.0;
         }
         __syncthreads();
         rr = bc[5];
@@ -1069,26 +1105,26 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(NT, MINB)
         // is superseded by the refreshed one)
         {
           double v[1] = {0.0};
-          publish_slice(xs, r0, nr, bh, bl);
-          csum_t0<1, CS>(cl, v, nr, red, pub, slot);  // the barrier that publishes x
-          gather_parts(cl, bh, bl, n, rows, rank);
+          publish_slice<CS>(cl, xs, r0, nr, bh, bl);
+          csum_t0<1, CS>(cl, v, nr, stride, red, pub, slot);  // the barrier that publishes x
+          __syncthreads();
           matvec_rows_ff(pr, n, r0, r1, bh, bl, yh, yl);
           __syncthreads();
         }
         double v[3] = {0.0, 0.0, 0.0};
         for (int i = threadIdx.x; i < nr; i += blockDim.x) {
-          const double ri = bs[i] - ((double)yh[i] + (double)yl[i]);
+          const double ri = bs[i] - join_ff(yh[i], yl[i]);
           rs[i] = ri;
           v[0] += ri * ri;
           v[1] += ws[i] * ri * ri;
-          if (sz) v[2] += ws[i] * __ldg(pr.sz + r0 + i) * ri;
+          if (sz) v[2] += ws[i] * szs[i] * ri;
         }
-        publish_slice(rs, r0, nr, ah, al);
-        csum_coarse<3, CS>(cl, pr, v, ws, rs, r0, nr, red, pub, slot, bc);
+        publish_slice<CS>(cl, rs, r0, nr, ah, al);
+        csum_coarse<3, CS>(cl, pr.cnb, cE, body, v, ws, rs, nr, stride, red, pub, slot, bc);
         if (threadIdx.x == 0) {
           bc[9] = v[0];
           bc[10] = v[1];
-          bc[11] = sz ? v[2] * __ldg(pr.inv_e) : 0.0;
+          bc[11] = sz ? v[2] * s_inv_e : 0.0;
         }
         __syncthreads();
         const double tr = bc[9];
@@ -1109,7 +1145,7 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(NT, MINB)
         }
       }
       // r of every CTA (buffer A), published with the reduction above
-      gather_parts(cl, ah, al, n, rows, rank);
+      __syncthreads();
       // with the deflation the new p is projected: p -= ((S 1)^T W p / E) 1,
       // where (S 1)^T W p = (S 1)^T W (r or z) (the old p is S-orthogonal to 1)
       double beta;
@@ -1130,24 +1166,24 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(NT, MINB)
         if (pr.band) {
           apply_band_rows(pr, n, r0, r1, ah, al, uhi, ulo, ws, zs);
         } else {
-          apply_bjacobi_rows(pr, r0, r1, ah, al, yh, yl);
+          apply_bjacobi_rows(pr, bj, nr, ah, al, yh, yl);
           __syncthreads();
-          for (int i = threadIdx.x; i < nr; i += blockDim.x) zs[i] = (double)yh[i] + (double)yl[i];
-          add_coarse(pr, r0, nr, zs, bc);
+          for (int i = threadIdx.x; i < nr; i += blockDim.x) zs[i] = join_ff(yh[i], yl[i]);
+          add_coarse();
         }
         __syncthreads();
         double v[2] = {0.0, 0.0};
         for (int i = threadIdx.x; i < nr; i += blockDim.x) {
           v[0] += ws[i] * zs[i] * qs[i];
-          if (sz) v[1] += ws[i] * __ldg(pr.sz + r0 + i) * zs[i];
+          if (sz) v[1] += ws[i] * szs[i] * zs[i];
         }
-        publish_slice(zs, r0, nr, bh, bl);
-        csum_t0<2, CS>(cl, v, nr, red, pub, slot);
+        publish_slice<CS>(cl, zs, r0, nr, bh, bl);
+        csum_t0<2, CS>(cl, v, nr, stride, red, pub, slot);
         if (threadIdx.x == 0) {
           bc[13] = fdiv(-v[0], pq);
-          bc[14] = sz ? v[1] * __ldg(pr.inv_e) : 0.0;
+          bc[14] = sz ? v[1] * s_inv_e : 0.0;
         }
-        gather_parts(cl, bh, bl, n, rows, rank);
+        __syncthreads();
         beta = bc[13];
         const double muz = bc[14];
         const float bh_ = (float)beta, bl_ = (float)(beta - (double)bh_);
@@ -1180,8 +1216,9 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(NT, MINB)
 size_t cg_cluster_smem(int max_n, int nt, int cs) {
   const size_t rmax = (size_t)(max_n + cs - 1) / cs;
   const size_t ldm = (size_t)schur_ld(max_n);
-  return (CG_RED_K * (size_t)nt + CG_BC + 8 * CG_RED_K + 4 + 7 * rmax + 1) * sizeof(double) +
-         (8 * ldm + 2 * rmax) * sizeof(float) + 64;
+  const size_t stride = std::min<size_t>(nt, (rmax + 31) / 32 * 32);
+  return (CG_RED_K * stride + CG_BC + 2 * (size_t)cs * CG_RED_K + 4 + 8 * rmax) * sizeof(double) + rmax * sizeof(BJRow) +
+         (rmax + 3) / 4 * 4 * sizeof(int) + (8 * ldm + 2 * rmax) * sizeof(float) + 64;
 }
 
 size_t cg_rep_smem(int max_n) {
@@ -1205,9 +1242,19 @@ static bool use_rep(int variant, int max_n) { return variant == 2 && cg_rep_smem
 static int dist_threads(int variant) { return variant == 3 ? 128 : variant == 5 ? 512 : 256; }
 static int dist_cluster(int) { return CG_CLUSTER; }
 
-size_t cg_variant_smem(int max_n, int variant) {
-  return use_rep(variant, max_n) ? cg_rep_smem(max_n)
-                                 : cg_cluster_smem(max_n, dist_threads(variant), dist_cluster(variant));
+// the sizes the row-distributed kernels take
+static bool dist_fits(int max_n, int nt, int cs) {
+  const size_t rmax = (size_t)(max_n + cs - 1) / cs;
+  return (CG_RED_K * (size_t)nt + CG_BC + 8 * CG_RED_K + 5 + 8 * rmax) * sizeof(double) +
+             8 * (size_t)schur_ld(max_n) * sizeof(float) + 64 <=
+         200 * 1024;
+}
+bool cg_variant_fits(int max_n, int variant) {
+  return variant == 2 || dist_fits(max_n, dist_threads(variant), dist_cluster(variant));
+}
+
+static size_t cg_variant_smem(int max_n, int variant) {
+  return use_rep(variant, max_n) ? cg_rep_smem(max_n) : cg_cluster_smem(max_n, dist_threads(variant), dist_cluster(variant));
 }
 
 template <int NT, int MINB, int CS>
@@ -1215,6 +1262,8 @@ static int launch_dist(const CGFFParams* prm, const int* order, int nprob, int* 
                        size_t smem, cudaStream_t st) {
   ILM_CHECK_CUDA(
       cudaFuncSetAttribute(k_cg_cluster<NT, MINB, CS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (CS > 8)
+    ILM_CHECK_CUDA(cudaFuncSetAttribute(k_cg_cluster<NT, MINB, CS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   k_cg_cluster<NT, MINB, CS><<<nclusters * CS, NT, smem, st>>>(prm, order, nprob, counter, max_n);
   ILM_CHECK_LAUNCH();
   return ILM_OK;
@@ -1240,7 +1289,7 @@ int launch_cg_cluster(const void* params_dev, const int* order, int nprob, int* 
     return ILM_OK;
   }
   const size_t smem = cg_variant_smem(max_n, variant);
-  if (smem > 200 * 1024) {
+  if (!dist_fits(max_n, dist_threads(variant), dist_cluster(variant))) {
     set_error("cluster CG: %d unknowns exceed the shared-memory layout of CG variant %d", max_n, variant);
     return ILM_ERR_SIZE_LIMIT;
   }
@@ -1252,19 +1301,32 @@ int launch_cg_cluster(const void* params_dev, const int* order, int nprob, int* 
   }
 }
 
-// One CTA per problem (no cluster): the small problems of a size-split CG
-// launch (batch CG variant 6), run beside the 8-CTA clusters of the large
-// ones in the CTA slots those leave free.
-int launch_cg_single(const void* params_dev, const int* order, int nprob, int* counter, int max_n, int nctas,
-                     cudaStream_t st) {
+// One queue of a size-split CG launch (batch CG variant 6): cs = 1, 4, 8 or 16
+// CTAs per problem
+int launch_cg_sized(const void* params_dev, const int* order, int nprob, int* counter, int max_n, int nclusters, int cs,
+                    cudaStream_t st) {
   const CGFFParams* prm = static_cast<const CGFFParams*>(params_dev);
   ILM_CHECK_CUDA(cudaMemsetAsync(counter, 0, sizeof(int), st));
-  const size_t smem = cg_cluster_smem(max_n, 256, 1);
-  if (smem > 200 * 1024) {
-    set_error("single-CTA CG: %d unknowns exceed its shared-memory layout", max_n);
+  if (!dist_fits(max_n, 256, cs)) {
+    set_error("cluster CG: %d unknowns exceed the shared-memory layout of %d CTAs", max_n, cs);
     return ILM_ERR_SIZE_LIMIT;
   }
-  return launch_dist<256, 3, 1>(prm, order, nprob, counter, max_n, nctas, smem, st);
+  const size_t smem = cg_cluster_smem(max_n, 256, cs);
+  switch (cs) {
+    case 1: return launch_dist<256, 3, 1>(prm, order, nprob, counter, max_n, nclusters, smem, st);
+    case 4: return launch_dist<256, 3, 4>(prm, order, nprob, counter, max_n, nclusters, smem, st);
+    case 16: return launch_dist<256, 3, 16>(prm, order, nprob, counter, max_n, nclusters, smem, st);
+    default: return launch_dist<256, 3, 8>(prm, order, nprob, counter, max_n, nclusters, smem, st);
+  }
+}
+
+// CTAs of the 256-thread kernel that the device holds at a time (three per SM
+// where the shared memory allows)
+int cg_cta_slots(int max_n, int cs) {
+  int dev = 0, nsm = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  return nsm * (int)std::min<size_t>(3, 228 * 1024 / (cg_cluster_smem(max_n, 256, cs) + 2048));
 }
 
 // co-resident CTAs of the single-CTA CG kernel on the whole device
@@ -1273,7 +1335,7 @@ int cg_single_slots(int max_n) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   const size_t smem = cg_cluster_smem(max_n, 256, 1);
-  if (smem > 200 * 1024) return 0;
+  if (!dist_fits(max_n, 256, 1)) return 0;
   if (cudaFuncSetAttribute(k_cg_cluster<256, 3, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
           cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_cg_cluster<256, 3, 1>, 256, smem) != cudaSuccess) {
@@ -1302,7 +1364,7 @@ int cg_cluster_count(int nprob, int max_n, int variant) {
   if (rep) {
     e = cudaFuncSetAttribute(k_cg_rep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&nc, k_cg_rep, &cfg);
-  } else if (smem > 200 * 1024) {
+  } else if (!dist_fits(max_n, nt, cs)) {
     e = cudaErrorInvalidValue;  // the launch refuses this variant; any count will do
   } else {
     switch (variant) {

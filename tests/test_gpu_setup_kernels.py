@@ -59,3 +59,44 @@ def test_batched_pair_sums_match_dense(cuda, kind, sep, nper):
     S = (il.create_RTLinvR if kind == 0 else il.create_CLinvCT)(c)
     torch.cuda.synchronize()
     assert (y - S @ x).abs().max().item() <= 1e-11 * (S.abs() @ x.abs()).max().item()
+
+
+@pytest.mark.parametrize("precond", ["none", "bjacobi"])
+@pytest.mark.parametrize("variant", [1, 3, 6])
+def test_batched_cg_cluster_sizes(cuda, precond, variant):
+    """Problems of each queue of the size split (clusters of 16, 8 and 4 CTAs;
+    row counts that do not divide), with the coarse correction of several
+    bodies: the FP64 residual of every solution meets the tolerance.  The
+    kernel's own true residual is formed in float-float, 2^-44 per operation on
+    |S| |x|: 1e-10 of |b| beside the 1e-9 asked for."""
+    import torch
+    import immersedlayers as il
+    from immersedlayers import bodies as B
+    from immersedlayers.batch import BatchProblemSpec, BatchSolver
+    h = 4.0 / 512
+    specs = []
+    for i, (nb, nper) in enumerate([(1, 5), (1, 33), (3, 47), (2, 97), (1, 193), (3, 129), (2, 201), (1, 401)]):
+        for kind in (0, 1):
+            bl = B.BodyList()
+            for q in range(nb):
+                b = B.circle(nper * 1.4 * h / (2 * np.pi), n=nper)
+                bl.append(B.Body(b.x + 1.1 * (q - 0.5 * (nb - 1)), b.y + 0.2 * q, b.nx, b.ny, b.ds))
+            specs.append(BatchProblemSpec(512, h, bl, kind, np.zeros(len(bl))))
+    bs = BatchSolver(specs, dtype=torch.float32)
+    if precond == "bjacobi":
+        bs.set_precond("bjacobi", 64)
+        bs.set_coarse(True)
+    bs.set_cg_variant(variant)
+    rng = np.random.default_rng(3)
+    rhs = torch.tensor(rng.standard_normal(bs.total_points), dtype=torch.float64, device="cuda")
+    # smooth data: S times a vector
+    rhs = bs.schur_apply(rhs)
+    x = bs.schur_solve(rhs, tol=1e-9, maxiter=20000)
+    r = bs.schur_apply(x) - rhs
+    torch.cuda.synchronize()
+    its, rr = bs.info()
+    assert (rr <= 1e-9).all(), (its, rr)
+    o = bs.point_offsets
+    for i in range(len(specs)):
+        a, b = o[i], o[i + 1]
+        assert r[a:b].norm().item() <= 1.1e-9 * rhs[a:b].norm().item(), (i, its[i])
