@@ -278,6 +278,54 @@ __global__ void k_jump_avg(int n, const T* __restrict__ p, const T* __restrict__
 
 using namespace ilm;
 
+namespace {
+
+// Non-blocking streams, kept for the next object: a set-up uses up to seven and
+// creating one takes some 40 us.  At most kIdleStreams are kept (each on the device it
+// was made on); one that is given back busy only delays its next owner's work.
+constexpr size_t kIdleStreams = 32;
+struct StreamPool {
+  std::mutex mu;
+  std::vector<std::pair<int, cudaStream_t>> idle;
+};
+StreamPool& stream_pool() {
+  static StreamPool* p = new StreamPool;  // (not destroyed: the driver may be gone by then)
+  return *p;
+}
+int take_stream(cudaStream_t* s) {
+  int dev = 0;
+  ILM_CHECK_CUDA(cudaGetDevice(&dev));
+  {
+    StreamPool& P = stream_pool();
+    std::lock_guard<std::mutex> lk(P.mu);
+    for (size_t k = 0; k < P.idle.size(); ++k)
+      if (P.idle[k].first == dev) {
+        *s = P.idle[k].second;
+        P.idle.erase(P.idle.begin() + (long)k);
+        return ILM_OK;
+      }
+  }
+  ILM_CHECK_CUDA(cudaStreamCreateWithFlags(s, cudaStreamNonBlocking));
+  return ILM_OK;
+}
+void give_stream(cudaStream_t s) {
+  if (!s) return;
+  int dev = 0;
+  const cudaError_t q = cudaStreamQuery(s);
+  if ((q == cudaSuccess || q == cudaErrorNotReady) && cudaStreamGetDevice(s, &dev) == cudaSuccess) {
+    StreamPool& P = stream_pool();
+    std::lock_guard<std::mutex> lk(P.mu);
+    if (P.idle.size() < kIdleStreams) {
+      P.idle.emplace_back(dev, s);
+      s = nullptr;
+    }
+  }
+  (void)cudaGetLastError();
+  if (s) cudaStreamDestroy(s);
+}
+
+}  // namespace
+
 struct ilm_batch_s {
   int nprob = 0, dtype = ILM_F64, ddf = ILM_DDF_YANG3, Ptot = 0, maxN = 0, max_grid = 0;
   std::vector<ilm_batch_problem_t> probs;
@@ -388,7 +436,7 @@ struct ilm_batch_s {
   std::vector<std::pair<const char*, double>> setup_ms;
   // the set-up's device memory: geometry, work buffers and task tables are
   // views into two arenas (one allocation and one host->device copy each)
-  DevBuf arena_geom, arena_tasks;
+  DevBuf arena_geom, arena_tasks, arena_bj, arena_cgp;
   DevBuf px, py, ph;  // point coordinates (FP64) and per-problem h on the device
   // set while the Schur build of ilm_batch_create may still be running: it
   // continues past the call's return, and every launch that reads S waits
@@ -416,16 +464,13 @@ struct ilm_batch_s {
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_join) cudaEventDestroy(ev_join);
     if (ev_join3) cudaEventDestroy(ev_join3);
-    if (s2) cudaStreamDestroy(s2);
-    if (s3) cudaStreamDestroy(s3);
-    if (s_setup) cudaStreamDestroy(s_setup);
+    for (cudaStream_t s : {s2, s3, s_setup}) give_stream(s);
     for (cudaEvent_t e : {bj_ready, band_ready, coarse_ready})
       if (e) {
         cudaEventSynchronize(e);
         cudaEventDestroy(e);
       }
-    if (s_bj) cudaStreamDestroy(s_bj);
-    if (s_learn) cudaStreamDestroy(s_learn);
+    for (cudaStream_t s : {s_bj, s_learn}) give_stream(s);
     delete twin;
   }
 };
@@ -625,28 +670,33 @@ int check_band(ilm_batch_s* b) {
 }
 
 int ensure_setup_stream(ilm_batch_s* b) {
-  if (!b->s_setup) ILM_CHECK_CUDA(cudaStreamCreateWithFlags(&b->s_setup, cudaStreamNonBlocking));
+  if (!b->s_setup) ILM_TRY(take_stream(&b->s_setup));
+  return ILM_OK;
+}
+
+int ensure_bj_stream(ilm_batch_s* b) {
+  if (!b->s_bj) ILM_TRY(take_stream(&b->s_bj));
+  if (!b->bj_ready) ILM_CHECK_CUDA(cudaEventCreateWithFlags(&b->bj_ready, cudaEventDisableTiming));
   return ILM_OK;
 }
 
 // Block-Jacobi inverses (Gauss-Jordan, float-float) of the problems whose
 // preconditioner uses them: every problem under block-Jacobi, the problems
 // without a network under the learned preconditioner
-int ensure_block_inverses(ilm_batch_s* b) {
+int ensure_block_inverses(ilm_batch_s* b, bool coarse_only = false) {
   if (b->bj_block <= 0 || b->precond == 0) return ILM_OK;
   std::vector<BJBlockTask> todo;
   std::vector<int> todo_probs;
   for (int p = 0; p < b->nprob; ++p) {
     const bool need = b->precond == 1 || (b->precond == 2 && (b->has_band.empty() || !b->has_band[p]));
-    if (!need || b->bj_have[p]) continue;
+    if (!need || b->bj_have[p] || (coarse_only && b->coarse_nb[p] == 0)) continue;
     for (int t = b->bj_first[p]; t < b->bj_first[p + 1]; ++t) todo.push_back(b->bj_tasks_host[t]);
     b->bj_have[p] = 1;
     todo_probs.push_back(p);
   }
   if (todo.empty()) return ILM_OK;
   const auto t0 = std::chrono::steady_clock::now();
-  if (!b->s_bj) ILM_CHECK_CUDA(cudaStreamCreateWithFlags(&b->s_bj, cudaStreamNonBlocking));
-  if (!b->bj_ready) ILM_CHECK_CUDA(cudaEventCreateWithFlags(&b->bj_ready, cudaEventDisableTiming));
+  ILM_TRY(ensure_bj_stream(b));
   ILM_TRY(wait_schur_for(b, b->s_bj, todo_probs));
   ILM_TRY(b->lz_bjtasks.alloc(todo.size() * sizeof(BJBlockTask)));
   // (from pageable memory: the copy has read todo when the call returns)
@@ -659,8 +709,70 @@ int ensure_block_inverses(ilm_batch_s* b) {
   return ILM_OK;
 }
 
+// Many small device arrays carved out of one allocation; the ones with host
+// data are filled by one host->device copy through pinned staging memory
+// (kept by the library and grown on demand; one batch set-up at a time
+// uses it).  g_stage_done marks the end of the last copy out of it: the next
+// set-up waits for it before writing the staging memory again, so a copy's
+// stream need not be synchronised (work after it on that stream is ordered
+// after it anyway).
+std::mutex g_stage_mu;
+void* g_stage = nullptr;
+size_t g_stage_bytes = 0;
+cudaEvent_t g_stage_done = nullptr;
+
+struct ArenaBuilder {
+  struct Item {
+    DevBuf* dst;
+    size_t off, bytes;
+    const void* src;
+  };
+  std::vector<Item> items;
+  size_t total = 0, copy_end = 0;
+  void add(DevBuf* dst, size_t bytes, const void* src = nullptr) {
+    const size_t off = (total + 255) & ~(size_t)255;
+    items.push_back({dst, off, bytes, src});
+    total = off + std::max<size_t>(bytes, 1);
+    if (src && bytes) copy_end = off + bytes;
+  }
+  template <typename V>
+  void add(DevBuf* dst, const std::vector<V>& v) {
+    add(dst, v.size() * sizeof(V), v.data());
+  }
+  int commit(DevBuf& arena, cudaStream_t st) {
+    ILM_TRY(commit_layout(arena));
+    return commit_upload(arena, st);
+  }
+  // allocate the arena and point every buffer at its part
+  int commit_layout(DevBuf& arena) {
+    ILM_TRY(arena.alloc(std::max<size_t>(total, 256)));
+    for (const Item& it : items) it.dst->view(static_cast<unsigned char*>(arena.p) + it.off, it.bytes);
+    return ILM_OK;
+  }
+  // one copy of every buffer's host data (read now, so the host arrays may
+  // have been edited after commit_layout)
+  int commit_upload(DevBuf& arena, cudaStream_t st) {
+    if (!copy_end) return ILM_OK;
+    std::lock_guard<std::mutex> lk(g_stage_mu);
+    if (!g_stage_done) ILM_CHECK_CUDA(cudaEventCreateWithFlags(&g_stage_done, cudaEventDisableTiming));
+    ILM_CHECK_CUDA(cudaEventSynchronize(g_stage_done));  // the last copy out of the staging memory
+    if (g_stage_bytes < copy_end) {
+      if (g_stage) cudaFreeHost(g_stage);
+      g_stage = nullptr;
+      g_stage_bytes = 0;
+      ILM_CHECK_CUDA(cudaMallocHost(&g_stage, copy_end));
+      g_stage_bytes = copy_end;
+    }
+    for (const Item& it : items)
+      if (it.src && it.bytes) memcpy(static_cast<unsigned char*>(g_stage) + it.off, it.src, it.bytes);
+    ILM_CHECK_CUDA(cudaMemcpyAsync(arena.p, g_stage, copy_end, cudaMemcpyHostToDevice, st));
+    ILM_CHECK_CUDA(cudaEventRecord(g_stage_done, st));
+    return ILM_OK;
+  }
+};
+
 // CG parameter records for the current preconditioner, tolerance and limit
-int ensure_cg_params(ilm_batch_s* b, double tol, int maxiter) {
+int ensure_cg_params(ilm_batch_s* b, double tol, int maxiter, cudaStream_t st) {
   if (tol == b->cg_tol && maxiter == b->cg_maxiter && !b->params_dirty) return ILM_OK;
   ILM_TRY(check_band(b));
   // the size split's queues and stream, built here (outside any stream
@@ -694,7 +806,11 @@ int ensure_cg_params(ilm_batch_s* b, double tol, int maxiter) {
       cgff_params_set_coarse(dst, b->coarse_nb[p], &b->coarse_start[(size_t)p * (CG_COARSE_MAX + 1)],
                              b->coarse_Einv.as<double>() + (size_t)p * CG_COARSE_MAX * CG_COARSE_MAX);
   }
-  ILM_TRY(up(b->cgp, cg));
+  {
+    ArenaBuilder A;  // through pinned memory: a plain copy would wait for the stage before
+    A.add(&b->cgp, cg);
+    ILM_TRY(A.commit(b->arena_cgp, st));
+  }
   b->cg_tol = tol;
   b->cg_maxiter = maxiter;
   b->param_gen++;
@@ -860,7 +976,7 @@ int ensure_split(ilm_batch_s* b) {
     if (n <= kSplitN) max_small = std::max(max_small, n);
   }
   for (cudaStream_t* s : {&b->s2, &b->s3})
-    if (!*s) ILM_CHECK_CUDA(cudaStreamCreateWithFlags(s, cudaStreamNonBlocking));
+    if (!*s) ILM_TRY(take_stream(s));
   // timing-enabled fork / join events: with cudaEventDisableTiming the two
   // launches of the split measured as if serialised on GB300 (2.77 against
   // 2.44 ms per batched solve of the bench configuration, CUDA events around
@@ -986,68 +1102,6 @@ __global__ void k_scatter_rows(int Nsel, int P, const int* __restrict__ c2o, con
     band[(size_t)c2o[e / P] * P + e % P] = rows[e];
 }
 
-// Many small device arrays carved out of one allocation; the ones with host
-// data are filled by one host->device copy through pinned staging memory
-// (kept by the library and grown on demand; one batch set-up at a time
-// uses it).  g_stage_done marks the end of the last copy out of it: the next
-// set-up waits for it before writing the staging memory again, so a copy's
-// stream need not be synchronised (work after it on that stream is ordered
-// after it anyway).
-std::mutex g_stage_mu;
-void* g_stage = nullptr;
-size_t g_stage_bytes = 0;
-cudaEvent_t g_stage_done = nullptr;
-
-struct ArenaBuilder {
-  struct Item {
-    DevBuf* dst;
-    size_t off, bytes;
-    const void* src;
-  };
-  std::vector<Item> items;
-  size_t total = 0, copy_end = 0;
-  void add(DevBuf* dst, size_t bytes, const void* src = nullptr) {
-    const size_t off = (total + 255) & ~(size_t)255;
-    items.push_back({dst, off, bytes, src});
-    total = off + std::max<size_t>(bytes, 1);
-    if (src && bytes) copy_end = off + bytes;
-  }
-  template <typename V>
-  void add(DevBuf* dst, const std::vector<V>& v) {
-    add(dst, v.size() * sizeof(V), v.data());
-  }
-  int commit(DevBuf& arena, cudaStream_t st) {
-    ILM_TRY(commit_layout(arena));
-    return commit_upload(arena, st);
-  }
-  // allocate the arena and point every buffer at its part
-  int commit_layout(DevBuf& arena) {
-    ILM_TRY(arena.alloc(std::max<size_t>(total, 256)));
-    for (const Item& it : items) it.dst->view(static_cast<unsigned char*>(arena.p) + it.off, it.bytes);
-    return ILM_OK;
-  }
-  // one copy of every buffer's host data (read now, so the host arrays may
-  // have been edited after commit_layout)
-  int commit_upload(DevBuf& arena, cudaStream_t st) {
-    if (!copy_end) return ILM_OK;
-    std::lock_guard<std::mutex> lk(g_stage_mu);
-    if (!g_stage_done) ILM_CHECK_CUDA(cudaEventCreateWithFlags(&g_stage_done, cudaEventDisableTiming));
-    ILM_CHECK_CUDA(cudaEventSynchronize(g_stage_done));  // the last copy out of the staging memory
-    if (g_stage_bytes < copy_end) {
-      if (g_stage) cudaFreeHost(g_stage);
-      g_stage = nullptr;
-      g_stage_bytes = 0;
-      ILM_CHECK_CUDA(cudaMallocHost(&g_stage, copy_end));
-      g_stage_bytes = copy_end;
-    }
-    for (const Item& it : items)
-      if (it.src && it.bytes) memcpy(static_cast<unsigned char*>(g_stage) + it.off, it.src, it.bytes);
-    ILM_CHECK_CUDA(cudaMemcpyAsync(arena.p, g_stage, copy_end, cudaMemcpyHostToDevice, st));
-    ILM_CHECK_CUDA(cudaEventRecord(g_stage_done, st));
-    return ILM_OK;
-  }
-};
-
 // Set-up of a batch; without `build_schur` the Schur matrices are neither
 // allocated nor built (the FP64 refinement copy uses its parent's).
 int batch_create_impl(int nprob, const ilm_batch_problem_t* probs, const double* x, const double* y,
@@ -1168,17 +1222,26 @@ int batch_create_impl(int nprob, const ilm_batch_problem_t* probs, const double*
       }
   }
   // set-up streams (non-blocking: independent of the legacy stream): the
+  // work area of each problem's FFT convolution
+  std::vector<size_t> woff(nprob + 1, 0);
+  std::vector<int> P1(nprob), P2(nprob);
+  for (int p = 0; p < nprob; ++p) {
+    const int n1 = probs[p].nx - 1, n2 = probs[p].ny - 1;
+    P1[p] = good_fft_size(2 * n1 - 1);
+    P2[p] = good_fft_size(2 * n2 - 1);
+    woff[p + 1] = woff[p] + (size_t)n2 * (P1[p] / 2 + 1) * 2 * e;
+  }
   // geometry and task tables on sg, the Schur build on ss, overlapping the
   // host's task building
   struct Streams {
     cudaStream_t g = nullptr, s = nullptr;
     ~Streams() {
-      if (g) cudaStreamDestroy(g);
-      if (s) cudaStreamDestroy(s);
+      give_stream(g);
+      give_stream(s);
     }
   } SS;
-  ILM_CHECK_CUDA(cudaStreamCreateWithFlags(&SS.g, cudaStreamNonBlocking));
-  ILM_CHECK_CUDA(cudaStreamCreateWithFlags(&SS.s, cudaStreamNonBlocking));
+  ILM_TRY(take_stream(&SS.g));
+  ILM_TRY(take_stream(&SS.s));
   cudaStream_t sg = SS.g, ss = SS.s;
   DevBuf d_in[5], d_poff, d_grid, d_tpo[4], d_tso[4], d_cnt, d_spb;
   {
@@ -1196,9 +1259,12 @@ int batch_create_impl(int nprob, const ilm_batch_problem_t* probs, const double*
       A.add(&d_tpo[c], tpo[c]);
       A.add(&d_tso[c], tso[c]);
     }
-    for (int d = 0; d < 2; ++d) {
+    for (int d = 0; d < 2; ++d) {  // (these and the tile pointers are read back together)
       A.add(&B->bx[d], (size_t)Ptot * 4);
       A.add(&B->by[d], (size_t)Ptot * 4);
+    }
+    for (int c = 0; c < 4; ++c) A.add(&B->tptr[c], (size_t)tp_tot[c] * 4);
+    for (int d = 0; d < 2; ++d) {
       A.add(&B->wx[d], (size_t)Ptot * NTAP * e);
       A.add(&B->wy[d], (size_t)Ptot * NTAP * e);
       A.add(&B->wx64[d], (size_t)Ptot * NTAP * 8);
@@ -1212,7 +1278,6 @@ int batch_create_impl(int nprob, const ilm_batch_problem_t* probs, const double*
     A.add(&B->ds64, (size_t)Ptot * 8);
     int cnt_tot = 0;
     for (int c = 0; c < 4; ++c) {
-      A.add(&B->tptr[c], (size_t)tp_tot[c] * 4);
       A.add(&B->tpts[c], (size_t)std::max(ts_tot[c], 1) * 4);
       cnt_tot += tp_tot[c];
     }
@@ -1221,6 +1286,7 @@ int batch_create_impl(int nprob, const ilm_batch_problem_t* probs, const double*
     A.add(&B->fstar, B->ftot * e);
     A.add(&B->corr, B->ftot * e);
     A.add(&B->edges, B->etot * e);
+    A.add(&B->convwork, woff[nprob]);
     A.add(&B->jump, (size_t)Ptot * e);
     A.add(&B->avg, (size_t)Ptot * e);
     A.add(&B->g, (size_t)Ptot * e);
@@ -1320,18 +1386,18 @@ int batch_create_impl(int nprob, const ilm_batch_problem_t* probs, const double*
   B->hny.assign(nrmy, nrmy + Ptot);
   B->hds.assign(ds, ds + Ptot);
   // the windows' base indices and the tile pointers, for the boxes and task
-  // tables built on the host (the copies to pageable memory return once done)
-  std::vector<int> hbx[2], hby[2], htp[4];
-  for (int d = 0; d < 2; ++d) {
-    hbx[d].resize(Ptot);
-    hby[d].resize(Ptot);
-    ILM_CHECK_CUDA(cudaMemcpyAsync(hbx[d].data(), B->bx[d].p, (size_t)Ptot * 4, cudaMemcpyDeviceToHost, sg));
-    ILM_CHECK_CUDA(cudaMemcpyAsync(hby[d].data(), B->by[d].p, (size_t)Ptot * 4, cudaMemcpyDeviceToHost, sg));
-  }
-  for (int c = 0; c < 4; ++c) {
-    htp[c].resize(tp_tot[c]);
-    ILM_CHECK_CUDA(cudaMemcpyAsync(htp[c].data(), B->tptr[c].p, (size_t)tp_tot[c] * 4, cudaMemcpyDeviceToHost, sg));
-  }
+  // tables built on the host: one copy (to pageable memory: it returns once done)
+  const unsigned char* const back0 = static_cast<const unsigned char*>(B->bx[0].p);
+  const size_t back_bytes = static_cast<const unsigned char*>(B->tptr[3].p) + (size_t)tp_tot[3] * 4 - back0;
+  const std::unique_ptr<unsigned char[]> back(new unsigned char[back_bytes]);
+  ILM_CHECK_CUDA(cudaMemcpyAsync(back.get(), back0, back_bytes, cudaMemcpyDeviceToHost, sg));
+  auto read_back = [&](const DevBuf& d) {
+    return reinterpret_cast<const int*>(back.get() + (static_cast<const unsigned char*>(d.p) - back0));
+  };
+  const int* const hbx[2] = {read_back(B->bx[0]), read_back(B->bx[1])};
+  const int* const hby[2] = {read_back(B->by[0]), read_back(B->by[1])};
+  const int* const htp[4] = {read_back(B->tptr[0]), read_back(B->tptr[1]), read_back(B->tptr[2]),
+                             read_back(B->tptr[3])};
   ILM_CHECK_CUDA(cudaStreamSynchronize(sg));
   phase("DDF windows and tile lists (device) + read-back; host copy of the points");
   std::vector<int> ord(nprob);
@@ -1345,16 +1411,7 @@ int batch_create_impl(int nprob, const ilm_batch_problem_t* probs, const double*
     B->nclusters = cg_cluster_count(nprob, B->maxN);
   }
 
-  // FFT convolution jobs (fstar and corr in place); one work area per problem
-  std::vector<size_t> woff(nprob + 1, 0);
-  std::vector<int> P1(nprob), P2(nprob);
-  for (int p = 0; p < nprob; ++p) {
-    const int n1 = probs[p].nx - 1, n2 = probs[p].ny - 1;
-    P1[p] = good_fft_size(2 * n1 - 1);
-    P2[p] = good_fft_size(2 * n2 - 1);
-    woff[p + 1] = woff[p] + (size_t)n2 * (P1[p] / 2 + 1) * 2 * e;
-  }
-  ILM_TRY(B->convwork.alloc(woff[nprob]));
+  // FFT convolution jobs (fstar and corr in place)
   // Source box of each problem: every cell of the two convolution inputs that
   // can be non-zero (DDF windows of all points, both staggerings, widened by
   // the divergence stencil) lies in [ca, cb) x [ra, rb).  The scatters and
@@ -1457,7 +1514,7 @@ int batch_create_impl(int nprob, const ilm_batch_problem_t* probs, const double*
     T.fill0 = fills;
     fills += yb - ya;
     // occupied tiles of the box (ids into the problem's tile grid), packed
-    const int* tp = htp[pc].data() + tpo[pc][p];
+    const int* tp = htp[pc] + tpo[pc][p];
     T.pad_ = (int)nelist.size();  // offset into the packed list, resolved after upload
     for (int ty = T.ty0; ty < T.ty0 + ntyb; ++ty)
       for (int tx = T.tx0; tx < T.tx0 + T.ntxb; ++tx) {
@@ -1758,7 +1815,7 @@ int ilm_batch_solve(ilm_batch_t b, const void* fplus, const void* fminus, void* 
   b->launches = 0;
   ILM_TRY(batch_mark(b, st));
   ILM_TRY(batch_stage_a(b, fplus, fminus, st));
-  ILM_TRY(ensure_cg_params(b, tol, maxiter));
+  ILM_TRY(ensure_cg_params(b, tol, maxiter, st));
   ILM_TRY(batch_cg(b, st));
   ILM_TRY(st_convert(b->Ptot, ILM_F64, b->x64.p, b->dtype, s_out, st));
   ILM_CHECK_CUDA(cudaMemcpyAsync(b->s.p, s_out, (size_t)b->Ptot * es(b->dtype), cudaMemcpyDeviceToDevice, st));
@@ -1800,7 +1857,7 @@ int ilm_batch_solve_refined(ilm_batch_t b, const double* fplus, const double* fm
   b->nev = 0;
   b->launches = 0;
   // first solve in the batch's precision, and the FP64 right-hand side
-  ILM_TRY(ensure_cg_params(b, std::max(tol, kRefineFirstTol), maxiter));
+  ILM_TRY(ensure_cg_params(b, std::max(tol, kRefineFirstTol), maxiter, st));
   if (b->dtype == ILM_F64) {
     ILM_TRY(batch_stage_a(b, fplus, fminus, st));
   } else {
@@ -1847,7 +1904,7 @@ int ilm_batch_solve_refined(ilm_batch_t b, const double* fplus, const double* fm
     }
     if (worst <= tol || k >= max_refine) break;
     // correction: S d = r (FP64 vectors, float-float S), x += d
-    ILM_TRY(ensure_cg_params(b, kRefineInnerTol, maxiter));
+    ILM_TRY(ensure_cg_params(b, kRefineInnerTol, maxiter, st));
     ILM_CHECK_CUDA(cudaMemcpyAsync(b->rhs64.p, b->ref_r.p, (size_t)Ptot * 8, cudaMemcpyDeviceToDevice, st));
     ILM_TRY(batch_cg(b, st));
     ILM_TRY(st_axpby(Ptot, ILM_F64, 1.0, b->ref_x.p, 1.0, b->x64.p, b->ref_x.p, st));
@@ -1874,8 +1931,9 @@ int ilm_batch_set_precond(ilm_batch_t b, int mode, int block_size) {
   if (mode == 1) {
     ILM_REQUIRE(block_size >= 4 && block_size <= 72, "batch: block size %d outside [4, 72]", block_size);
     if (b->bj_block != block_size) {
-      // inverses still being formed write into the arrays rebuilt here
-      if (b->bj_ready) ILM_CHECK_CUDA(cudaEventSynchronize(b->bj_ready));
+      // inverses still being formed write into the arrays rebuilt here, and a
+      // solve may still read them
+      if (b->bj_block > 0) ILM_CHECK_CUDA(cudaDeviceSynchronize());
       // blocks of ~block_size consecutive points (at most 1.5 x block_size);
       // their inverses are formed by the next solve, for the problems whose
       // preconditioner uses them (ensure_block_inverses)
@@ -1908,16 +1966,21 @@ int ilm_batch_set_precond(ilm_batch_t b, int mode, int block_size) {
       }
       b->bj_first[b->nprob] = (int)bst.size();
       ILM_REQUIRE(max_sz <= 144, "batch: preconditioner block of %d points", max_sz);
-      ILM_TRY(b->bj_inv.alloc(std::max<size_t>(total, 1) * sizeof(float)));
-      ILM_TRY(b->bj_inv_lo.alloc(std::max<size_t>(total, 1) * sizeof(float)));
+      ILM_TRY(ensure_bj_stream(b));
+      ArenaBuilder A;  // the tables, then the inverses
+      A.add(&b->bj_blk, blk);
+      A.add(&b->bj_start, bst);
+      A.add(&b->bj_size, bsz);
+      A.add(&b->bj_off, boff);
+      A.add(&b->lz_bjtasks, b->bj_tasks_host.size() * sizeof(BJBlockTask));
+      A.add(&b->bj_inv, std::max<size_t>(total, 1) * sizeof(float));
+      A.add(&b->bj_inv_lo, std::max<size_t>(total, 1) * sizeof(float));
+      ILM_TRY(A.commit(b->arena_bj, b->s_bj));
+      ILM_CHECK_CUDA(cudaEventRecord(b->bj_ready, b->s_bj));
       for (size_t t = 0; t < b->bj_tasks_host.size(); ++t) {
         b->bj_tasks_host[t].out_hi = b->bj_inv.as<float>() + boff[t];
         b->bj_tasks_host[t].out_lo = b->bj_inv_lo.as<float>() + boff[t];
       }
-      ILM_TRY(up(b->bj_blk, blk));
-      ILM_TRY(up(b->bj_start, bst));
-      ILM_TRY(up(b->bj_size, bsz));
-      ILM_TRY(up(b->bj_off, boff));
       b->bj_max_sz = max_sz;
       b->bj_have.assign(b->nprob, 0);
       b->bj_block = block_size;
@@ -2013,7 +2076,7 @@ int ilm_batch_solve_graph(ilm_batch_t b, const void* fplus, const void* fminus, 
   ILM_REQUIRE(tol > 0 && maxiter > 0, "batch_solve_graph: bad tolerance / iteration limit");
   cudaStream_t st = as_stream(stream);
   ILM_REQUIRE(st != nullptr, "batch_solve_graph: needs a created stream (the legacy default stream cannot be captured)");
-  ILM_TRY(ensure_cg_params(b, tol, maxiter));
+  ILM_TRY(ensure_cg_params(b, tol, maxiter, st));
   ILM_TRY(wait_schur_host(b));
   for (cudaEvent_t e : {b->bj_ready, b->band_ready, b->coarse_ready})
     if (e) ILM_CHECK_CUDA(cudaEventSynchronize(e));
@@ -2253,6 +2316,9 @@ int ilm_batch_set_coarse(ilm_batch_t b, int kind_mask, const int* body_start) {
     b->coarse_nb[p] = tasks[t].nb;
     for (int q = 0; q < M1; ++q) b->coarse_start[(size_t)p * M1 + q] = tasks[t].cst[q];
   }
+  // the correction goes with block-Jacobi: its inverses form from here on,
+  // while the caller prepares the first solve
+  ILM_TRY(ensure_block_inverses(b, true));
   b->setup_ms.emplace_back("coarse correction (issued; E and E^-1 on the device)",
                            std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count());
   return ILM_OK;
@@ -2313,7 +2379,7 @@ int ilm_batch_set_learned(ilm_batch_t b, ilm_net_t net, int kind_mask, const int
   // the set-up runs on its own stream, without host synchronisation: the CG
   // launches wait for band_ready, and the network's timeout flag is checked
   // before the first solve (check_band)
-  if (!b->s_learn) ILM_CHECK_CUDA(cudaStreamCreateWithFlags(&b->s_learn, cudaStreamNonBlocking));
+  if (!b->s_learn) ILM_TRY(take_stream(&b->s_learn));
   if (!b->band_ready) ILM_CHECK_CUDA(cudaEventCreateWithFlags(&b->band_ready, cudaEventDisableTiming));
   cudaStream_t sl = b->s_learn;
   DevBuf d_c2o, d_sst, d_sln, dfeat, tmp;
@@ -2330,8 +2396,9 @@ int ilm_batch_set_learned(ilm_batch_t b, ilm_net_t net, int kind_mask, const int
     ArenaBuilder S;  // the body segments the CG reads (the same for every call)
     S.add(&b->lseg_start, ls);
     S.add(&b->lseg_len, ll);
+    S.add(&b->band, (size_t)std::max(Ptot, 1) * P * sizeof(float));
+    S.add(&b->band_err, sizeof(int));
     ILM_TRY(S.commit(b->arena_learned, sl));
-    if (b->band_k < 0) ILM_TRY(b->band.alloc((size_t)std::max(Ptot, 1) * P * sizeof(float)));
   }
   phase("learned: segments (host) and upload");
   if (Nsel > 0) {
@@ -2346,7 +2413,6 @@ int ilm_batch_set_learned(ilm_batch_t b, ilm_net_t net, int kind_mask, const int
                                                                             b->band.as<float>());
     ILM_CHECK_LAUNCH();
     if (int* flag = net_tc_flag(net)) {  // the timeout flag, moved into the batch
-      ILM_TRY(b->band_err.alloc(sizeof(int)));
       ILM_CHECK_CUDA(cudaMemcpyAsync(b->band_err.p, flag, sizeof(int), cudaMemcpyDeviceToDevice, sl));
       ILM_CHECK_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), sl));
       b->band_check = true;
@@ -2382,7 +2448,7 @@ int ilm_batch_schur_solve(ilm_batch_t b, const double* rhs, double* x, double to
   ILM_REQUIRE(b && rhs && x, "batch_schur_solve: null argument");
   ILM_REQUIRE(tol > 0 && maxiter > 0, "batch_schur_solve: bad tolerance / iteration limit");
   cudaStream_t st = as_stream(stream);
-  ILM_TRY(ensure_cg_params(b, tol, maxiter));
+  ILM_TRY(ensure_cg_params(b, tol, maxiter, st));
   ILM_CHECK_CUDA(cudaMemcpyAsync(b->rhs64.p, rhs, (size_t)b->Ptot * 8, cudaMemcpyDeviceToDevice, st));
   ILM_TRY(wait_schur(b, st));
   ILM_TRY(wait_precond(b, st));

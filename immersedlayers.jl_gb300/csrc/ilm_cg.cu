@@ -1269,14 +1269,6 @@ static int launch_dist(const CGFFParams* prm, const int* order, int nprob, int* 
   return ILM_OK;
 }
 
-template <int NT, int MINB, int CS>
-static cudaError_t clusters_dist(int* nc, cudaLaunchConfig_t* cfg, size_t smem) {
-  cudaError_t e =
-      cudaFuncSetAttribute(k_cg_cluster<NT, MINB, CS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(nc, k_cg_cluster<NT, MINB, CS>, cfg);
-  return e;
-}
-
 int launch_cg_cluster(const void* params_dev, const int* order, int nprob, int* counter, int max_n, int nclusters,
                       cudaStream_t st, int variant) {
   const CGFFParams* prm = static_cast<const CGFFParams*>(params_dev);
@@ -1352,34 +1344,13 @@ int cg_cluster_count(int nprob, int max_n, int variant) {
   // co-resident clusters of the kernel launch_cg_cluster will pick (the
   // persistent clusters beyond that would only find the queue empty)
   const bool rep = use_rep(variant, max_n);
-  const int nt = rep ? CGR_THREADS : dist_threads(variant);
   const int cs = rep ? CG_CLUSTER : dist_cluster(variant);
   const size_t smem = cg_variant_smem(max_n, variant);
-  int nc = 0;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(cs * nsm);
-  cfg.blockDim = dim3(nt);
-  cfg.dynamicSmemBytes = smem;
-  cudaError_t e;
-  if (rep) {
-    e = cudaFuncSetAttribute(k_cg_rep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&nc, k_cg_rep, &cfg);
-  } else if (!dist_fits(max_n, nt, cs)) {
-    e = cudaErrorInvalidValue;  // the launch refuses this variant; any count will do
-  } else {
-    switch (variant) {
-      case 3: e = clusters_dist<128, 6, CG_CLUSTER>(&nc, &cfg, smem); break;
-      case 4: e = clusters_dist<256, 2, CG_CLUSTER>(&nc, &cfg, smem); break;
-      case 5: e = clusters_dist<512, 1, CG_CLUSTER>(&nc, &cfg, smem); break;
-      default: e = clusters_dist<256, 3, CG_CLUSTER>(&nc, &cfg, smem); break;
-    }
-  }
-  if (e != cudaSuccess || nc <= 0) {
-    (void)cudaGetLastError();
-    const int per_sm = variant == 3 ? 6 : variant == 4 ? 2 : variant == 5 ? 1 : 3;
-    nc = std::max(1, per_sm * nsm / cs);
-  }
-  return std::min(nc, nprob);
+  // (from the launch bounds and the shared memory: the occupancy query takes
+  // 0.1 ms of a set-up; clusters that are not resident find the queue empty)
+  const int bound = rep ? 3 : variant == 3 ? 6 : variant == 4 ? 2 : variant == 5 ? 1 : 3;
+  const int per_sm = std::max(1, std::min(bound, (int)(228 * 1024 / (smem + 2048))));
+  return std::min(std::max(1, per_sm * nsm / cs), nprob);
 }
 
 size_t cgff_params_size() { return sizeof(CGFFParams); }
