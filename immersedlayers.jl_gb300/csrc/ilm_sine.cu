@@ -133,11 +133,23 @@ __global__ void __launch_bounds__(SR_T) k_sine_rows(int N, int lx, int ly, int n
   const double* __restrict__ xa = in + (size_t)row * ldin - jin;
   const double* __restrict__ xb = xa + ldin;
   pdl_wait();
+  unsigned any = 0u;
   for (int j = t; j < N; j += SR_T) {
     const bool ok = j >= 1 && j >= jin && j < jin + nin;
-    B[j] = make_double2(ok ? xa[j] : 0.0, ok && two ? xb[j] : 0.0);
+    const double2 v = make_double2(ok ? xa[j] : 0.0, ok && two ? xb[j] : 0.0);
+    any |= (unsigned)__double2hiint(v.x) << 1 | (unsigned)__double2loint(v.x) | (unsigned)__double2hiint(v.y) << 1 |
+           (unsigned)__double2loint(v.y);
+    B[j] = v;
   }
-  __syncthreads();
+  // rows of zeros (beyond the bodies, where a source is regularized surface
+  // data): no transform
+  if (!__syncthreads_or(any != 0u)) {
+    for (int i = t; i < nout; i += SR_T) {
+      out[(size_t)row * ldout + i] = 0.0;
+      if (two) out[(size_t)(row + 1) * ldout + i] = 0.0;
+    }
+    return;
+  }
   if (FOLD) {
     // folds: level l leaves p_j at N_l - j and hands z_j - z_{N_l - j} at j to the next
     for (int l = 0; l < lx; ++l) {

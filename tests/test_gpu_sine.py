@@ -60,3 +60,21 @@ def test_inverse_laplacian_f64(cuda, nx, ny):
     assert err <= 2e-14, err
     il.inverse_laplacian_(w, c)  # in place
     assert torch.equal(w.data, out.data)
+
+
+@pytest.mark.parametrize("nx,ny,rows", [(97, 120, [0]), (97, 120, [118]), (130, 201, [7, 64, 65, 199]), (600, 311, [1]),
+                                        (1100, 350, [20, 348]), (49, 66, [])])
+def test_inverse_laplacian_rows_of_zeros(cuda, nx, ny, rows):
+    """A field that is zero but for some rows (first, last, unpaired ones; none:
+    zero out): the pairs of zero rows are not transformed."""
+    grid = il.PhysicalGrid.from_cells(nx, 0.5, ny=ny)
+    c = il.SurfaceScalarCache(None, grid)
+    g = torch.Generator(device="cuda").manual_seed(nx)
+    f = torch.zeros(ny - 1, nx - 1, dtype=torch.float64, device=cuda)
+    for r in rows:
+        f[r] = torch.randn(nx - 1, dtype=torch.float64, device=cuda, generator=g) + 0.3
+    out = il.NodesPrimal.zeros(grid)
+    out.data.fill_(7.0)
+    il.inverse_laplacian_(out, il.NodesPrimal(grid, f.reshape(-1).clone()), c)
+    ref = _reference(f) * 0.25
+    assert float((out.component(0) - ref).norm()) <= 2e-14 * float(ref.norm())
