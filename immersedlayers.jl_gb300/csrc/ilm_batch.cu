@@ -407,7 +407,7 @@ struct ilm_batch_s {
   // CG variant 6 (size split): clusters by problem size on three streams,
   // joined by events (ensure_split)
   bool split_ready = false;
-  int n_big = 0, n_large = 0, n_small = 0, max_small = 0, nctas_small = 0, cs_big = 8, cs_small = 1;
+  int n_big = 0, n_large = 0, n_small = 0, max_small = 0, nctas_small = 0, nclusters_mid = 1, cs_big = 8, cs_small = 1;
   cudaStream_t s2 = nullptr, s3 = nullptr;
   // lazy set-up of the first solve (block-Jacobi inverses, deflation
   // vectors): its own non-blocking stream, so that it overlaps the solve's
@@ -984,19 +984,23 @@ int ensure_split(ilm_batch_s* b) {
   // between the stages, which is how the difference was found)
   for (cudaEvent_t* e : {&b->ev_fork, &b->ev_join, &b->ev_join3})
     if (!*e) ILM_CHECK_CUDA(cudaEventCreate(e));
-  const int n_small = b->nprob - n_large, n_mid = n_large - n_big;
+  const int n_small = b->nprob - n_large;
+  int n_mid = n_large - n_big;
   const int slots = cg_cta_slots(b->maxN, 8);
   b->cs_big = 16 * n_big + 8 * n_mid + n_small <= slots ? 16 : 8;
   b->cs_small = b->cs_big * n_big + 8 * n_mid + 4 * n_small <= slots ? 4 : 1;
   if (b->cs_big == 8) n_big = 0;  // one queue of clusters of 8
+  n_mid = n_large - n_big;
   b->n_big = n_big;
   b->n_large = n_large;
   b->n_small = n_small;
   b->max_small = max_small;
-  // the CTA slots the large problems' clusters leave free (at least 8)
-  b->nctas_small = b->cs_small == 4 ? n_small
-                                    : std::max(8, std::min(n_small, (n_small ? cg_single_slots(max_small) : 0) -
-                                                                        8 * std::min(n_large, b->nclusters)));
+  // One CTA per small problem: the slots that the clusters of the large ones
+  // leave, and a ninth of all where these want them all (64 problems or more
+  // above kSplitN: 50 CTAs beside 50 clusters; with 8 CTAs left the small ones of
+  // 256 problems took 2.7 ms, with 48 0.8)
+  b->nctas_small = b->cs_small == 4 ? n_small : std::min(n_small, std::max(slots - 8 * n_large, slots / 9));
+  b->nclusters_mid = std::max(1, std::min(n_mid, (slots - b->nctas_small) / 8));
   b->split_ready = true;
   return ILM_OK;
 }
@@ -1026,8 +1030,8 @@ int batch_cg(ilm_batch_s* b, cudaStream_t st) {
         b->launches++;
       }
       if (n_mid > 0) {
-        ILM_TRY(launch_cg_sized(b->cgp.p, order + b->n_big, n_mid, counter, b->maxN, std::min(n_mid, b->nclusters), 8,
-                                st));
+        ILM_TRY(launch_cg_sized(b->cgp.p, order + b->n_big, n_mid, counter, b->maxN,
+                                b->cs_small == 4 ? n_mid : b->nclusters_mid, 8, st));
         b->launches++;
       }
       if (b->n_big > 0) ILM_CHECK_CUDA(cudaStreamWaitEvent(st, b->ev_join3, 0));

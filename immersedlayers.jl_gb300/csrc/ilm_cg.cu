@@ -1321,22 +1321,6 @@ int cg_cta_slots(int max_n, int cs) {
   return nsm * (int)std::min<size_t>(3, 228 * 1024 / (cg_cluster_smem(max_n, 256, cs) + 2048));
 }
 
-// co-resident CTAs of the single-CTA CG kernel on the whole device
-int cg_single_slots(int max_n) {
-  int dev = 0, nsm = 148, nb = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const size_t smem = cg_cluster_smem(max_n, 256, 1);
-  if (!dist_fits(max_n, 256, 1)) return 0;
-  if (cudaFuncSetAttribute(k_cg_cluster<256, 3, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-          cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_cg_cluster<256, 3, 1>, 256, smem) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return 0;
-  }
-  return nb * nsm;
-}
-
 int cg_cluster_count(int nprob, int max_n, int variant) {
   int dev = 0, nsm = 148;
   cudaGetDevice(&dev);

@@ -4,6 +4,10 @@
 // Replaces CartesianGrids' plan_laplacian(...; with_inverse=true) / `L \ w`
 // (called from src/grid_operators.jl:177-179, built at src/cache.jl:321-324).
 //
+// A single FP64 field goes through ilm_sine.cu and a single FP32 field through
+// ilm_fft_field.cu where these take its size; the passes here serve the batches,
+// the other sizes and the spectra.
+//
 // Pipeline for an n1 x n2 field (x fastest) and padded sizes P1 >= 2 n1 - 1,
 // P2 >= 2 n2 - 1 (P = 2^a or 3 * 2^a):
 //   1. k_rfft_rows  : each of the n2 rows -> real FFT of length P1 (complex

@@ -16,8 +16,9 @@
 //    stage right-hand sides are point-local gathers (E exp(aL) T is a gather
 //    with the DDF window smeared by the heat kernel) and the stage Schur
 //    complements S_a = E exp(aL) R are short-range: they are assembled once as
-//    sparse matrices (float-float values) and solved by the cluster CG with a
-//    warm start from the previous step;
+//    sparse matrices (float-float values) and solved with a warm start from
+//    the previous step by an FP32 inverse refined with FP64 residuals, FP64 CG
+//    where that stalls (ilm_cg64.cu);
 //  * the grid is touched once per step: T <- exp(dt kappa L) T +
 //    b2 dt exp(2/3 dt kappa L) R sigma_2 + b3 dt R sigma_3 + (constant field).
 #include <math.h>

@@ -814,7 +814,6 @@ int launch_block_inverse(const BJBlockTask* tasks_dev, int ntasks, int max_sz, c
 int launch_cg_sized(const void* params_dev, const int* order, int nprob, int* counter, int max_n, int nclusters, int cs,
                     cudaStream_t st);
 int cg_cta_slots(int max_n, int cs);
-int cg_single_slots(int max_n);
 int launch_cg_cluster(const void* params_dev, const int* order, int nprob, int* counter, int max_n, int nclusters,
                       cudaStream_t st, int variant = 0);
 int cg_cluster_count(int nprob, int max_n, int variant = 0);

@@ -17,8 +17,9 @@
 // instead of O(N * P^2 log P), and gives the same matrix (up to FP64 rounding) provided
 // every stencil stays clear of the grid's ghost layer.
 //
-// The solve (ilm_cg64.cu) is CG in the ds-weighted inner product (the matrices
-// are M*diag(w) with M symmetric) in FP64: an FP32 matvec loses the Krylov
+// The solve (ilm_cg64.cu) refines an FP32 inverse with FP64 residuals and goes
+// on by CG in the ds-weighted inner product (the matrices are M*diag(w) with M
+// symmetric) in FP64 where that stalls: an FP32 matvec in the CG loses the Krylov
 // convergence on these ill-conditioned (cond ~ 1e4-1e5) and, for the
 // Dirichlet problem, indefinite (one negative eigenvalue) systems.
 // Convergence is declared on the FP64 residual ||b - A x||_2 <= tol ||b||_2.

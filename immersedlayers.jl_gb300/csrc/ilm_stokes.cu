@@ -13,9 +13,13 @@
 // The reference forms S and Ss densely (2N and N columns of operator
 // applications) and LU-solves them.  L^-2 is two grid-truncated LGF
 // convolutions, which is not translation invariant, so S has no point-pair
-// closed form.  Both Schur systems are solved matrix-free, in the symmetric
+// closed form.  S is solved matrix-free; Ss is translation invariant and is
+// taken from the point-pair sums (ilm_schur.cu) and solved by the refined FP32
+// inverse (ilm_cg64.cu) where every window stays clear of the ghost layer, else
+// matrix-free as S.  The matrix-free solves take the symmetric
 // form y = W sigma (W = diag(ds)): -S W^-1 and Ss W^-1 are symmetric
-// positive semi-definite.  All right-hand sides are solved together by block
+// positive semi-definite.  One right-hand side runs CG with its scalars on the
+// device; several are solved together by block
 // CG: each iteration applies the operator to every column of the direction
 // block, A-orthonormalises the block (eigen-decomposition of its s x s Gram
 // matrix; directions that have become dependent are dropped), and forms the

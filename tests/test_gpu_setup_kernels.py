@@ -100,3 +100,37 @@ def test_batched_cg_cluster_sizes(cuda, precond, variant):
     for i in range(len(specs)):
         a, b = o[i], o[i + 1]
         assert r[a:b].norm().item() <= 1.1e-9 * rhs[a:b].norm().item(), (i, its[i])
+
+
+def test_batched_solve_queues(cuda):
+    """A batch whose default solve runs in three queues (16, 8 and 4 CTAs per
+    problem) against the same batch on clusters of 8: both to a residual of
+    1e-10, so the fields agree to 1e-8 (the strengths of the slow modes, up to a
+    condition number of 1e5 off, act on the field by their small eigenvalues)."""
+    import torch
+    from immersedlayers import bodies as B
+    from immersedlayers.batch import BatchProblemSpec, BatchSolver
+    h = 4.0 / 512
+    rng = np.random.default_rng(8)
+    specs = []
+    for n in (9, 150, 193, 260, 385, 410):
+        for kind in (0, 1):
+            b = B.circle(n * 1.4 * h / (2 * np.pi), n=n)
+            t = 2 * np.pi * np.arange(n) / n
+            a = rng.standard_normal(4)
+            specs.append(BatchProblemSpec(512, h, b, kind, a[0] * np.cos(t) + a[1] * np.sin(2 * t) + a[2] * np.cos(3 * t)))
+    bs = BatchSolver(specs, dtype=torch.float64)
+    bs.set_precond("bjacobi", 64)
+    bs.set_coarse(True)
+    fp, fm = bs.surface_data()
+    out = {}
+    for variant in (6, 1):
+        bs.set_cg_variant(variant)
+        f, _ = bs.solve(fp, fm, tol=1e-10, maxiter=20000)
+        torch.cuda.synchronize()
+        its, rr = bs.info()
+        assert (rr <= 1e-10).all(), (variant, its, rr)
+        out[variant] = f.clone()
+    for i in range(len(specs)):
+        a, b = bs.field(out[6], i), bs.field(out[1], i)
+        assert (a - b).abs().max().item() <= 1e-8 * b.abs().max().item(), i
