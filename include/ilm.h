@@ -286,7 +286,9 @@ ILM_API int ilm_schur_build(ilm_cache_t c, int which, double scale, double* A_de
 /* ---- problem solves (test/literate/problems.jl:259-298, neumann.jl:101-142) */
 /* Dirichlet Poisson: inputs fplus/fminus (ScalarData, device, cache dtype);
  * outputs f (Nodes{Primal}) and s (ScalarData).  The Schur system is solved
- * by CG on the device to rel. residual `tol` (FP64).                        */
+ * on the device to rel. residual `tol` (FP64): by an FP32 inverse, formed
+ * once per point set and refined with FP64 residuals, and by FP64 CG where
+ * that stalls.                                                              */
 ILM_API int ilm_solve_dirichlet(ilm_cache_t c, const void* fplus, const void* fminus,
                         void* f_out, void* s_out, double tol, int maxiter,
                         ilm_solve_info_t* info, ilm_stream_t stream);
@@ -327,9 +329,10 @@ ILM_API int ilm_solve_neumann_full(ilm_cache_t c, const void* vplus, const void*
  * velocity, s_out: Nodes{Dual} streamfunction, sigma_out: VectorData
  * traction (filtered twice, :165).  The Schur systems -C_s L^-2 C_s^T
  * (create_CL2invCT, src/matrix_operators.jl:102) and -C_s L^-1 C_s^T on
- * scalars (create_CLinvCT_scalar, :71) are solved matrix-free by
- * (preconditioned) CG in place of the reference's dense LU; info reports
- * both solves (iterations summed, worst relative residual).               */
+ * scalars (create_CLinvCT_scalar, :71) are solved by (preconditioned) CG in
+ * place of the reference's dense LU, the first matrix-free, the second from
+ * its dense matrix where every window stays clear of the ghost layer; info
+ * reports both solves (iterations summed, worst relative residual).       */
 ILM_API int ilm_solve_stokes(ilm_cache_t c, const void* vplus, const void* vminus, void* v_out, void* s_out,
                              void* sigma_out, double tol, int maxiter, ilm_solve_info_t* info,
                              ilm_stream_t stream);
@@ -338,8 +341,9 @@ ILM_API int ilm_solve_stokes(ilm_cache_t c, const void* vplus, const void* vminu
  * with one S).  vplus/vminus: nrhs x 2N (right-hand side r at offset 2N r);
  * v_out: nrhs Edges{Primal} fields, s_out: nrhs Nodes{Dual} fields,
  * sigma_out: nrhs x 2N, each contiguous in the cache dtype.  Both Schur
- * systems are solved by block CG over all right-hand sides (maxiter block
- * iterations each, Krylov vectors FP64); precond = 1 preconditions S with
+ * systems (the scalar one where its matrix is not dense) are solved by block
+ * CG over all right-hand sides (maxiter block iterations each, Krylov vectors
+ * FP64; a single right-hand side by CG with its scalars on the device); precond = 1 preconditions S with
  * the inverse of the gauge-shifted point-point Schur complement -E L^-1 E^T
  * on each velocity component (N <= 4096; built once per cache and kept
  * until the points move), 0 runs plain block CG.  info: nrhs entries
@@ -470,9 +474,10 @@ ILM_API int ilm_batch_cg_times(ilm_batch_t b, double* start_us, double* end_us, 
  * vectors (one cluster barrier per iteration, every vector operation in
  * every CTA), 3 row-distributed with 128-thread CTAs (twice the resident
  * clusters), 4 256-thread CTAs at most two per SM, 5 512-thread CTAs one
- * per SM, 6 size split: problems above 192 points on variant 1's clusters,
- * the smaller ones one CTA each (no cluster barriers) on a second stream in
- * the CTA slots the clusters leave free, joined by events (the Schur-only
+ * per SM, 6 size split: problems above 384 points, above 192 and the smaller
+ * ones in queues of their own on three streams, joined by events, with 16, 8
+ * and 4 CTAs per problem where the batch leaves the slots free, else 8, 8 and
+ * one (the Schur-only
  * entry points run every problem on variant 1).  ilm_batch_autotune solves the given
  * data with every variant (one untimed and `reps` timed solves each, each
  * between CUDA events on `stream`), keeps the fastest and returns it in
