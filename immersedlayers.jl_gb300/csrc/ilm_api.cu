@@ -941,7 +941,11 @@ int ilm_schur_build(ilm_cache_t c, int which, double scale, double* A_dev, ilm_s
               "Schur kind %d needs a vector cache", which);
   ILM_REQUIRE(!vec || which != ILM_SCHUR_GLINVD_CROSS, "Schur kind %d needs a scalar cache", which);
   cudaStream_t st = as_stream(stream);
-  if (!vec && which <= ILM_SCHUR_NRTRN) return schur_build(c, which, scale, A_dev, st);
+  if (!vec && which <= ILM_SCHUR_NRTRN) {
+    ILM_TRY(schur_build(c, which, scale, A_dev, st));
+    ILM_CHECK_CUDA(cudaStreamSynchronize(st));  // the matrix is complete on return
+    return ILM_OK;
+  }
   return schur_build_columns(c, which, scale, A_dev, st);
 }
 
@@ -1040,19 +1044,18 @@ int ilm_solve_dirichlet(ilm_cache_t c, const void* fplus, const void* fminus, vo
   ILM_TRY(pscr(c, 5, &x64));
   ILM_TRY(gscr(c, 3, &fstar));
   ILM_TRY(gscr(c, 4, &corr));
-  ILM_TRY(st_axpby(N, c->dtype, 1.0, fplus, -1.0, fminus, jump, st));
-  ILM_TRY(st_axpby(N, c->dtype, 0.5, fplus, 0.5, fminus, avg, st));
+  ILM_TRY(st_jump_average(N, c->dtype, fplus, fminus, jump, avg, st));
   ILM_TRY(ilm_surface_divergence(c, jump, fstar, stream));
   ILM_TRY(inverse_laplacian_kind(c, ILM_NODES_PRIMAL, fstar, fstar, st));
   GatherTerm t{PC_P, fstar, CF_ONE};
   ILM_TRY(launch_gather(c, &t, 1, g, false, 1.0, st));
-  ILM_TRY(st_axpby(N, c->dtype, 1.0, g, -1.0, avg, g, st));
-  ILM_TRY(st_convert(N, c->dtype, g, ILM_F64, rhs64, st));
+  ILM_TRY(st_difference64(N, c->dtype, g, avg, static_cast<double*>(rhs64), st));
   ILM_TRY(cached_schur(c, ILM_SCHUR_RTLINVR, st));
-  const int cg = schur_cg(c, ILM_SCHUR_RTLINVR, static_cast<double*>(rhs64), static_cast<double*>(x64), tol,
-                          maxiter, info, st);
+  const bool direct = c->dtype == ILM_F64;  // the solution goes straight into the output
+  const int cg = schur_cg(c, ILM_SCHUR_RTLINVR, static_cast<double*>(rhs64), static_cast<double*>(direct ? s_out : x64),
+                          tol, maxiter, info, st);
   if (cg != ILM_OK && cg != ILM_ERR_NOT_CONVERGED) return cg;
-  ILM_TRY(st_convert(N, ILM_F64, x64, c->dtype, s_out, st));
+  if (!direct) ILM_TRY(st_convert(N, ILM_F64, x64, c->dtype, s_out, st));
   ILM_TRY(scatter_scalar(c, PC_P, s_out, CF_ONE, corr, st));
   ILM_TRY(inverse_laplacian_kind(c, ILM_NODES_PRIMAL, corr, corr, st));
   ILM_TRY(st_axpby(np, c->dtype, 1.0, corr, 1.0, fstar, f_out, st));
@@ -1092,18 +1095,17 @@ int ilm_solve_neumann_full(ilm_cache_t c, const void* vplus, const void* vminus,
   ILM_TRY(pscr(c, 5, &x64));
   ILM_TRY(gscr(c, 3, &fstar));
   ILM_TRY(gscr(c, 4, &corr));
-  ILM_TRY(st_axpby(N, c->dtype, 1.0, vplus, -1.0, vminus, jump, st));
-  ILM_TRY(st_axpby(N, c->dtype, 0.5, vplus, 0.5, vminus, avg, st));
+  ILM_TRY(st_jump_average(N, c->dtype, vplus, vminus, jump, avg, st));
   ILM_TRY(scatter_scalar(c, PC_P, jump, CF_ONE, fstar, st));
   ILM_TRY(inverse_laplacian_kind(c, ILM_NODES_PRIMAL, fstar, fstar, st));
   ILM_TRY(ilm_surface_grad(c, fstar, g, stream));
-  ILM_TRY(st_axpby(N, c->dtype, 1.0, g, -1.0, avg, g, st));
-  ILM_TRY(st_convert(N, c->dtype, g, ILM_F64, rhs64, st));
+  ILM_TRY(st_difference64(N, c->dtype, g, avg, static_cast<double*>(rhs64), st));
   ILM_TRY(cached_schur(c, ILM_SCHUR_CLINVCT, st));
-  const int cg = schur_cg(c, ILM_SCHUR_CLINVCT, static_cast<double*>(rhs64), static_cast<double*>(x64), tol,
-                          maxiter, info, st);
+  const bool direct = c->dtype == ILM_F64;  // the solutions go straight into the outputs
+  const int cg = schur_cg(c, ILM_SCHUR_CLINVCT, static_cast<double*>(rhs64), static_cast<double*>(direct ? df_out : x64),
+                          tol, maxiter, info, st);
   if (cg != ILM_OK && cg != ILM_ERR_NOT_CONVERGED) return cg;
-  ILM_TRY(st_convert(N, ILM_F64, x64, c->dtype, df_out, st));
+  if (!direct) ILM_TRY(st_convert(N, ILM_F64, x64, c->dtype, df_out, st));
   ILM_TRY(ilm_surface_divergence(c, df_out, corr, stream));
   ILM_TRY(inverse_laplacian_kind(c, ILM_NODES_PRIMAL, corr, corr, st));
   ILM_TRY(st_axpby(np, c->dtype, 1.0, corr, 1.0, fstar, f_out, st));
@@ -1113,10 +1115,10 @@ int ilm_solve_neumann_full(ilm_cache_t c, const void* vplus, const void* vminus,
   ilm_solve_info_t info2{0, 1, 0.0};
   ILM_TRY(ilm_surface_grad_cross(c, fstar, g, stream));
   ILM_TRY(st_convert(N, c->dtype, g, ILM_F64, rhs64, st));
-  const int cg2 = schur_cg(c, ILM_SCHUR_CLINVCT, static_cast<double*>(rhs64), static_cast<double*>(x64), tol,
-                           maxiter, &info2, st);
+  const int cg2 = schur_cg(c, ILM_SCHUR_CLINVCT, static_cast<double*>(rhs64), static_cast<double*>(direct ? ds_out : x64),
+                           tol, maxiter, &info2, st);
   if (cg2 != ILM_OK && cg2 != ILM_ERR_NOT_CONVERGED) return cg2;
-  ILM_TRY(st_convert(N, ILM_F64, x64, c->dtype, ds_out, st));
+  if (!direct) ILM_TRY(st_convert(N, ILM_F64, x64, c->dtype, ds_out, st));
   ILM_TRY(ilm_surface_curl(c, 0, ILM_SCALAR_DATA, df_out, s_out, stream));   // s*
   ILM_TRY(ilm_surface_curl_cross(c, 0, ds_out, corr, stream));               // C^x_s^T ds (Nodes{Dual})
   ILM_TRY(st_axpby(nd, c->dtype, 1.0, s_out, -1.0, corr, corr, st));

@@ -715,6 +715,8 @@ int st_grad_edges(const ilm_grid_s* g, int dtype, const void* q, void* t, double
 int st_div_edgegrad(const ilm_grid_s* g, int dtype, const void* t, void* q, double scale, cudaStream_t st);
 int st_laplacian(int n1, int n2, int dtype, const void* in, void* out, double scale, cudaStream_t st);
 int st_axpby(size_t n, int dtype, double a, const void* x, double b, const void* y, void* out, cudaStream_t st);
+int st_jump_average(size_t n, int dtype, const void* plus, const void* minus, void* jump, void* avg, cudaStream_t st);
+int st_difference64(size_t n, int dtype, const void* a, const void* b, double* out, cudaStream_t st);
 int st_fill(size_t n, int dtype, double v, void* out, cudaStream_t st);
 int st_affine(size_t n, int dtype, double a, const void* x, double b, void* out, cudaStream_t st);
 int st_convert(size_t n, int dtype_in, const void* in, int dtype_out, void* out, cudaStream_t st);

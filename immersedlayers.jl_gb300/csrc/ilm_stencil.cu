@@ -414,6 +414,24 @@ __global__ void k_mul_add(size_t n, const T* __restrict__ a, const T* __restrict
     out[i] += a[i] * b[i];
 }
 
+// surface jump and average of the two sides' data (one launch, not two)
+template <typename T>
+__global__ void k_jump_average(size_t n, const T* __restrict__ p, const T* __restrict__ m, T* __restrict__ jump,
+                               T* __restrict__ avg) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const T a = p[i], b = m[i];
+    jump[i] = a - b;
+    avg[i] = (T)0.5 * a + (T)0.5 * b;
+  }
+}
+
+// a - b, rounded in the cache's type, as FP64
+template <typename T>
+__global__ void k_difference64(size_t n, const T* __restrict__ a, const T* __restrict__ b, double* __restrict__ out) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+    out[i] = (double)(T)(a[i] - b[i]);
+}
+
 template <typename T>
 __global__ void k_axpby(size_t n, T a, const T* __restrict__ x, T b, const T* __restrict__ y, T* __restrict__ o) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -662,6 +680,25 @@ int st_axpby(size_t n, int dtype, double a, const void* x, double b, const void*
   DISPATCH(dtype, {
     k_axpby<T><<<nblocks(n), 256, 0, st>>>(n, (T)a, static_cast<const T*>(x), (T)b, static_cast<const T*>(y),
                                            static_cast<T*>(out));
+  });
+  ILM_CHECK_LAUNCH();
+  return ILM_OK;
+}
+
+int st_jump_average(size_t n, int dtype, const void* plus, const void* minus, void* jump, void* avg, cudaStream_t st) {
+  if (n == 0) return ILM_OK;
+  DISPATCH(dtype, {
+    k_jump_average<T><<<nblocks(n), 256, 0, st>>>(n, static_cast<const T*>(plus), static_cast<const T*>(minus),
+                                                  static_cast<T*>(jump), static_cast<T*>(avg));
+  });
+  ILM_CHECK_LAUNCH();
+  return ILM_OK;
+}
+
+int st_difference64(size_t n, int dtype, const void* a, const void* b, double* out, cudaStream_t st) {
+  if (n == 0) return ILM_OK;
+  DISPATCH(dtype, {
+    k_difference64<T><<<nblocks(n), 256, 0, st>>>(n, static_cast<const T*>(a), static_cast<const T*>(b), out);
   });
   ILM_CHECK_LAUNCH();
   return ILM_OK;
