@@ -266,34 +266,31 @@ __global__ void k_conv_gather2(int N, int n1, int n2, const T* __restrict__ f, i
   if (lane == 0) (set ? out1 : out0)[k] = acc;
 }
 
-// y = S x for a CSR float-float matrix (FP64 accumulation), one warp per row
-__global__ void k_spmv_ff(int n, const int* __restrict__ rowptr, const int* __restrict__ col,
-                          const float* __restrict__ vhi, const float* __restrict__ vlo, const double* __restrict__ x,
-                          double* __restrict__ y) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (warp >= n) return;
-  double acc = 0.0;
-  for (int e = rowptr[warp] + lane; e < rowptr[warp + 1]; e += 32)
-    acc += ((double)vhi[e] + (double)vlo[e]) * x[col[e]];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-  if (lane == 0) y[warp] = acc;
-}
-
-// stage right-hand sides.  rhs = (avg - (g + sum_t c_t v_t)) / denom
+// Stage right-hand sides, a warp per point: rhs = (avg - (g + c0 v0 + c1 S x +
+// c2 v2)) / denom, S a stage matrix in CSR (rowptr null: without its term and
+// the next)
 __global__ void k_stage_rhs(int n, const double* __restrict__ avg, const double* __restrict__ g, double c0,
-                            const double* __restrict__ v0, double c1, const double* __restrict__ v1, double c2,
-                            const double* __restrict__ v2, double c3, const double* __restrict__ v3, double inv_denom,
+                            const double* __restrict__ v0, double c1, const int* __restrict__ rowptr,
+                            const int* __restrict__ col, const float* __restrict__ vhi, const float* __restrict__ vlo,
+                            const double* __restrict__ x, double c2, const double* __restrict__ v2, double inv_denom,
                             double* __restrict__ rhs) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
   if (k >= n) return;
-  double s = g[k];
-  if (v0) s += c0 * v0[k];
-  if (v1) s += c1 * v1[k];
-  if (v2) s += c2 * v2[k];
-  if (v3) s += c3 * v3[k];
-  rhs[k] = (avg[k] - s) * inv_denom;
+  double q = 0.0;
+  if (rowptr) {
+    for (int e = rowptr[k] + lane; e < rowptr[k + 1]; e += 32) q += ((double)vhi[e] + (double)vlo[e]) * x[col[e]];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) q += __shfl_down_sync(0xffffffffu, q, o);
+  }
+  if (lane == 0) {
+    double s = g[k] + c0 * v0[k];
+    if (rowptr) {
+      s += c1 * q;
+      s += c2 * v2[k];
+    }
+    rhs[k] = (avg[k] - s) * inv_denom;
+  }
 }
 
 }  // namespace
@@ -322,7 +319,7 @@ struct ilm_heat_s {
   DevBuf rowptr[4], colidx[4], vhi[4], vlo[4];
   size_t nnz[4] = {0, 0, 0, 0};
   DevBuf e[4], avg64, cfield;
-  DevBuf g1, g3, rhs, q1, q2, sig[3], sig_t;
+  DevBuf g1, g3, rhs, sig[3], sig_t;
   DevBuf tmp[4];
   DevBuf cgs, iters, relres;
   CG64Inverse inv[3];             // FP32 inverses of the three stage systems
@@ -582,8 +579,6 @@ int ilm_heat_create(ilm_cache_t c, double kappa, double dt, const double* tb_plu
   ILM_TRY(H->g1.alloc((size_t)N * 8));
   ILM_TRY(H->g3.alloc((size_t)N * 8));
   ILM_TRY(H->rhs.alloc((size_t)N * 8 * 3));
-  ILM_TRY(H->q1.alloc((size_t)N * 8));
-  ILM_TRY(H->q2.alloc((size_t)N * 8));
   for (int s = 0; s < 3; ++s) {
     ILM_TRY(H->sig[s].alloc((size_t)N * 8));
     ILM_CHECK_CUDA(cudaMemset(H->sig[s].p, 0, (size_t)N * 8));
@@ -612,7 +607,6 @@ int ilm_heat_advance(ilm_heat_t H, void* T, void* sigma_out, int nsteps, ilm_str
   const int N = c->npts;
   const double dt = H->dt;
   const int wb = (2 * N * 32 + 255) / 256;
-  const int pb = (N + 255) / 256;
   const int sb = (N * 32 + 255) / 256;
   double* rhs = H->rhs.as<double>();
   for (int step = 0; step < nsteps; ++step) {
@@ -631,33 +625,34 @@ int ilm_heat_advance(ilm_heat_t H, void* T, void* sigma_out, int nsteps, ilm_str
                                                  H->gwy[1].as<double>(), H->g3.as<double>());
     ILM_CHECK_LAUNCH();
     // stage 2: S_{a/3} sigma1 = (avg - g1 - dt a21 e_{a/3}) / (dt a21)
-    k_stage_rhs<<<pb, 256, 0, st>>>(N, H->avg64.as<double>(), H->g1.as<double>(), dt * H->a21, H->e[0].as<double>(),
-                                     0.0, nullptr, 0.0, nullptr, 0.0, nullptr, 1.0 / (dt * H->a21), rhs);
+    k_stage_rhs<<<sb, 256, 0, st>>>(N, H->avg64.as<double>(), H->g1.as<double>(), dt * H->a21, H->e[0].as<double>(),
+                                     0.0, nullptr, nullptr, nullptr, nullptr, nullptr, 0.0, nullptr,
+                                     1.0 / (dt * H->a21), rhs);
     ILM_CHECK_LAUNCH();
     ILM_TRY(run_cg(H, 0, st));
     // stage 3: S_{2a/3} sigma2 = (avg - [g3 + dt a31 (e_a + S_a sigma1) + dt a32 e_{2a/3}]) / (dt a32)
-    k_spmv_ff<<<sb, 256, 0, st>>>(N, H->rowptr[2].as<int>(), H->colidx[2].as<int>(), H->vhi[2].as<float>(),
-                                  H->vlo[2].as<float>(), H->sig[0].as<double>(), H->q1.as<double>());
-    ILM_CHECK_LAUNCH();
-    k_stage_rhs<<<pb, 256, 0, st>>>(N, H->avg64.as<double>(), H->g3.as<double>(), dt * H->a31, H->e[2].as<double>(),
-                                     dt * H->a31, H->q1.as<double>(), dt * H->a32, H->e[1].as<double>(), 0.0, nullptr,
-                                     1.0 / (dt * H->a32), rhs + N);
+    k_stage_rhs<<<sb, 256, 0, st>>>(N, H->avg64.as<double>(), H->g3.as<double>(), dt * H->a31, H->e[2].as<double>(),
+                                     dt * H->a31, H->rowptr[2].as<int>(), H->colidx[2].as<int>(),
+                                     H->vhi[2].as<float>(), H->vlo[2].as<float>(), H->sig[0].as<double>(), dt * H->a32,
+                                     H->e[1].as<double>(), 1.0 / (dt * H->a32), rhs + N);
     ILM_CHECK_LAUNCH();
     ILM_TRY(run_cg(H, 1, st));
     // final: S_0 sigma3 = (avg - [g3 + dt b2 (e_{2a/3} + S_{2a/3} sigma2) + dt b3 e_0]) / (dt b3)   (b1 = 0)
-    k_spmv_ff<<<sb, 256, 0, st>>>(N, H->rowptr[1].as<int>(), H->colidx[1].as<int>(), H->vhi[1].as<float>(),
-                                  H->vlo[1].as<float>(), H->sig[1].as<double>(), H->q2.as<double>());
-    ILM_CHECK_LAUNCH();
-    k_stage_rhs<<<pb, 256, 0, st>>>(N, H->avg64.as<double>(), H->g3.as<double>(), dt * H->b2, H->e[1].as<double>(),
-                                     dt * H->b2, H->q2.as<double>(), dt * H->b3, H->e[3].as<double>(), 0.0, nullptr,
-                                     1.0 / (dt * H->b3), rhs + 2 * N);
+    k_stage_rhs<<<sb, 256, 0, st>>>(N, H->avg64.as<double>(), H->g3.as<double>(), dt * H->b2, H->e[1].as<double>(),
+                                     dt * H->b2, H->rowptr[1].as<int>(), H->colidx[1].as<int>(),
+                                     H->vhi[1].as<float>(), H->vlo[1].as<float>(), H->sig[1].as<double>(), dt * H->b3,
+                                     H->e[3].as<double>(), 1.0 / (dt * H->b3), rhs + 2 * N);
     ILM_CHECK_LAUNCH();
     ILM_TRY(run_cg(H, 2, st));
     // grid: T <- exp(aL) T + dt b2 exp(2a/3 L) R sigma2 + dt b3 R sigma3 + cfield
-    ILM_TRY(st_convert(N, ILM_F64, H->sig[1].p, c->dtype, H->sig_t.p, st));
-    ILM_TRY(ilm_regularize(c, ILM_NODES_PRIMAL, H->sig_t.p, H->tmp[2].p, st));
-    ILM_TRY(st_convert(N, ILM_F64, H->sig[2].p, c->dtype, H->sig_t.p, st));
-    ILM_TRY(ilm_regularize(c, ILM_NODES_PRIMAL, H->sig_t.p, H->tmp[3].p, st));
+    for (int k = 1; k <= 2; ++k) {
+      const void* sig = H->sig[k].p;
+      if (c->dtype != ILM_F64) {
+        ILM_TRY(st_convert(N, ILM_F64, sig, c->dtype, H->sig_t.p, st));
+        sig = H->sig_t.p;
+      }
+      ILM_TRY(ilm_regularize(c, ILM_NODES_PRIMAL, sig, H->tmp[k + 1].p, st));
+    }
     ILM_TRY((c->dtype == ILM_F64 ? apply_if<double> : apply_if<float>)(H, 2, T, H->tmp[0].p, 1, dt * H->b2, H->tmp[2].p,
                                                                        H->tmp[1].p, dt * H->b3, H->tmp[3].p,
                                                                        H->cfield.p, T, st));
