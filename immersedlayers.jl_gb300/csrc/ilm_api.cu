@@ -86,9 +86,8 @@ static int scatter_scalar(ilm_cache_s* c, int pc, const void* f, int coef, void*
 // Edges{Primal} <- (a_u in1u + b_u in2u, a_v in1v + b_v in2v)
 static int scatter_edges(ilm_cache_s* c, const void* u1, int cu1, const void* u2, int cu2, const void* v1, int cv1,
                          const void* v2, int cv2, void* out, cudaStream_t st) {
-  ILM_TRY(launch_scatter(c, PC_U, u1, cu1, u2, cu2, out, st));
   void* vout = comp_ptr(&c->grid, ILM_EDGES_PRIMAL, c->dtype, out, 1);
-  return launch_scatter(c, PC_V, v1, cv1, v2, cv2, vout, st);
+  return launch_scatter_edges(c, u1, cu1, u2, cu2, out, v1, cv1, v2, cv2, vout, st);
 }
 
 static int normal_scatter_edges(ilm_cache_s* c, const void* f, void* out, cudaStream_t st) {

@@ -264,22 +264,33 @@ k_scatter(int n1, int n2, int ntx, const int* __restrict__ ne, const int* __rest
 // write zeros into the empty tiles, SCAT_TPB consecutive tiles (row-major
 // tile ids) each, skipping the occupied ones.  Every tile is written by
 // exactly one block; the long occupied-tile blocks start first and the zero
-// fill's bandwidth overlaps their load latency.
+// fill's bandwidth overlaps their load latency.  Both components of an edge
+// field go in one launch (blockIdx.y): 6 us each, mostly latency, on small grids.
 constexpr int SCAT_TPB = 32;
 template <typename T>
+struct ScatterJob {
+  int n1, n2, ntx, ntiles, nocc;
+  const int *ne, *ne_cnt, *ptr, *pts, *bx, *by;
+  const T *wx, *wy, *in1, *in2;
+  int c1, c2;
+  T* out;
+};
+template <typename T>
 __global__ void __launch_bounds__(TILE_X* TILE_Y, 6)
-k_scatter_all(int n1, int n2, int ntx, int ntiles, int nocc, const int* __restrict__ ne,
-              const int* __restrict__ ne_cnt, const int* __restrict__ tptr, const int* __restrict__ tpts,
-              const int* __restrict__ bx, const int* __restrict__ by, const T* __restrict__ wx,
-              const T* __restrict__ wy, const T* __restrict__ wsc, const T* __restrict__ nx,
-              const T* __restrict__ ny, const T* __restrict__ in1, int c1, const T* __restrict__ in2, int c2,
-              T* __restrict__ out) {
+k_scatter_all(const ScatterJob<T> j0, const ScatterJob<T> j1, const T* __restrict__ wsc, const T* __restrict__ nx,
+              const T* __restrict__ ny) {
   __shared__ int s_ptr[SCAT_TPB + 1];
   __shared__ ScatterSmem<T> sm;
   pdl_begin();
+  const bool second = blockIdx.y != 0;
+  const int n1 = second ? j1.n1 : j0.n1, n2 = second ? j1.n2 : j0.n2, ntx = second ? j1.ntx : j0.ntx;
+  const int ntiles = second ? j1.ntiles : j0.ntiles, nocc = second ? j1.nocc : j0.nocc;
+  const int* __restrict__ tptr = second ? j1.ptr : j0.ptr;
+  T* __restrict__ out = second ? j1.out : j0.out;
   const int tid = threadIdx.y * TILE_X + threadIdx.x;
   if ((int)blockIdx.x >= nocc) {  // zero writer
     const int t0 = ((int)blockIdx.x - nocc) * SCAT_TPB;
+    if (t0 >= ntiles) return;  // (the other component has more tiles)
     if (tid <= SCAT_TPB) s_ptr[tid] = tptr[min(t0 + tid, ntiles)];
     __syncthreads();
     const int nt = min(SCAT_TPB, ntiles - t0);
@@ -296,12 +307,15 @@ k_scatter_all(int n1, int n2, int ntx, int ntiles, int nocc, const int* __restri
     }
     return;
   }
-  if ((int)blockIdx.x >= *ne_cnt) return;  // launched for an upper bound after a device re-binning
-  const int t = ne[blockIdx.x];
+  // (launched for an upper bound after a device re-binning)
+  if ((int)blockIdx.x >= *(second ? j1.ne_cnt : j0.ne_cnt)) return;
+  const int t = (second ? j1.ne : j0.ne)[blockIdx.x];
   const int x0 = (t % ntx) * TILE_X, y0 = (t / ntx) * TILE_Y;
   const int i = x0 + threadIdx.x, j = y0 + threadIdx.y;
-  const T acc = occupied_tile_sum<T>(sm, tptr[t], tptr[t + 1], x0, i, j, tpts, bx, by, wx, wy, wsc, nx, ny, in1, c1,
-                                     in2, c2);
+  const T acc = occupied_tile_sum<T>(sm, tptr[t], tptr[t + 1], x0, i, j, second ? j1.pts : j0.pts,
+                                     second ? j1.bx : j0.bx, second ? j1.by : j0.by, second ? j1.wx : j0.wx,
+                                     second ? j1.wy : j0.wy, wsc, nx, ny, second ? j1.in1 : j0.in1,
+                                     second ? j1.c1 : j0.c1, second ? j1.in2 : j0.in2, second ? j1.c2 : j0.c2);
   if (i < n1 && j < n2) out[(size_t)j * n1 + i] = acc;
 }
 
@@ -380,33 +394,63 @@ int fill_zero(void* out, size_t bytes, cudaStream_t st) {
   return ILM_OK;
 }
 
+template <typename T>
+static ScatterJob<T> scatter_job(ilm_cache_s* c, int pc, const void* in1, int coef1, const void* in2, int coef2,
+                                 void* out) {
+  const Shape2 sh = c->grid.shape(pc);
+  const TileList& tl = c->tiles[pc];
+  const int dx = pc_dx(pc), dy = pc_dy(pc);
+  return ScatterJob<T>{sh.n1,
+                       sh.n2,
+                       tl.ntx,
+                       tl.ntx * tl.nty,
+                       tl.nne_launch,
+                       tl.ne.as<int>(),
+                       tl.ne_cnt.as<int>(),
+                       tl.ptr.as<int>(),
+                       tl.pts.as<int>(),
+                       c->bx[dx].as<int>(),
+                       c->by[dy].as<int>(),
+                       c->wx[dx].as<T>(),
+                       c->wy[dy].as<T>(),
+                       static_cast<const T*>(in1),
+                       static_cast<const T*>(in2),
+                       coef1,
+                       coef2,
+                       static_cast<T*>(out)};
+}
+
+template <typename T>
+static int run_scatter_all(ilm_cache_s* c, const ScatterJob<T>& a, const ScatterJob<T>* b, cudaStream_t st) {
+  auto blocks = [](const ScatterJob<T>& J) { return J.ntiles ? J.nocc + (J.ntiles + SCAT_TPB - 1) / SCAT_TPB : 0; };
+  const int nb = std::max(blocks(a), b ? blocks(*b) : 0);
+  if (nb == 0) return ILM_OK;
+  ILM_CHECK_CUDA(launch_pdl(k_scatter_all<T>, dim3(nb, b ? 2 : 1), dim3(TILE_X, TILE_Y), st, a, b ? *b : a,
+                            c->wscale.as<T>(), c->nx.as<T>(), c->ny.as<T>()));
+  return ILM_OK;
+}
+
+// both components of an edge field (overwriting)
+int launch_scatter_edges(ilm_cache_s* c, const void* u1, int cu1, const void* u2, int cu2, void* u_out, const void* v1,
+                         int cv1, const void* v2, int cv2, void* v_out, cudaStream_t st) {
+  if (c->dtype == ILM_F64) {
+    const auto b = scatter_job<double>(c, PC_V, v1, cv1, v2, cv2, v_out);
+    return run_scatter_all(c, scatter_job<double>(c, PC_U, u1, cu1, u2, cu2, u_out), &b, st);
+  }
+  const auto b = scatter_job<float>(c, PC_V, v1, cv1, v2, cv2, v_out);
+  return run_scatter_all(c, scatter_job<float>(c, PC_U, u1, cu1, u2, cu2, u_out), &b, st);
+}
+
 int launch_scatter(ilm_cache_s* c, int pc, const void* in1, int coef1, const void* in2, int coef2, void* out,
                    cudaStream_t st, bool accumulate) {
   const Shape2 sh = c->grid.shape(pc);
   const TileList& tl = c->tiles[pc];
   const int dx = pc_dx(pc), dy = pc_dy(pc);
   dim3 blk(TILE_X, TILE_Y);
-  if (!accumulate) {
-    // overwrite: one launch over every tile (zeros where no point reaches)
-    const int ntiles = tl.ntx * tl.nty;
-    if (ntiles == 0) return ILM_OK;
-    const int nocc = tl.nne_launch;
-    const int nb = nocc + (ntiles + SCAT_TPB - 1) / SCAT_TPB;
+  if (!accumulate) {  // overwrite: one launch over every tile (zeros where no point reaches)
     if (c->dtype == ILM_F64)
-      ILM_CHECK_CUDA(launch_pdl(k_scatter_all<double>, dim3(nb), blk, st, sh.n1, sh.n2, tl.ntx, ntiles, nocc,
-                                tl.ne.as<int>(), tl.ne_cnt.as<int>(), tl.ptr.as<int>(), tl.pts.as<int>(),
-                                c->bx[dx].as<int>(), c->by[dy].as<int>(), c->wx[dx].as<double>(),
-                                c->wy[dy].as<double>(), c->wscale.as<double>(), c->nx.as<double>(),
-                                c->ny.as<double>(), static_cast<const double*>(in1), coef1,
-                                static_cast<const double*>(in2), coef2, static_cast<double*>(out)));
-    else
-      ILM_CHECK_CUDA(launch_pdl(k_scatter_all<float>, dim3(nb), blk, st, sh.n1, sh.n2, tl.ntx, ntiles, nocc,
-                                tl.ne.as<int>(), tl.ne_cnt.as<int>(), tl.ptr.as<int>(), tl.pts.as<int>(),
-                                c->bx[dx].as<int>(), c->by[dy].as<int>(), c->wx[dx].as<float>(),
-                                c->wy[dy].as<float>(), c->wscale.as<float>(), c->nx.as<float>(),
-                                c->ny.as<float>(), static_cast<const float*>(in1), coef1,
-                                static_cast<const float*>(in2), coef2, static_cast<float*>(out)));
-    return ILM_OK;
+      return run_scatter_all<double>(c, scatter_job<double>(c, pc, in1, coef1, in2, coef2, out), nullptr, st);
+    return run_scatter_all<float>(c, scatter_job<float>(c, pc, in1, coef1, in2, coef2, out), nullptr, st);
   }
   // accumulate: the occupied tiles only (the others add nothing)
   const int nb = tl.nne_launch;

@@ -699,6 +699,8 @@ int cache_rebin_points(ilm_cache_s* c, const double* x, const double* y, const d
                        const double* ds, cudaStream_t st);
 int cache_sync_host(ilm_cache_s* c);
 // out_pc(cell) = sum_k w_k (a_k in1_k + b_k in2_k) phi phi ; in2 may be null
+int launch_scatter_edges(ilm_cache_s* c, const void* u1, int cu1, const void* u2, int cu2, void* u_out, const void* v1,
+                         int cv1, const void* v2, int cv2, void* v_out, cudaStream_t st);
 int launch_scatter(ilm_cache_s* c, int pc, const void* in1, int coef1, const void* in2, int coef2,
                    void* out, cudaStream_t st, bool accumulate = false);
 // out_k (+)= sum_t coef_t * E_{pc_t} arr_t
