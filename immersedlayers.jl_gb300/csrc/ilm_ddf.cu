@@ -275,14 +275,14 @@ struct ScatterJob {
   int c1, c2;
   T* out;
 };
-template <typename T>
+template <typename T, bool TWO>
 __global__ void __launch_bounds__(TILE_X* TILE_Y, 6)
 k_scatter_all(const ScatterJob<T> j0, const ScatterJob<T> j1, const T* __restrict__ wsc, const T* __restrict__ nx,
               const T* __restrict__ ny) {
   __shared__ int s_ptr[SCAT_TPB + 1];
   __shared__ ScatterSmem<T> sm;
   pdl_begin();
-  const bool second = blockIdx.y != 0;
+  const bool second = TWO && blockIdx.y != 0;
   const int n1 = second ? j1.n1 : j0.n1, n2 = second ? j1.n2 : j0.n2, ntx = second ? j1.ntx : j0.ntx;
   const int ntiles = second ? j1.ntiles : j0.ntiles, nocc = second ? j1.nocc : j0.nocc;
   const int* __restrict__ tptr = second ? j1.ptr : j0.ptr;
@@ -425,8 +425,8 @@ static int run_scatter_all(ilm_cache_s* c, const ScatterJob<T>& a, const Scatter
   auto blocks = [](const ScatterJob<T>& J) { return J.ntiles ? J.nocc + (J.ntiles + SCAT_TPB - 1) / SCAT_TPB : 0; };
   const int nb = std::max(blocks(a), b ? blocks(*b) : 0);
   if (nb == 0) return ILM_OK;
-  ILM_CHECK_CUDA(launch_pdl(k_scatter_all<T>, dim3(nb, b ? 2 : 1), dim3(TILE_X, TILE_Y), st, a, b ? *b : a,
-                            c->wscale.as<T>(), c->nx.as<T>(), c->ny.as<T>()));
+  ILM_CHECK_CUDA(launch_pdl(b ? k_scatter_all<T, true> : k_scatter_all<T, false>, dim3(nb, b ? 2 : 1),
+                            dim3(TILE_X, TILE_Y), st, a, b ? *b : a, c->wscale.as<T>(), c->nx.as<T>(), c->ny.as<T>()));
   return ILM_OK;
 }
 
