@@ -1,6 +1,6 @@
 // FP32 LGF convolution of one field (the operators and solves of a cache): the
-// three passes of ilm_fft.cu for padded sizes from 64 to 8192, with no job
-// table to upload and two to four register stages per transform.
+// three passes of ilm_fft.cu for padded sizes from 2048 to 8192, with no job
+// table to upload and three or four register stages per transform.
 //
 // A transform of L points runs on L / E threads, each with E = 16 (L = 2^a) or
 // 24 (3 * 2^a) values in registers: a stage is E / R DFTs of R points (R = 4 to
@@ -17,9 +17,8 @@
 //     loaded nor stored.
 // The batched passes hold a transform in two steps of up to 32 points per
 // thread, which ends at 1024 points (beyond, radix-4 stages between two shared
-// buffers).  Measured, us per field: 105^2 23 -> 17, 257^2 33 -> 21, 405^2 37 ->
-// 19, 600^2 92 -> 31, 1023^2 179 -> 38, 2047^2 495 -> 152; the data stay in L2, the
-// exchanges and FP32 issue bound the passes.
+// buffers).  Measured, us per field: 1023^2 179 -> 38, 2047^2 495 -> 152; the data
+// stay in L2, the exchanges and FP32 issue bound the passes.
 #include <algorithm>
 
 #include "ilm_fftcore.cuh"
@@ -33,14 +32,6 @@ struct Stages {
 };
 constexpr Stages stages_of(int L) {
   switch (L) {
-    case 64: return {16, {16, 4, 0, 0}};
-    case 96: return {24, {8, 12, 0, 0}};
-    case 128: return {16, {16, 8, 0, 0}};
-    case 192: return {24, {8, 24, 0, 0}};
-    case 256: return {16, {16, 16, 0, 0}};
-    case 384: return {24, {8, 4, 12, 0}};
-    case 512: return {16, {16, 8, 4, 0}};
-    case 768: return {24, {8, 8, 12, 0}};
     case 1024: return {16, {16, 8, 8, 0}};
     case 1536: return {24, {8, 8, 24, 0}};
     case 2048: return {16, {16, 16, 8, 0}};
@@ -293,14 +284,6 @@ int run_cols(const FieldJob& J, int ncols, cudaStream_t st) {
 
 int rows_any(int H, const FieldJob& J, bool inverse, cudaStream_t st) {
   switch (H) {
-    case 64: return run_rows<64>(J, inverse, st);
-    case 96: return run_rows<96>(J, inverse, st);
-    case 128: return run_rows<128>(J, inverse, st);
-    case 192: return run_rows<192>(J, inverse, st);
-    case 256: return run_rows<256>(J, inverse, st);
-    case 384: return run_rows<384>(J, inverse, st);
-    case 512: return run_rows<512>(J, inverse, st);
-    case 768: return run_rows<768>(J, inverse, st);
     case 1024: return run_rows<1024>(J, inverse, st);
     case 1536: return run_rows<1536>(J, inverse, st);
     case 2048: return run_rows<2048>(J, inverse, st);
@@ -312,16 +295,6 @@ int rows_any(int H, const FieldJob& J, bool inverse, cudaStream_t st) {
 
 int cols_any(int L, const FieldJob& J, int ncols, cudaStream_t st) {
   switch (L) {
-    case 64: return run_cols<64>(J, ncols, st);
-    case 96: return run_cols<96>(J, ncols, st);
-    case 128: return run_cols<128>(J, ncols, st);
-    case 192: return run_cols<192>(J, ncols, st);
-    case 256: return run_cols<256>(J, ncols, st);
-    case 384: return run_cols<384>(J, ncols, st);
-    case 512: return run_cols<512>(J, ncols, st);
-    case 768: return run_cols<768>(J, ncols, st);
-    case 1024: return run_cols<1024>(J, ncols, st);
-    case 1536: return run_cols<1536>(J, ncols, st);
     case 2048: return run_cols<2048>(J, ncols, st);
     case 3072: return run_cols<3072>(J, ncols, st);
     case 4096: return run_cols<4096>(J, ncols, st);
@@ -332,10 +305,15 @@ int cols_any(int L, const FieldJob& J, int ncols, cudaStream_t st) {
 
 }  // namespace
 
-// P1 / 2 and P2 are 2^a or 3 * 2^a (good_fft_size)
+// P1 / 2 and P2 are 2^a or 3 * 2^a (good_fft_size).  Below 2048 points the passes
+// of ilm_fft.cu stay although these would be faster (405^2 37 and 19 us, 600^2 92
+// and 31): where a result cancels (the surface values of a smooth double layer on
+// one nearly circular body are 1/200 of the field), another order of the FP32
+// roundings moves it by up to 2e-4 there, by some 1e-5 from 2048 points on; the
+// errors against 64 bits are the same.
 bool field_conv_supported(int P1, int P2) {
   const int H = P1 / 2;
-  return H >= 64 && H <= 4096 && P2 >= 64 && P2 <= 6144;
+  return H >= 1024 && H <= 4096 && P2 >= 2048 && P2 <= 6144;
 }
 
 int field_conv_apply(ConvPlan* p, const float* in, float* out, double scale, cudaStream_t st) {
