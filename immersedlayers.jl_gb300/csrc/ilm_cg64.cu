@@ -16,7 +16,9 @@
 // with FP64 residuals: x += P (b - S x).  Each step gains cond(S) eps_32, so a
 // few steps, each one product with S and one (cheap) with P, replace the ~60
 // to ~300 iterations; the residual that is tested is the FP64 one.  Where a
-// step gains less than a factor of four the CG goes on from there.
+// step gains less than a factor of four the CG goes on from there.  The
+// correction that follows the residual that passes stays if its own residual
+// passes too (that is the one reported), else it is taken back.
 //
 // Two exchanges: a single cluster of 16 CTAs (rows written straight into the
 // other CTAs' shared memory, hardware cluster barrier), and a cooperative
@@ -64,7 +66,7 @@ struct CG64Args {
   int ld;           // row stride of the resident dense slab (doubles)
   int slab_nnz;     // CSR: entries of the largest slab
   int nv;           // stride of the shared-memory vectors (n rounded up to 4)
-  double* gq;       // grid variant: exchange (two vectors of n doubles, two sums per CTA)
+  double* gq;       // grid variant: exchange (two vectors of n doubles, three sums per CTA)
   CG64State* state;
 };
 
@@ -76,7 +78,7 @@ __device__ __forceinline__ double warp_sum(double v) {
 
 // shared-memory scalars: [0, 8) and [8, 16) warp partials, then the results
 struct Scal {
-  double part[16];
+  double part[C64_CLUSTER];
   float part32[8];
   double a, b, c;   // first sum, second sum, derived scalar
   unsigned top;     // refinement: largest magnitude bits of b
@@ -291,12 +293,14 @@ __global__ void __launch_bounds__(C64_T, 1) k_cg64(const CG64Args A) {
     // sends W r, in FP32, and x: two barriers per step.  The norm of a residual is
     // summed beside the product with P and judged beside the next residual's, by
     // the last warp, off the chain of the others: so the correction after the
-    // residual that passes is always taken.  It is wanted: that residual is rich in
-    // the modes that P gets least right, the slow ones, and x is further off for it
-    // than a CG iterate of that residual (steps gained a factor of four so far).
+    // residual that passes is always taken, and its residual is there.  It is
+    // wanted: the residual that passes is rich in the modes that P gets least right,
+    // the slow ones, and x is further off for it than a CG iterate of that residual.
+    // Nothing says that P contracts on it, so its residual decides (1.3 us of a
+    // solve on the grid, 2 on the cluster).
     float* v = reinterpret_cast<float*>(p);               // W r scaled into FP32's range
     float* gv = reinterpret_cast<float*>(A.gq + n);       // grid: its exchange
-    double* gs = A.gq + 2 * (size_t)n;                    // grid: the CTAs' sums
+    double* gs = A.gq + 2 * (size_t)n;                    // grid: the CTAs' sums (three each)
     const int lane = t & 31, warp = t >> 5;
     const float kappa = P.invs[1];
     if (t == 0) s.top = 0u;
@@ -430,6 +434,51 @@ __global__ void __launch_bounds__(C64_T, 1) k_cg64(const CG64Args A) {
       barrier();
       if (!ok) break;
       gather_x();
+    }
+    if (ok && flags == DONE) {
+      // the residual of the x that has had one correction more (other CTAs may
+      // still read the sums of the round before: not through tot)
+      if (warp == LAST) {
+        double a = 0.0;
+        for (int i = lane; i < nr; i += 32) a = fma(r[r0 + i], r[r0 + i], a);
+        send(s.part, gs + 2 * G, rank, warp_sum(a), lane, 32);
+      }
+      if (GRID) {  // no CTA waits: the last to arrive decides, and takes x back where it has to
+        for (int i = t; i < nr; i += C64_T) {
+          P.x[r0 + i] = x[r0 + i];
+          __stcg(A.gq + n + r0 + i, old[i]);
+        }
+        __syncthreads();
+        if (t == 0) {
+          __threadfence();
+          s_ok = atomicAdd(&A.state->finished, 1u) + 1 == (unsigned)G;
+          __threadfence();
+        }
+        __syncthreads();
+        if (!s_ok) return;
+      } else {
+        barrier();
+      }
+      if (warp == LAST) {
+        double a = 0.0;
+        for (int k = lane; k < G; k += 32) a += GRID ? __ldcg(gs + 2 * G + k) : s.part[k];
+        const double now = warp_sum(a);
+        if (lane == 0) {
+          if (converged(now)) s.a = now;
+          else s.flag = DONE | UNDO;
+        }
+      }
+      __syncthreads();
+      flags = s.flag;
+      if (GRID) {
+        if (flags & UNDO)
+          for (int j = t; j < n; j += C64_T) P.x[j] = __ldcg(A.gq + n + j);
+        if (t == 0) {
+          *P.iters = it;
+          *P.relres = fmin(sqrt(s.a / s.b), P.tol);
+        }
+        return;
+      }
     }
     if (ok) {
       done = flags & DONE;
@@ -902,7 +951,7 @@ int cg64_inverse(CG64Inverse* I, const CG64Problem& P, cudaStream_t st) {
   return ILM_OK;
 }
 
-size_t cg64_scratch_bytes(int n) { return sizeof(CG64State) + 4 * (size_t)n * sizeof(double); }
+size_t cg64_scratch_bytes(int n) { return sizeof(CG64State) + 5 * (size_t)n * sizeof(double); }
 
 bool cg64_fits(int n) { return 5 * (size_t)((n + 3) / 4 * 4) * sizeof(double) <= (size_t)C64_MAX_GRID; }
 

@@ -540,10 +540,10 @@ struct CG64Inverse {
   }
 };
 int cg64_inverse(CG64Inverse* I, const CG64Problem& P, cudaStream_t st);
-struct CG64State {                 // head of the scratch: results and the grid variant's barrier
+struct CG64State {                 // head of the scratch: results and the grid variant's counters
   int iters, timeout;
   double relres;
-  unsigned arrived, pad;
+  unsigned arrived, finished;
 };
 size_t cg64_scratch_bytes(int n);
 bool cg64_fits(int n);  // the vectors of n unknowns fit a CTA's shared memory
