@@ -1007,7 +1007,7 @@ int schur_cg(ilm_cache_s* c, int which, const double* rhs, double* x, double tol
     info->rel_residual = rr;
     info->converged = rr <= tol ? 1 : 0;
   }
-  if (rr > tol) {
+  if (!(rr <= tol)) {
     set_error("Schur CG did not reach rel. residual %g in %d iterations (%g)", tol, it, rr);
     return ILM_ERR_NOT_CONVERGED;
   }
@@ -1276,8 +1276,8 @@ static int solve_refined(ilm_cache_s* c, bool neumann, const double* fplus, cons
     double nrm[2];
     ILM_CHECK_CUDA(cudaMemcpyAsync(nrm, c->ref_norm.p, sizeof(nrm), cudaMemcpyDeviceToHost, st));
     ILM_CHECK_CUDA(cudaStreamSynchronize(st));
-    rel = nrm[1] > 0.0 ? std::sqrt(nrm[0] / nrm[1]) : 0.0;
-    if (rel <= tol || k >= max_refine) break;
+    rel = nrm[1] == 0.0 ? 0.0 : std::sqrt(nrm[0] / nrm[1]);
+    if (!(rel > tol) || k >= max_refine) break;
     // correction: S d = r by the FP64 CG, x += d
     ilm_solve_info_t ci{0, 0, 0.0};
     const int rc = schur_cg(c, neumann ? ILM_SCHUR_CLINVCT : ILM_SCHUR_RTLINVR, c->ref_r.as<double>(),
@@ -1296,7 +1296,7 @@ static int solve_refined(ilm_cache_s* c, bool neumann, const double* fplus, cons
   ILM_TRY(st_axpby(np, ILM_F64, 1.0, corr, 1.0, fstar, f_out, st));
   ILM_CHECK_CUDA(cudaStreamSynchronize(st));
   if (info) *info = ilm_solve_info_t{total_its, rel <= tol ? 1 : 0, rel};
-  if (rel > tol) {
+  if (!(rel <= tol)) {
     set_error("refined solve: FP64 Schur residual %g after %d refinement steps (target %g)", rel, max_refine, tol);
     return ILM_ERR_NOT_CONVERGED;
   }

@@ -1903,7 +1903,7 @@ int ilm_batch_solve_refined(ilm_batch_t b, const double* fplus, const double* fm
     ILM_CHECK_CUDA(cudaStreamSynchronize(st));
     double worst = 0.0;
     for (int p = 0; p < np; ++p) {
-      rel[p] = nrm[2 * p + 1] > 0.0 ? std::sqrt(nrm[2 * p] / nrm[2 * p + 1]) : 0.0;
+      rel[p] = nrm[2 * p + 1] == 0.0 ? 0.0 : std::sqrt(nrm[2 * p] / nrm[2 * p + 1]);
       worst = std::max(worst, rel[p]);
     }
     if (worst <= tol || k >= max_refine) break;

@@ -438,7 +438,7 @@ __global__ void __cluster_dims__(CG_CLUSTER, 1, 1) __launch_bounds__(CGR_THREADS
         pr_ += w[j] * p[j] * r[j];
       }
       block_sum2(pq, pr_, red);
-      if (pq == 0.0) break;
+      if (!(fabs(pq) > 0.0)) break;  // zero, or not a number
       const double alpha = fdiv(pre ? pr_ : rz, pq);
       double rr = 0.0, rzn = 0.0;
       for (int j = threadIdx.x; j < n; j += blockDim.x) {
@@ -498,7 +498,7 @@ __global__ void __cluster_dims__(CG_CLUSTER, 1, 1) __launch_bounds__(CGR_THREADS
         __syncthreads();
       }
     }
-    relres = bnorm > 0 ? sqrt(rlast) / bnorm : 0.0;
+    relres = bnorm == 0.0 ? 0.0 : sqrt(rlast) / bnorm;  // (data that are no numbers: NaN)
     if (best < relres) {  // stopped past the best iterate: return that one
       relres = best;
       cl.sync();  // every CTA's rows of the best iterate are in pr.x
@@ -1074,7 +1074,7 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(NT, MINB)
         pq = bc[3];
         alpha = bc[4];
       }
-      if (pq == 0.0) break;
+      if (!(fabs(pq) > 0.0)) break;  // zero, or not a number
       double rr, rzn, mur;  // mur: the deflation's projection of p = r + beta p
       {
         double v[3] = {0.0, 0.0, 0.0};
@@ -1197,7 +1197,7 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(NT, MINB)
       }
       __syncthreads();
     }
-    relres = bnorm > 0 ? sqrt(rlast) / bnorm : 0.0;
+    relres = bnorm == 0.0 ? 0.0 : sqrt(rlast) / bnorm;  // (data that are no numbers: NaN)
     if (best < relres) {  // stopped past the best iterate: return that one
       relres = best;
       for (int i = threadIdx.x; i < nr; i += blockDim.x) xs[i] = pr.x[r0 + i];

@@ -534,7 +534,7 @@ __global__ void __launch_bounds__(C64_T, 1) k_cg64(const CG64Args A) {
     double pq = 0.0;
     for (int j = t; j < n; j += C64_T) pq = fma(w[j] * p[j], q[j], pq);
     block_sums(pq, 0.0, false, n, s, [&](double u, double) { s.c = rz / u; });
-    if (s.a == 0.0) break;
+    if (!(fabs(s.a) > 0.0)) break;  // zero, or not a number
     const double alpha = s.c;
     double rs = 0.0, rzn = 0.0;
     for (int j = t; j < n; j += C64_T) {
@@ -548,7 +548,7 @@ __global__ void __launch_bounds__(C64_T, 1) k_cg64(const CG64Args A) {
     ++it;
     block_sums(rs, rzn, true, n, s, [&](double u, double v) {
       s.c = v / rz;
-      s.flag = below(u);
+      s.flag = below(u) || !(u <= 1.7e308);
     });
     last = s.a;
     rzn = s.b;
@@ -572,6 +572,7 @@ __global__ void __launch_bounds__(C64_T, 1) k_cg64(const CG64Args A) {
         done = true;
         break;
       }
+      if (!(last <= 1.7e308)) break;  // not a number
       if (guard) {
         const double rel = bnorm > 0 ? sqrt(last) / bnorm : 0.0;
         if (rel < best) {
@@ -588,7 +589,7 @@ __global__ void __launch_bounds__(C64_T, 1) k_cg64(const CG64Args A) {
     __syncthreads();
   }
   double relres = 0.0;
-  if (guard || (rank == 0 && t == 0)) relres = bb > 0 ? sqrt(last / bb) : 0.0;
+  if (guard || (rank == 0 && t == 0)) relres = bb == 0.0 ? 0.0 : sqrt(last / bb);  // (data that are no numbers: NaN)
   if (done) relres = fmin(relres, P.tol);  // (squares were compared)
   __syncthreads();
   if (guard && best < relres) relres = best;  // stopped past the best iterate: P.x holds it

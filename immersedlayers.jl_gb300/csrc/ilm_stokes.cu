@@ -463,8 +463,8 @@ int cg_single(int n, const BlockApply& A, const BlockPrec* M, const double* b, d
   ILM_CHECK_CUDA(cudaMemsetAsync(Yb, 0, (size_t)n * sizeof(double), st));
   ILM_TRY(precond(P));
   ILM_TRY(read());
-  if (!(h[0] > 0.0)) return ILM_OK;
-  *relres = 1.0;
+  if (h[0] == 0.0) return ILM_OK;
+  *relres = h[0] / h[0];  // 1, or NaN
   double best = 1.0;
   int it = 0, last_gain = 0;
   while (it < maxiter) {
@@ -538,7 +538,7 @@ int block_cg(int n, int s, const BlockApply& A, const BlockPrec* M, const double
   bool all_zero = true;
   for (int j = 0; j < s; ++j) {
     bn[j] = sqrt(std::max(hg[j + (size_t)j * s], 0.0));
-    relres[j] = bn[j] > 0.0 ? 1.0 : 0.0;
+    relres[j] = bn[j] == 0.0 ? 0.0 : bn[j] / bn[j];  // 1, or NaN
     all_zero = all_zero && bn[j] == 0.0;
   }
   *iters = 0;
@@ -553,7 +553,7 @@ int block_cg(int n, int s, const BlockApply& A, const BlockPrec* M, const double
     ILM_TRY(gram(R, s, R, s, n, w.G2.as<double>(), d, st));
     out.resize(s);
     for (int j = 0; j < s; ++j)
-      out[j] = bn[j] > 0.0 ? sqrt(std::max(d[j + (size_t)j * s], 0.0)) / bn[j] : 0.0;
+      out[j] = bn[j] == 0.0 ? 0.0 : sqrt(std::max(d[j + (size_t)j * s], 0.0)) / bn[j];
     return ILM_OK;
   };
   ILM_TRY(precond(R, P));
@@ -979,9 +979,9 @@ int ilm_solve_stokes_multi_refined(ilm_cache_t c, int nrhs, const double* vplus,
       bool all = true;
       double worst = 0.0;
       for (int j = 0; j < nrhs; ++j) {
-        relk[j] = bn[j] > 0.0 ? sqrt(std::max(g[j + (size_t)j * nrhs], 0.0)) / bn[j] : 0.0;
+        relk[j] = bn[j] == 0.0 ? 0.0 : sqrt(std::max(g[j + (size_t)j * nrhs], 0.0)) / bn[j];
         all = all && relk[j] <= tol;
-        worst = std::max(worst, relk[j]);
+        worst = relk[j] > worst || relk[j] != relk[j] ? relk[j] : worst;
       }
       if (!(worst < worst_prev)) {
         // the correction did not reduce the FP64 residual (the corrections'

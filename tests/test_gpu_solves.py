@@ -199,3 +199,50 @@ def test_shape_masks_area(cuda):
         comps = w.numpy_components()
         for comp in (comps if isinstance(comps, tuple) else (comps,)):
             assert abs(comp.sum() * h * h - 0.5) < 1e-3, kind.__name__
+
+
+@pytest.mark.parametrize("solve", ["dirichlet", "neumann_full", "dirichlet_refined", "neumann_refined", "stokes",
+                                   "stokes_multi", "stokes_multi_refined"])
+@pytest.mark.parametrize("n", [64, 400])
+def test_nan_is_not_converged(cuda, solve, n):
+    """One NaN in the surface data (both exchange variants of the solver): the
+    solve ends, and neither says that it converged nor gives a residual within
+    the tolerance."""
+    import torch
+    import immersedlayers as il
+    nx = max(64, int(n / 1.79))
+    g = il.PhysicalGrid.from_cells(nx, 4.0 / nx)
+    bl = il.BodyList().append(il.circle(min(1.6, n * 1.4 * g.h / (2 * np.pi)), n=n))
+    vec = solve.startswith("stokes")
+    if vec and n > 64:
+        pytest.skip("one size: the variants are those of the scalar solves")
+    d = np.cos(np.arange(2 * n if vec else n))
+    d[3] = np.nan
+    dt = torch.float32 if solve == "dirichlet_refined" else torch.float64
+    plus = torch.tensor(d, dtype=dt, device=cuda)
+    c = (il.SurfaceVectorCache if vec else il.SurfaceScalarCache)(bl, g, dtype=dt)
+    kw = dict(tol=1e-8, maxiter=200)
+    if solve == "stokes_multi" or solve == "stokes_multi_refined":
+        info = getattr(il, "solve_" + solve)(c, torch.stack([plus, torch.ones_like(plus)]), **kw)[-1][0]
+    else:
+        data = il.VectorData if vec else il.ScalarData
+        info = getattr(il, "solve_" + solve)(c, data(plus), data(torch.zeros_like(plus)), **kw)[-1]
+    assert not info["converged"] and not info["rel_residual"] <= 1e-8, info
+
+
+@pytest.mark.parametrize("variant", [1, 2, 6])
+@pytest.mark.parametrize("precond", ["none", "bjacobi"])
+def test_nan_problem_of_a_batch(cuda, variant, precond):
+    """A NaN in one problem's data: that problem's residual is no number within
+    the tolerance, the others are solved."""
+    import torch
+    from immersedlayers import workloads as W
+    from immersedlayers.batch import BatchSolver
+    bs = BatchSolver(W.batch_specs(4, sizes=(64, 96)))
+    bs.set_precond(precond, *([64] if precond == "bjacobi" else []))
+    bs.set_cg_variant(variant)
+    fp, fm = bs.surface_data()
+    fp[bs.point_offsets[1] + 5] = float("nan")
+    bs.solve(fp, fm, tol=1e-6, maxiter=500)
+    _, rr = bs.info()
+    assert not rr[1] <= 1e-6 and (np.delete(rr, 1) <= 1e-6).all(), rr
