@@ -598,26 +598,6 @@ __device__ void matvec_rows_ff(const CGFFParams& pr, int n, int r0, int r1, cons
   }
 }
 
-// v = hi + lo by integer operations (a conversion takes a slot of the FP64
-// unit), outside FP32's range by conversions
-__device__ __forceinline__ FF split_ff(double v) {
-  const unsigned h = (unsigned)__double2hiint(v), l = (unsigned)__double2loint(v);
-  const unsigned e = h >> 20 & 0x7ffu, sg = h & 0x80000000u;
-  if (e < 949u || e > 1149u) {
-    if ((h << 1 | l) == 0u) return FF{0.f, 0.f};
-    const float f = (float)v;
-    return FF{f, (float)(v - (double)f)};
-  }
-  const float hi = __uint_as_float(sg | (e - 896u) << 23 | (h & 0xfffffu) << 3 | l >> 29);
-  return ff_renorm(hi, (float)(int)(l & 0x1fffffffu) * __uint_as_float(sg | (e - 948u) << 23));
-}
-__device__ __forceinline__ double widen_any(float x) {
-  const unsigned b = __float_as_uint(x), e = b >> 23 & 0xffu;
-  if (e - 1u < 254u) return widen(x);
-  return b << 1 == 0u ? 0.0 : (double)x;
-}
-__device__ __forceinline__ double join_ff(float hi, float lo) { return widen_any(hi) + widen_any(lo); }
-
 // z[i - r0] = (W^-1 C^T C r)_i for the owned rows (float-float).  u = C r is
 // formed for every point (one thread per point, coefficient rows read from
 // L2; the same values in every CTA), so the owned rows, including those
@@ -732,7 +712,7 @@ __device__ void apply_bjacobi_rows(const CGFFParams& pr, const BJRow* __restrict
 // On return the totals are in v[] of the first warp; thread 0 derives what
 // the other threads need, stores it in the broadcast area and the caller
 // synchronises the CTA before reading it.  Each FP64 partial is split into a
-// float-float pair (~48 bits) and the sums run in FP32 float-float
+// float-float pair (49 bits) and the sums run in FP32 float-float
 // arithmetic: GB300 issues FP64 at a small fraction of the FP32 rate and a
 // chain of dependent FP64 adds costs far more latency than the same chain of
 // FP32 two-sums.  A warp sums one value of the CTA and sends it to every CTA

@@ -448,6 +448,28 @@ __device__ __forceinline__ double widen(float x) {
   return e == 0u ? 0.0 : __hiloint2double((int)((b & 0x80000000u) | (e + 896u) << 20 | (b & 0x7fffffu) >> 3), (int)(b << 29));
 }
 
+// v = hi + lo with hi rounded to nearest (2^-49 |v| at most; a truncated hi leaves
+// a remainder of 29 bits, one more than lo holds to 2^-49) by integer operations
+// (a conversion takes a slot of the FP64 unit), outside FP32's range by conversions
+__device__ __forceinline__ FF split_ff(double v) {
+  const unsigned h = (unsigned)__double2hiint(v), l = (unsigned)__double2loint(v);
+  const unsigned e = h >> 20 & 0x7ffu, sg = h & 0x80000000u;
+  if (e < 949u || e > 1149u) {
+    if ((h << 1 | l) == 0u) return FF{0.f, 0.f};
+    const float f = (float)v;
+    return FF{f, (float)(v - (double)f)};
+  }
+  const unsigned lr = l + (1u << 28), hr = (h & 0x7fffffffu) + (lr < l);  // (a carry goes on into the exponent)
+  const float hi = __uint_as_float(sg | (hr - (896u << 20)) << 3 | lr >> 29);
+  return FF{hi, (float)((int)(l << 3) >> 3) * __uint_as_float(sg | (e - 948u) << 23)};
+}
+__device__ __forceinline__ double widen_any(float x) {
+  const unsigned b = __float_as_uint(x), e = b >> 23 & 0xffu;
+  if (e - 1u < 254u) return widen(x);
+  return b << 1 == 0u ? 0.0 : (double)x;
+}
+__device__ __forceinline__ double join_ff(float hi, float lo) { return widen_any(hi) + widen_any(lo); }
+
 // acc += S * (p_hi + p_lo) with S = s_hi + s_lo
 __device__ __forceinline__ void ff_fma(FF& acc, float s_hi, float s_lo, float p_hi, float p_lo) {
   const float ph = s_hi * p_hi;
