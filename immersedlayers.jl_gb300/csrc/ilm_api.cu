@@ -969,7 +969,7 @@ int cached_schur(ilm_cache_s* c, int which, cudaStream_t st) {
     P.A = S64.as<double>();
     P.w = c->ds64.as<double>();
     P.n = c->npts;
-    ILM_TRY(cg64_inverse(&inv, P, st));
+    ILM_TRY(cg64_inverse(&inv, &c->inv_tmp, P, st));
   }
   ready = true;
   return ILM_OK;

@@ -35,6 +35,7 @@
 #include <math.h>
 
 #include <algorithm>
+#include <utility>
 
 #include "ilm_internal.cuh"
 
@@ -916,17 +917,22 @@ __global__ void __launch_bounds__(1024) k_inv_kappa(int n, int ld, const float* 
 
 }  // namespace
 
-int cg64_inverse(CG64Inverse* I, const CG64Problem& P, cudaStream_t st) {
+int cg64_inverse(CG64Inverse* I, DevBuf* tmp, const CG64Problem& P, cudaStream_t st) {
   const int n = P.n, nt = (n + GJ - 1) / GJ, ld = nt * GJ + GJ;
   const size_t bytes = (size_t)nt * GJ * ld * sizeof(float);
-  ILM_TRY(I->a.alloc(bytes));
-  ILM_TRY(I->b.alloc(bytes));
-  // scalars, two diagonal blocks, FP64 sums
-  ILM_TRY(I->s.alloc((4 + 2 * GJ * GJ) * sizeof(float) + (size_t)n * sizeof(double)));
+  I->ready = false;
+  // (scalars, two diagonal blocks, FP64 sums in s)
+  if (I->a.alloc(bytes) != ILM_OK || tmp->alloc(bytes) != ILM_OK ||
+      I->s.alloc((4 + 2 * GJ * GJ) * sizeof(float) + (size_t)n * sizeof(double)) != ILM_OK) {
+    (void)cudaGetLastError();
+    I->a.release();
+    return ILM_OK;
+  }
   float* sc = I->s.as<float>();
   float* D[2] = {sc + 4, sc + 4 + GJ * GJ};
   double* sums = reinterpret_cast<double*>(sc + 4 + 2 * GJ * GJ);
-  float* T[2] = {I->a.as<float>(), I->b.as<float>()};
+  float* T[2] = {I->a.as<float>(), tmp->as<float>()};
+  if (nt & 1) std::swap(T[0], T[1]);  // the last step writes a
   k_inv_sums<<<(n * 32 + 255) / 256, 256, 0, st>>>(n, P.A, P.rowptr, P.vhi, P.vlo, P.w, sums);
   ILM_CHECK_LAUNCH();
   k_inv_shift<<<1, 1024, 0, st>>>(n, sums, P.w, sc);
@@ -946,7 +952,6 @@ int cg64_inverse(CG64Inverse* I, const CG64Problem& P, cudaStream_t st) {
   ILM_CHECK_LAUNCH();
   I->n = n;
   I->ld = ld;
-  I->inv = T[nt & 1];
   I->g = reinterpret_cast<float*>(sums);
   I->ready = true;
   return ILM_OK;

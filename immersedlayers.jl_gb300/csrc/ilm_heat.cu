@@ -588,8 +588,9 @@ int ilm_heat_create(ilm_cache_t c, double kappa, double dt, const double* tb_plu
   ILM_CHECK_CUDA(cudaMemset(H->iters.p, 0, 4 * sizeof(int)));
   ILM_TRY(H->relres.alloc(3 * sizeof(double)));
   ILM_TRY(H->cgs.alloc(cg64_scratch_bytes(N)));
+  DevBuf tmp;
   if (N <= HEAT_MAX_POINTS)
-    for (int s = 0; s < 3; ++s) ILM_TRY(cg64_inverse(&H->inv[s], stage_problem(H, s), nullptr));
+    for (int s = 0; s < 3; ++s) ILM_TRY(cg64_inverse(&H->inv[s], &tmp, stage_problem(H, s), nullptr));
   ILM_CHECK_CUDA(cudaDeviceSynchronize());
   *out = guard.release();
   return ILM_OK;

@@ -550,18 +550,20 @@ struct CG64Problem {
 // FP32 inverse of W S for CG64Problem::inv, formed on the device without a
 // host wait; unusable ones (S far from definite) are marked and skipped.
 struct CG64Inverse {
-  DevBuf a, b, s;
+  DevBuf a, s;
   int n = 0, ld = 0;
   bool ready = false;              // formed for the current S
-  const float *inv = nullptr, *g = nullptr;
+  const float* g = nullptr;
   void attach(CG64Problem* P) const {
-    P->inv = inv;
+    P->inv = a.as<float>();
     P->invg = g;
     P->invs = s.as<float>();
     P->ldi = ld;
   }
 };
-int cg64_inverse(CG64Inverse* I, const CG64Problem& P, cudaStream_t st);
+// tmp: the second matrix of the elimination, free for the next inverse on st.
+// Without the memory for it (ready stays false) the CG alone solves.
+int cg64_inverse(CG64Inverse* I, DevBuf* tmp, const CG64Problem& P, cudaStream_t st);
 struct CG64State {                 // head of the scratch: results and the grid variant's counters
   int iters, timeout;
   double relres;
@@ -602,7 +604,8 @@ struct ilm_cache_s {
   // scratch point buffers (FP64 and cache dtype)
   ilm::DevBuf p_scr[8];
   // cached Schur complements for the problem solves, and their FP32 inverses
-  ilm::DevBuf S_dir64, S_neu64;
+  // (inv_tmp: formed in)
+  ilm::DevBuf S_dir64, S_neu64, inv_tmp;
   ilm::CG64Inverse inv_dir, inv_neu;
   bool S_dir_ready = false, S_neu_ready = false;
   // surface filter: W = E R 1 (cache dtype) and a grid buffer of the cache's class
