@@ -246,8 +246,12 @@ std::map<std::pair<int, int>, void*> g_twiddles;             // (L, dtype) -> de
 std::map<std::tuple<int, int, int>, void*> g_spectra;        // (P1, P2, dtype) -> spectrum
 int g_lgf_M = -1;
 double* g_lgf = nullptr;
+DevTable& lgf_own() {                // owns g_lgf, with the plans that use it
+  static DevTable* p = new DevTable;  // (not destroyed: the driver may be gone by then)
+  return *p;
+}
 float2* g_lgf_ff = nullptr;        // float-float copy of g_lgf
-const double* g_lgf_ff_src = nullptr;  // the FP64 table it was split from
+int g_lgf_ff_M = -1;               // size of the FP64 table it was split from
 
 void gauss_legendre(int n, std::vector<double>& x, std::vector<double>& w) {
   x.resize(n);
@@ -817,11 +821,20 @@ int lgf_table_device(int M, const double** tab, int* ld, cudaStream_t st) {
   k_lgf_table<<<grid, 128, 0, st>>>(MM, da.as<double>(), ds.as<double>(), dw.as<double>(), nq, d);
   ILM_CHECK_LAUNCH();
   ILM_CHECK_CUDA(cudaStreamSynchronize(st));
-  if (g_lgf) cudaFree(g_lgf);
+  lgf_own() = dev_table(d);
   g_lgf = d;
   g_lgf_M = MM;
   *tab = g_lgf;
   *ld = MM + 1;
+  return ILM_OK;
+}
+
+int lgf_table_shared(int M, DevTable* tab, int* ld, cudaStream_t st) {
+  const double* G = nullptr;
+  ILM_TRY(lgf_table_device(M, &G, ld, st));
+  std::lock_guard<std::mutex> lk(g_mu);
+  *tab = lgf_own();  // (another thread's larger one, perhaps)
+  *ld = g_lgf_M + 1;
   return ILM_OK;
 }
 
@@ -841,7 +854,7 @@ int lgf_table_ff_device(int M, const float2** tab, int* ld, cudaStream_t st) {
   int ldd = 0;
   ILM_TRY(lgf_table_device(M, &G, &ldd, st));
   std::lock_guard<std::mutex> lk(g_mu);
-  if (g_lgf_ff && g_lgf_ff_src == G) {
+  if (g_lgf_ff && g_lgf_ff_M == ldd - 1) {
     *tab = g_lgf_ff;
     *ld = ldd;
     return ILM_OK;
@@ -857,7 +870,7 @@ int lgf_table_ff_device(int M, const float2** tab, int* ld, cudaStream_t st) {
   ILM_CHECK_CUDA(cudaStreamSynchronize(st));
   if (g_lgf_ff) cudaFree(g_lgf_ff);
   g_lgf_ff = d;
-  g_lgf_ff_src = G;
+  g_lgf_ff_M = ldd - 1;
   *tab = g_lgf_ff;
   *ld = ldd;
   return ILM_OK;

@@ -8,6 +8,7 @@
 
 #include <algorithm>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <thread>
@@ -311,13 +312,20 @@ int fill_zero(void* out, size_t bytes, cudaStream_t st);
 // ---------------------------------------------------------------------------
 // FFT convolution (inverse Laplacian)
 // ---------------------------------------------------------------------------
+// Device table shared by the plans that use it, freed with the last
+using DevTable = std::shared_ptr<const double>;
+inline DevTable dev_table(double* d) {
+  return DevTable(d, [](const double* p) { cudaFree(const_cast<double*>(p)); });
+}
+
 // Sine-transform solver of one field size (ilm_sine.cu)
 struct SinePlan {
   int n1 = 0, n2 = 0, N = 0, MB = 0, L = 0, ldg = 0;
   const void* tw = nullptr;      // twiddles of length 2 N
-  const double* tab = nullptr;   // per-mode constants (shared, library-owned)
+  const double* tab = nullptr;   // per-mode constants
   const double* s2 = nullptr;    // 2 sin(pi m / N), 0 <= m < 2 N
-  const double* lgf = nullptr;   // G(m, n), row stride ldg (shared, library-owned)
+  const double* lgf = nullptr;   // G(m, n), row stride ldg
+  DevTable tab_own, lgf_own;
   DevBuf work;                   // modes (n2 x N) and the ring's sources and potentials
 };
 bool sine_supported(int n1, int n2);
@@ -385,6 +393,8 @@ int conv_resources(int P1, int P2, int dtype, const void** spec, const void** tw
 int good_fft_size(int n);
 // G(m,n) table for 0<=m,n<=M (row-major (M+1)x(M+1), FP64, device; library-owned)
 int lgf_table_device(int M, const double** tab, int* ld, cudaStream_t st);
+// the same table, kept for its holder when the library's grows
+int lgf_table_shared(int M, DevTable* tab, int* ld, cudaStream_t st);
 int lgf_table_ff_device(int M, const float2** tab, int* ld, cudaStream_t st);  // (hi, lo) pairs
 int conv_plan_init(ConvPlan* plan, int n1, int n2, int dtype, cudaStream_t st);
 // out = (1/factor) * G * in (linear convolution), in/out n1 x n2 (x fastest)

@@ -31,9 +31,10 @@
 #include <math.h>
 
 #include <algorithm>
+#include <deque>
 #include <map>
+#include <memory>
 #include <mutex>
-#include <tuple>
 
 #include "ilm_fftcore.cuh"
 
@@ -608,14 +609,42 @@ __global__ void __launch_bounds__(256) k_ring_potential(int N, int n2, const dou
   }
 }
 
-__global__ void k_copy_table(const double* __restrict__ src, int lds, int n, double* __restrict__ dst) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dst[(size_t)blockIdx.y * n + i] = src[(size_t)blockIdx.y * lds + i];
+// The mode tables in use, by (N, n2), and the last few beside them (a cache that
+// is made again finds its own): kKeptTables of up to 5 MB.
+using TabKey = std::pair<int, int>;
+constexpr size_t kKeptTables = 8;
+struct ModeTables {
+  std::mutex mu;
+  std::map<TabKey, std::weak_ptr<const double>> all;
+  std::deque<DevTable> kept;
+};
+ModeTables& mode_tables() {
+  static ModeTables* p = new ModeTables;  // (not destroyed: the driver may be gone by then)
+  return *p;
 }
-
-std::mutex s_mu;
-std::map<std::pair<int, int>, double*> s_tabs;  // (N, n2) -> mode table, 2 sin table
-std::map<int, double*> s_lgf;                   // M -> (M + 1)^2 table of G
+DevTable find_table(const TabKey& key) {
+  ModeTables& T = mode_tables();
+  std::lock_guard<std::mutex> lk(T.mu);
+  auto it = T.all.find(key);
+  return it == T.all.end() ? nullptr : it->second.lock();
+}
+// the first one added wins
+DevTable add_table(const TabKey& key, const DevTable& t) {
+  ModeTables& T = mode_tables();
+  DevTable out = t, old;  // (freed after the lock)
+  std::lock_guard<std::mutex> lk(T.mu);
+  for (auto it = T.all.begin(); it != T.all.end();) it = it->second.expired() ? T.all.erase(it) : std::next(it);
+  auto it = T.all.find(key);
+  if (it != T.all.end())
+    if (DevTable first = it->second.lock()) return first;
+  T.all[key] = out;
+  T.kept.push_back(out);
+  if (T.kept.size() > kKeptTables) {
+    old = T.kept.front();
+    T.kept.pop_front();
+  }
+  return out;
+}
 
 }  // namespace
 
@@ -635,48 +664,24 @@ int sine_plan_init(SinePlan* p, int n1, int n2, const void* tw, cudaStream_t st)
   p->MB = modes_per_cta(n2);
   const int nch = chunks(p->MB);
   p->L = (n2 + nch - 1) / nch;
-  const int M = std::max(N, n2 + 1);
-  p->ldg = M + 1;
-  {
-    std::lock_guard<std::mutex> lk(s_mu);
-    auto it = s_tabs.find({N, n2});
-    if (it != s_tabs.end()) p->tab = it->second;
-    auto ig = s_lgf.find(M);
-    if (ig != s_lgf.end()) p->lgf = ig->second;
-  }
   const size_t ntab = (size_t)(TB_HEAD + 2 * nch) * N;
-  if (!p->tab) {
+  p->tab_own = find_table({N, n2});
+  if (!p->tab_own) {
     double* d = nullptr;
     if (cudaMalloc(&d, (ntab + 2 * (size_t)N) * sizeof(double)) != cudaSuccess) {
       set_error("cudaMalloc sine-transform tables failed");
       return ILM_ERR_NO_MEMORY;
     }
+    const DevTable t = dev_table(d);
     k_mode_table<<<(2 * N + 127) / 128, 128, 0, st>>>(N, n2, nch, p->L, d, d + ntab);
     ILM_CHECK_LAUNCH();
     ILM_CHECK_CUDA(cudaStreamSynchronize(st));
-    std::lock_guard<std::mutex> lk(s_mu);
-    auto r = s_tabs.emplace(std::make_pair(N, n2), d);
-    if (!r.second) cudaFree(d);  // another thread was first
-    p->tab = r.first->second;
+    p->tab_own = add_table({N, n2}, t);
   }
+  p->tab = p->tab_own.get();
   p->s2 = p->tab + ntab;
-  if (!p->lgf) {
-    const double* G = nullptr;
-    int ld = 0;
-    double* d = nullptr;
-    if (cudaMalloc(&d, (size_t)(M + 1) * (M + 1) * sizeof(double)) != cudaSuccess) {
-      set_error("cudaMalloc lattice Green's function copy failed");
-      return ILM_ERR_NO_MEMORY;
-    }
-    ILM_TRY(lgf_table_device(M, &G, &ld, st));
-    k_copy_table<<<dim3((M + 1 + 255) / 256, M + 1), 256, 0, st>>>(G, ld, M + 1, d);
-    ILM_CHECK_LAUNCH();
-    ILM_CHECK_CUDA(cudaStreamSynchronize(st));
-    std::lock_guard<std::mutex> lk(s_mu);
-    auto r = s_lgf.emplace(M, d);
-    if (!r.second) cudaFree(d);
-    p->lgf = r.first->second;
-  }
+  ILM_TRY(lgf_table_shared(std::max(N, n2 + 1), &p->lgf_own, &p->ldg, st));
+  p->lgf = p->lgf_own.get();
   return p->work.alloc(((size_t)n2 * N + 4 * (size_t)N + 4 * (size_t)n2) * sizeof(double));
 }
 
