@@ -1283,11 +1283,16 @@ int launch_cg_sized(const void* params_dev, const int* order, int nprob, int* co
     set_error("cluster CG: %d unknowns exceed the shared-memory layout of %d CTAs", max_n, cs);
     return ILM_ERR_SIZE_LIMIT;
   }
+  // (a device that grants no clusters of 16, a partition say, takes those of 8)
+  if (cs == 16) {
+    const size_t smem = cg_cluster_smem(max_n, 256, 16);
+    if (launch_dist<256, 3, 16>(prm, order, nprob, counter, max_n, nclusters, smem, st) == ILM_OK) return ILM_OK;
+    return launch_cg_sized(params_dev, order, nprob, counter, max_n, nclusters, 8, st);
+  }
   const size_t smem = cg_cluster_smem(max_n, 256, cs);
   switch (cs) {
     case 1: return launch_dist<256, 3, 1>(prm, order, nprob, counter, max_n, nclusters, smem, st);
     case 4: return launch_dist<256, 3, 4>(prm, order, nprob, counter, max_n, nclusters, smem, st);
-    case 16: return launch_dist<256, 3, 16>(prm, order, nprob, counter, max_n, nclusters, smem, st);
     default: return launch_dist<256, 3, 8>(prm, order, nprob, counter, max_n, nclusters, smem, st);
   }
 }

@@ -649,7 +649,7 @@ size_t plan(const CG64Problem& P, bool grid, int G, CG64Args* A) {
 }
 
 template <bool CSR>
-int run_cluster(const CG64Args& A, size_t smem, cudaStream_t st) {
+cudaError_t run_cluster(const CG64Args& A, size_t smem, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(C64_CLUSTER);
   cfg.blockDim = dim3(C64_T);
@@ -661,16 +661,20 @@ int run_cluster(const CG64Args& A, size_t smem, cudaStream_t st) {
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  ILM_CHECK_CUDA(cudaLaunchKernelEx(&cfg, k_cg64<CSR, false>, A));
-  return ILM_OK;
+  return cudaLaunchKernelEx(&cfg, k_cg64<CSR, false>, A);
 }
 
 template <bool CSR>
-int run_grid(CG64Args& A, int G, size_t smem, cudaStream_t st) {
+cudaError_t run_grid(CG64Args& A, int G, size_t smem, cudaStream_t st) {
   void* args[1] = {&A};
-  ILM_CHECK_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(k_cg64<CSR, true>), dim3(G), dim3(C64_T), args,
-                                             smem, st));
-  return ILM_OK;
+  return cudaLaunchCooperativeKernel(reinterpret_cast<void*>(k_cg64<CSR, true>), dim3(G), dim3(C64_T), args, smem, st);
+}
+
+// a launch that the device (a partition of it, or a context limited to some of
+// its SMs) has no room for
+bool no_room(cudaError_t e) {
+  return e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorInvalidClusterSize ||
+         e == cudaErrorLaunchOutOfResources || e == cudaErrorInvalidConfiguration || e == cudaErrorNotSupported;
 }
 
 template <bool CSR, bool GRID>
@@ -961,7 +965,7 @@ size_t cg64_scratch_bytes(int n) { return sizeof(CG64State) + 5 * (size_t)n * si
 
 bool cg64_fits(int n) { return 5 * (size_t)((n + 3) / 4 * 4) * sizeof(double) <= (size_t)C64_MAX_GRID; }
 
-int launch_cg64(const CG64Problem& P, void* scratch, cudaStream_t st, int variant) {
+int launch_cg64(const CG64Problem& P, void* scratch, cudaStream_t st) {
   const int n = P.n;
   if (!cg64_fits(n)) {
     set_error("CG: problem of %d unknowns exceeds the shared-memory solver", n);
@@ -979,20 +983,27 @@ int launch_cg64(const CG64Problem& P, void* scratch, cudaStream_t st, int varian
   const long long entries = (long long)n * (csr ? std::min(P.max_row_nnz, n) : n);
   size_t smem = plan(P, false, C64_CLUSTER, &A);
   const bool few = P.inv ? n <= (csr ? C64_CLUSTER_CSR : C64_CLUSTER_DENSE) : entries <= C64_CLUSTER_ENTRIES;
-  if ((variant == 1 || (variant == 0 && few)) && smem <= (size_t)C64_MAX_CLUSTER &&
-      (csr || A.resident)) {
+  if (few && smem <= (size_t)C64_MAX_CLUSTER && (csr || A.resident)) {
     ILM_CHECK_CUDA((csr ? kernel_attributes<true, false>() : kernel_attributes<false, false>()));
-    return csr ? run_cluster<true>(A, smem, st) : run_cluster<false>(A, smem, st);
+    const cudaError_t e = csr ? run_cluster<true>(A, smem, st) : run_cluster<false>(A, smem, st);
+    if (!no_room(e)) {
+      ILM_CHECK_CUDA(e);
+      return ILM_OK;
+    }
+    (void)cudaGetLastError();
   }
-  const int sms = device_sms();
-  if (sms < 1) {
-    set_error("CG: no device");
-    return ILM_ERR_CUDA;
-  }
-  smem = plan(P, true, std::min(sms, n), &A);
   ILM_CHECK_CUDA((csr ? kernel_attributes<true, true>() : kernel_attributes<false, true>()));
-  const int G = (n + A.R - 1) / A.R;
-  return csr ? run_grid<true>(A, G, smem, st) : run_grid<false>(A, G, smem, st);
+  // a CTA per SM; where they cannot all be resident, half as many, down to four (at
+  // which 256 unknowns still fit: rows streamed from L2 need more than C64_T)
+  cudaError_t e = cudaErrorCooperativeLaunchTooLarge;
+  for (int ctas = device_sms(); ctas >= 4 && no_room(e); ctas /= 2) {
+    (void)cudaGetLastError();
+    smem = plan(P, true, std::min(ctas, n), &A);
+    const int G = (n + A.R - 1) / A.R;
+    e = csr ? run_grid<true>(A, G, smem, st) : run_grid<false>(A, G, smem, st);
+  }
+  ILM_CHECK_CUDA(e);
+  return ILM_OK;
 }
 
 }  // namespace ilm

@@ -582,8 +582,7 @@ struct CG64State {                 // head of the scratch: results and the grid 
 size_t cg64_scratch_bytes(int n);
 bool cg64_fits(int n);  // the vectors of n unknowns fit a CTA's shared memory
 inline int cg64_csr_slab(const CG64Problem& P, int rows) { return P.max_row_nnz * rows; }
-// variant: 0 by size, 1 one cluster, 2 cooperative grid
-int launch_cg64(const CG64Problem& P, void* scratch, cudaStream_t st, int variant = 0);
+int launch_cg64(const CG64Problem& P, void* scratch, cudaStream_t st);
 
 }  // namespace ilm
 

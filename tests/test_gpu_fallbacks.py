@@ -10,32 +10,56 @@ import pytest
 pytestmark = pytest.mark.gpu
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
-# passes every call on but those it is told to refuse (refuse_*), and counts the live
-# device allocations of watch_bytes
+# passes every call on but those it is told to refuse (refuse_*, most_ctas), and counts
+# the live device allocations of watch_bytes
 SHIM = r"""
 #define _GNU_SOURCE
+#include <cuda_runtime_api.h>
 #include <dlfcn.h>
 #include <stddef.h>
 static void* real(const char* name) { return dlsym(dlopen("libcudart.so.13", RTLD_LAZY | RTLD_NOLOAD), name); }
 size_t refuse_bytes = 0, watch_bytes = 0;
-int refused = 0, live = 0;
+int refuse_cluster = 0, refuse_attribute = 0, most_ctas = 1 << 30, refused = 0, live = 0;
 static void* ptrs[64];
-int cudaMalloc(void** p, size_t n) {
+cudaError_t cudaMalloc(void** p, size_t n) {
   if (refuse_bytes && n == refuse_bytes) {
     ++refused;
     /* the runtime's own refusal, so that its last error is set as in earnest */
-    return ((int (*)(void**, size_t))real("cudaMalloc"))(p, (size_t)1 << 50);
+    return ((cudaError_t (*)(void**, size_t))real("cudaMalloc"))(p, (size_t)1 << 50);
   }
-  int e = ((int (*)(void**, size_t))real("cudaMalloc"))(p, n);
+  cudaError_t e = ((cudaError_t (*)(void**, size_t))real("cudaMalloc"))(p, n);
   if (e == 0 && watch_bytes && n == watch_bytes)
     for (int k = 0; k < 64; ++k)
       if (!ptrs[k]) { ptrs[k] = *p; ++live; break; }
   return e;
 }
-int cudaFree(void* p) {
+cudaError_t cudaFree(void* p) {
   for (int k = 0; p && k < 64; ++k)
     if (ptrs[k] == p) { ptrs[k] = 0; --live; }
-  return ((int (*)(void*))real("cudaFree"))(p);
+  return ((cudaError_t (*)(void*))real("cudaFree"))(p);
+}
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void** args) {
+  for (unsigned k = 0; refuse_cluster && k < c->numAttrs; ++k)
+    if (c->attrs[k].id == cudaLaunchAttributeClusterDimension && (int)c->attrs[k].val.clusterDim.x >= refuse_cluster) {
+      ++refused;
+      return cudaErrorInvalidClusterSize;
+    }
+  return ((cudaError_t (*)(const cudaLaunchConfig_t*, const void*, void**))real("cudaLaunchKernelExC"))(c, f, args);
+}
+cudaError_t cudaFuncSetAttribute(const void* f, enum cudaFuncAttribute a, int v) {
+  if (refuse_cluster && a == cudaFuncAttributeNonPortableClusterSizeAllowed && refuse_attribute) {
+    ++refused;
+    return cudaErrorNotSupported;
+  }
+  return ((cudaError_t (*)(const void*, enum cudaFuncAttribute, int))real("cudaFuncSetAttribute"))(f, a, v);
+}
+cudaError_t cudaLaunchCooperativeKernel(const void* f, struct dim3 g, struct dim3 b, void** args, size_t sm, cudaStream_t st) {
+  if ((int)g.x > most_ctas) {
+    ++refused;
+    return cudaErrorCooperativeLaunchTooLarge;
+  }
+  return ((cudaError_t (*)(const void*, struct dim3, struct dim3, void**, size_t, cudaStream_t))real(
+      "cudaLaunchCooperativeKernel"))(f, g, b, args, sm, st);
 }
 """
 
@@ -85,7 +109,9 @@ def child(cuda, tmp_path_factory):
     src, shim = str(d / "shim.c"), str(d / "shim.so")
     with open(src, "w") as f:
         f.write(SHIM)
-    subprocess.run(["gcc", "-shared", "-fPIC", "-o", shim, src, "-ldl"], check=True, capture_output=True)
+    from immersedlayers import _build
+    inc = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(_build.nvcc()))), "include")
+    subprocess.run(["gcc", "-shared", "-fPIC", "-I" + inc, "-o", shim, src, "-ldl"], check=True, capture_output=True)
 
     def run(body):
         code = f"ROOT, SHIM = {ROOT!r}, {shim!r}\n" + HEAD + textwrap.dedent(body)
@@ -133,4 +159,42 @@ def test_memory_of_the_inverses(child):
     integ = heat(grid, bl)
     integ.advance(1)
     assert live.value == 6, live.value
+    """)
+
+
+@pytest.mark.parametrize("n,most,refusals", [(150, 152, 1), (256, 4, 6), (400, 9, 4), (700, 8, 5), (700, 100, 1)])
+def test_solve_on_fewer_sms(child, n, most, refusals):
+    """No cluster of 16 and at most `most` CTAs of a cooperative launch: the solve
+    takes the grid, and half as many CTAs until they fit (S in shared memory, or
+    with 700 points on 4 CTAs streamed from L2)."""
+    child(f"""
+    n = {n}
+    grid, bl, c, plus, minus = case(n)
+    setting("refuse_cluster", C.c_int).value = 16
+    setting("most_ctas", C.c_int).value = {most}
+    _, s, info = il.solve_dirichlet(c, plus, minus, tol=1e-10, maxiter=20000)
+    assert setting("refused", C.c_int).value == {refusals}, setting("refused", C.c_int).value
+    assert info["converged"] and true_residual(c, plus, s) <= 1e-10 + 1e-12
+    integ = heat(grid, bl)
+    integ.advance(2)
+    assert max(integ.info()["rel_residual"]) <= 1e-11
+    """)
+
+
+def test_batch_without_large_clusters(child):
+    """A batch whose largest problem would take a cluster of 16 CTAs takes one of 8."""
+    child("""
+    from immersedlayers.batch import BatchProblemSpec, BatchSolver
+    n = 400
+    grid, bl, c, plus, minus = case(n)
+    sol = []
+    for refuse in (0, 16):
+        setting("refuse_cluster", C.c_int).value = setting("refuse_attribute", C.c_int).value = refuse
+        bs = BatchSolver([BatchProblemSpec(grid.nx, grid.h, bl, 0, plus.data.cpu().numpy())], dtype=torch.float64)
+        _, s = bs.solve(*bs.surface_data(), tol=1e-9, maxiter=5000)
+        assert (bs.info()[1] <= 1e-9).all()
+        sol.append(s.clone())
+    assert setting("refused", C.c_int).value > 0
+    # two solutions of relative residual 1e-9, condition some 1e3
+    assert float((sol[0] - sol[1]).norm()) <= 1e-5 * float(sol[0].norm())
     """)
