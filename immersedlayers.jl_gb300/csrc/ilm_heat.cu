@@ -95,7 +95,9 @@ __device__ __forceinline__ unsigned stage_value(double v, float2 f, double* d, f
   return (unsigned)__double2hiint(v) & 0x7fffffffu;
 }
 
-// what the tile's largest magnitude allows
+// what the tile's largest magnitude allows: in float-float from 2^-46 on, where
+// what split64 drops of values below 2^-74 (2^-98, times 2% of far taps) stays
+// under 2^-53 of it
 enum { IF_ZERO = 0, IF_SPLIT = 1, IF_FP64 = 2 };
 __device__ __forceinline__ int tile_mode(unsigned mag, unsigned low, unsigned* red) {
   if (threadIdx.x == 0) red[0] = red[1] = 0u;
@@ -108,7 +110,7 @@ __device__ __forceinline__ int tile_mode(unsigned mag, unsigned low, unsigned* r
   }
   __syncthreads();
   const unsigned top = red[0] >> 20, any = red[0] | red[1];
-  return any == 0u ? IF_ZERO : top >= 963u && top <= 1143u ? IF_SPLIT : IF_FP64;
+  return any == 0u ? IF_ZERO : top >= 977u && top <= 1143u ? IF_SPLIT : IF_FP64;
 }
 
 // one output: centre index at, tap distance step

@@ -167,3 +167,38 @@ def test_heat_integrating_factor_tiles(cuda, fourier, scale):
     free = np.maximum(np.abs(x)[:, None], np.abs(y)[None, :]) > reach
     assert free.sum() > 300
     assert np.abs(T - ref)[free].max() < 1e-13 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("scale", [2.0 ** -44, 2.0 ** -50, 2.0 ** -59])
+def test_heat_integrating_factor_small_values(cuda, scale):
+    """A step is linear, and a power of two changes no FP64 rounding: the step of
+    a field times `scale` is the step times `scale`.  Spikes of 1 over values of
+    2^-18: their FP64 sums are good to 2^-53 2^-18 = 4e-22 away from the spikes;
+    float-float taps (on at most 2%) of 48 bits give as much.  1e-18 is far below
+    what values cut to 24 bits would leave (2^-18 2^-23 of 2%, 9e-15)."""
+    import torch
+    out = []
+    for s in (1.0, scale):
+        il, og, b, sys, u0, _ = _setup(torch.float64, 0.5)
+        x, y = og.coords(O.NODES_PRIMAL)
+        T0 = 2.0 ** -18 * np.random.default_rng(6).standard_normal((len(x), len(y)))
+        T0[::64, ::32] = 1.0
+        prob = il.DirichletHeatConductionProblem(
+            sys.base_cache.g, b, dtype=torch.float64, phys_params={"diffusivity": 1.0, "Fourier": 0.5},
+            bc={"exterior": lambda t, x, c, p, m: il.zeros_surface(c),
+                "interior": lambda t, x, c, p, m: il.zeros_surface(c)}, timestep_func=il.timestep_fourier)
+        sys = il.construct_system(prob)
+        u0 = il.init_sol(sys)
+        u0.state.set_numpy(s * T0)
+        integ = il.init(u0, (0.0, 1.0), sys, tol=1e-12, maxiter=500)
+        integ.advance(1)
+        torch.cuda.synchronize()
+        out.append(il.temperature(integ).numpy_components() / s)
+    r = O.heat_kernel_1d(0.5).size // 2
+    away = np.ones(T0.shape, bool)
+    i, j = np.arange(T0.shape[0])[:, None], np.arange(T0.shape[1])[None, :]
+    away &= (np.minimum(i % 64, 64 - i % 64) > r) | (np.minimum(j % 32, 32 - j % 32) > r)
+    reach = 0.4 + (3 + r) * og.h
+    away &= np.maximum(np.abs(x)[:, None], np.abs(y)[None, :]) > reach
+    assert away.sum() > 300
+    assert np.abs(out[0] - out[1])[away].max() < 1e-18
