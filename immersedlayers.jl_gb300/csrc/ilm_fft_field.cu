@@ -42,8 +42,7 @@ constexpr Stages stages_of(int L) {
   return {0, {0, 0, 0, 0}};
 }
 constexpr int num_stages(int L) {
-  const Stages s = stages_of(L);
-  return s.r[2] == 0 ? 2 : s.r[3] == 0 ? 3 : 4;
+  return stages_of(L).r[3] == 0 ? 3 : 4;
 }
 // radix of stage s of the forward (dir = 0) or inverse (1: reversed) transform
 constexpr int radix_of(int L, int s, int dir) { return stages_of(L).r[dir ? num_stages(L) - 1 - s : s]; }
@@ -124,37 +123,30 @@ struct FieldJob {
   float scale;
 };
 
-// threads of a row CTA: two warps of short rows (many CTAs), one row of long ones
-constexpr int row_threads(int H) { return H / stages_of(H).e > 64 ? H / stages_of(H).e : 64; }
-
-// rows: real transforms of length 2 H
+// rows: real transforms of length 2 H, a CTA of H / E threads each
 template <int H>
-__global__ void __launch_bounds__(row_threads(H)) k_rows_field(const FieldJob J) {
-  constexpr int E = stages_of(H).e, T = H / E, RB = row_threads(H) / T, ns = num_stages(H);
-  constexpr int R0 = radix_of(H, 0, 0), RL = radix_of(H, ns - 1, 0), CS = transform_floats2(H);
+__global__ void __launch_bounds__(H / stages_of(H).e) k_rows_field(const FieldJob J) {
+  constexpr int E = stages_of(H).e, T = H / E, ns = num_stages(H);
+  constexpr int R0 = radix_of(H, 0, 0), RL = radix_of(H, ns - 1, 0);
   extern __shared__ __align__(16) float2 sm_field[];
-  const int rr = threadIdx.x / T, t = threadIdx.x - rr * T, row = blockIdx.x * RB + rr;
-  float2* s = sm_field + rr * CS;
-  const bool act = rr < RB && row < J.n2;
-  const float* __restrict__ x = J.in + (size_t)(act ? row : 0) * J.n1;
+  const int t = threadIdx.x, row = blockIdx.x;
+  float2* s = sm_field;
+  const float* __restrict__ x = J.in + (size_t)row * J.n1;
   float2 a[E];
 #pragma unroll
   for (int b = 0; b < E / R0; ++b)
 #pragma unroll
     for (int r = 0; r < R0; ++r) {
       const int m = 2 * (t + b * T + r * (H / R0));
-      a[b * R0 + r] = make_float2(act && m < J.n1 ? __ldg(x + m) : 0.f, act && m + 1 < J.n1 ? __ldg(x + m + 1) : 0.f);
+      a[b * R0 + r] = make_float2(m < J.n1 ? __ldg(x + m) : 0.f, m + 1 < J.n1 ? __ldg(x + m + 1) : 0.f);
     }
-  stages_from<H, 0, 0>(a, t, rr < RB ? s : sm_field, J.tw1, 2);
+  stages_from<H, 0, 0>(a, t, s, J.tw1, 2);
   __syncthreads();
-  if (rr < RB) {
 #pragma unroll
-    for (int b = 0; b < E / RL; ++b)
+  for (int b = 0; b < E / RL; ++b)
 #pragma unroll
-      for (int r = 0; r < RL; ++r) s[fpos(t + b * T + r * (H / RL))] = a[b * RL + r];
-  }
+    for (int r = 0; r < RL; ++r) s[fpos(t + b * T + r * (H / RL))] = a[b * RL + r];
   __syncthreads();
-  if (!act) return;
   float2* __restrict__ W = J.work + (size_t)row * (H + 1);
   for (int k = t; k <= H; k += T) {
     const float2 zk = s[fpos(k == H ? 0 : k)];
@@ -168,22 +160,20 @@ __global__ void __launch_bounds__(row_threads(H)) k_rows_field(const FieldJob J)
 }
 
 template <int H>
-__global__ void __launch_bounds__(row_threads(H)) k_irows_field(const FieldJob J) {
-  constexpr int E = stages_of(H).e, T = H / E, RB = row_threads(H) / T, ns = num_stages(H);
-  constexpr int R0 = radix_of(H, 0, 1), RL = radix_of(H, ns - 1, 1), CS = transform_floats2(H);
+__global__ void __launch_bounds__(H / stages_of(H).e) k_irows_field(const FieldJob J) {
+  constexpr int E = stages_of(H).e, T = H / E, ns = num_stages(H);
+  constexpr int R0 = radix_of(H, 0, 1), RL = radix_of(H, ns - 1, 1);
   extern __shared__ __align__(16) float2 sm_field[];
-  const int rr = threadIdx.x / T, t = threadIdx.x - rr * T, row = blockIdx.x * RB + rr;
-  float2* s = sm_field + (rr < RB ? rr : 0) * CS;
-  const bool act = rr < RB && row < J.n2;
-  const float2* __restrict__ W = J.work + (size_t)(act ? row : 0) * (H + 1);
+  const int t = threadIdx.x, row = blockIdx.x;
+  const float2* __restrict__ W = J.work + (size_t)row * (H + 1);
   float2 a[E];
 #pragma unroll
   for (int b = 0; b < E / R0; ++b)
 #pragma unroll
     for (int r = 0; r < R0; ++r) {
       const int k = t + b * T + r * (H / R0);
-      const float2 xk = act ? W[k] : make_float2(0.f, 0.f);
-      float2 xc = act ? W[H - k] : make_float2(0.f, 0.f);
+      const float2 xk = W[k];
+      float2 xc = W[H - k];
       xc.y = -xc.y;
       float2 e = __ldg(J.tw1 + k);
       e.y = -e.y;
@@ -191,8 +181,7 @@ __global__ void __launch_bounds__(row_threads(H)) k_irows_field(const FieldJob J
       const float2 ed = cmul(e, d);
       a[b * R0 + r] = make_float2(0.5f * (p.x - ed.y), 0.5f * (p.y + ed.x));
     }
-  stages_from<H, 0, 1>(a, t, s, J.tw1, 2);
-  if (!act) return;
+  stages_from<H, 0, 1>(a, t, sm_field, J.tw1, 2);
   float* __restrict__ o = J.out + (size_t)row * J.n1;
 #pragma unroll
   for (int b = 0; b < E / RL; ++b)
@@ -207,8 +196,8 @@ __global__ void __launch_bounds__(row_threads(H)) k_irows_field(const FieldJob J
 // spectral columns per CTA: 4 (a 32-byte sector of every row) where that is at
 // most 512 threads, so that a thread's values stay in registers, else 2
 constexpr int field_cw(int L) { return 4 * (L / stages_of(L).e) <= 512 ? 4 : 2; }
-// stride of a column's buffer: 2 (mod 16) for 4 or 8 columns side by side in a
-// half-warp (with the pad of fpos the 16 lanes hit 16 bank pairs)
+// stride of a column's buffer: 4 (mod 16) for four columns side by side in a
+// half-warp, 8 for two (with the pad of fpos the 16 lanes hit 16 bank pairs)
 constexpr int field_cs(int L) {
   int c = transform_floats2(L);
   while (c % 16 != (field_cw(L) == 4 ? 4 : 8)) ++c;
@@ -266,10 +255,9 @@ int run(K kernel, int grid, int threads, size_t smem, const FieldJob& J, cudaStr
 
 template <int H>
 int run_rows(const FieldJob& J, bool inverse, cudaStream_t st) {
-  constexpr int T = row_threads(H), RB = T / (H / stages_of(H).e);
-  const size_t smem = (size_t)RB * transform_floats2(H) * sizeof(float2);
-  const int grid = (J.n2 + RB - 1) / RB;
-  return inverse ? run(k_irows_field<H>, grid, T, smem, J, st) : run(k_rows_field<H>, grid, T, smem, J, st);
+  constexpr int T = H / stages_of(H).e;
+  const size_t smem = transform_floats2(H) * sizeof(float2);
+  return inverse ? run(k_irows_field<H>, J.n2, T, smem, J, st) : run(k_rows_field<H>, J.n2, T, smem, J, st);
 }
 
 template <int L>

@@ -13,8 +13,9 @@ from test_gpu_sine import _reference
 pytestmark = pytest.mark.gpu
 
 
-# every row length (64 .. 4096 and 3 * 2^a) and column length (64 .. 6144), full and
-# nearly empty padding, odd sizes; one below the shortest (the general kernels)
+# padded sizes from 64 to 8192 x 6144, full and nearly empty padding, odd sizes: the
+# general kernels, and from 2048 on both sides those of single fields, all of which
+# the next test reaches
 @pytest.mark.parametrize("nx,ny", [(30, 70), (65, 34), (70, 40), (100, 65), (110, 97), (140, 130), (1025, 1024), (900, 1025), (1400, 1400), (2000, 1200), (2900, 600), (200, 1100),
                                    (4096, 800), (300, 1500), (600, 800), (500, 900), (1500, 140), (1500, 100),
                                    (1500, 300), (1500, 250), (1500, 500), (250, 2050), (260, 3000), (250, 3072)])
@@ -31,3 +32,12 @@ def test_inverse_laplacian_f32(cuda, nx, ny):
     assert err <= 6e-6, err
     il.inverse_laplacian_(w, c)  # in place
     assert torch.equal(w.data, out.data)
+
+
+# every row length (1024, 1536, .. 4096) and column length (2048, 3072, 4096, 6144) of
+# the single-field kernels, at the fewest and the most values that take it, odd sizes
+@pytest.mark.parametrize("nx,ny", [(770, 770), (1025, 1025), (1026, 900), (1537, 1026), (1538, 800), (2049, 1537),
+                                   (2050, 770), (3073, 900), (3074, 1026), (900, 1538), (1025, 2049), (1030, 2050),
+                                   (1100, 3073), (4097, 3073)])
+def test_inverse_laplacian_f32_instances(cuda, nx, ny):
+    test_inverse_laplacian_f32(cuda, nx, ny)
