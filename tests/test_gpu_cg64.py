@@ -17,9 +17,10 @@ TOL = 1e-10
 
 
 # fewer points than CTAs, one row per CTA, whole and partial 32 x 32 tiles of
-# the inverse, either side of the cluster / grid rule (256 unknowns), a partial
-# last slice, a slice too large for shared memory; points 0.45 h apart (S
-# numerically singular: the inverse is refused or useless, and the CG runs)
+# the inverse, either side of 256 (the cluster / grid rule of the CG without an
+# inverse; the one with it is tested below), a partial last slice, a slice too
+# large for shared memory; points 0.45 h apart (S numerically singular: the
+# inverse is refused or useless, and the CG runs)
 @pytest.mark.parametrize("n,ds", [(3, 1.4), (16, 1.4), (32, 1.4), (33, 1.4), (131, 1.4), (256, 1.4), (257, 1.4),
                                   (700, 1.4), (1870, 1.4), (180, 0.45)])
 def test_dense_solve_residual(cuda, n, ds):
@@ -96,3 +97,31 @@ def test_reported_residual_warm_start(cuda, ds, tol):
     rep = integ.info()["rel_residual"][2]
     assert true <= tol + 1e-10
     assert abs(rep - true) <= 1e-3 * true + 1e-10, (rep, true)
+
+
+@pytest.mark.parametrize("n", [320, 321])
+def test_dense_solve_either_side_of_the_variants(cuda, n):
+    test_dense_solve_residual(cuda, n, 1.4)
+
+
+@pytest.mark.parametrize("n", [17, 560, 561])
+def test_stage_solves_either_side_of_the_variants(cuda, n):
+    """The heat march's sparse systems in the cluster and on the grid: every stage
+    within its tolerance, and the constraint E T = 1 with it.  The last stage's
+    residual is the constraint's over dt b3, its right-hand side the change that a
+    step makes there, below 1 / (dt b3): 1e-11, and the fields' rounding."""
+    nx = max(64, int(n / 1.79))
+    grid = il.PhysicalGrid.from_cells(nx, 4.0 / nx)
+    bl = il.BodyList().append(il.circle(min(1.6, n * 1.4 * grid.h / (2 * np.pi)), n=n))
+    one = lambda t, x, c, p, m: il.ones_surface(c)
+    prob = il.DirichletHeatConductionProblem(grid, bl, dtype=torch.float64,
+                                             phys_params={"diffusivity": 1.0, "Fourier": 0.5},
+                                             bc={"exterior": one, "interior": one}, timestep_func=il.timestep_fourier)
+    system = il.construct_system(prob)
+    integ = il.init(il.init_sol(system), (0.0, 1.0), system, tol=1e-11, maxiter=2000)
+    for _ in range(3):  # cold, then warm starts
+        integ.advance(1)
+        assert max(integ.info()["rel_residual"]) <= 1e-11
+        ET = il.zeros_surface(system.base_cache)
+        il.interpolate_(ET, integ.u.state, system.base_cache)
+        assert float((ET.data - 1.0).norm()) <= 1e-11 * n ** 0.5 + 1e-13 * n ** 0.5
