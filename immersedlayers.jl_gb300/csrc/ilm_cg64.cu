@@ -297,8 +297,8 @@ __global__ void __launch_bounds__(C64_T, 1) k_cg64(const CG64Args A) {
     // residual that passes is always taken, and its residual is there.  It is
     // wanted: the residual that passes is rich in the modes that P gets least right,
     // the slow ones, and x is further off for it than a CG iterate of that residual.
-    // Nothing says that P contracts on it, so its residual decides (1.3 us of a
-    // solve on the grid, 2 on the cluster).
+    // Nothing says that P contracts on it, so its residual decides (about 1 us of
+    // a solve).
     float* v = reinterpret_cast<float*>(p);               // W r scaled into FP32's range
     float* gv = reinterpret_cast<float*>(A.gq + n);       // grid: its exchange
     double* gs = A.gq + 2 * (size_t)n;                    // grid: the CTAs' sums (three each)
@@ -444,11 +444,11 @@ __global__ void __launch_bounds__(C64_T, 1) k_cg64(const CG64Args A) {
         for (int i = lane; i < nr; i += 32) a = fma(r[r0 + i], r[r0 + i], a);
         send(s.part, gs + 2 * G, rank, warp_sum(a), lane, 32);
       }
-      if (GRID) {  // no CTA waits: the last to arrive decides, and takes x back where it has to
-        for (int i = t; i < nr; i += C64_T) {
-          P.x[r0 + i] = x[r0 + i];
-          __stcg(A.gq + n + r0 + i, old[i]);
-        }
+      for (int i = t; i < nr; i += C64_T) {
+        P.x[r0 + i] = x[r0 + i];
+        if (GRID) __stcg(A.gq + n + r0 + i, old[i]);
+      }
+      if (GRID) {  // no CTA waits: the last to arrive decides for all rows
         __syncthreads();
         if (t == 0) {
           __threadfence();
@@ -457,29 +457,26 @@ __global__ void __launch_bounds__(C64_T, 1) k_cg64(const CG64Args A) {
         }
         __syncthreads();
         if (!s_ok) return;
-      } else {
+      } else {     // every CTA decides for its own
         barrier();
       }
       if (warp == LAST) {
         double a = 0.0;
         for (int k = lane; k < G; k += 32) a += GRID ? __ldcg(gs + 2 * G + k) : s.part[k];
-        const double now = warp_sum(a);
-        if (lane == 0) {
-          if (converged(now)) s.a = now;
-          else s.flag = DONE | UNDO;
+        a = warp_sum(a);
+        const bool keep = converged(a);
+        if (!keep) {
+          if (GRID)
+            for (int j = lane; j < n; j += 32) P.x[j] = __ldcg(A.gq + n + j);
+          else
+            for (int i = lane; i < nr; i += 32) P.x[r0 + i] = old[i];
         }
-      }
-      __syncthreads();
-      flags = s.flag;
-      if (GRID) {
-        if (flags & UNDO)
-          for (int j = t; j < n; j += C64_T) P.x[j] = __ldcg(A.gq + n + j);
-        if (t == 0) {
+        if ((GRID || rank == 0) && lane == 0) {
           *P.iters = it;
-          *P.relres = fmin(sqrt(s.a / s.b), P.tol);
+          *P.relres = fmin(sqrt((keep ? a : last) / bb), P.tol);
         }
-        return;
       }
+      return;  // (nothing more is written to another CTA)
     }
     if (ok) {
       done = flags & DONE;
