@@ -35,6 +35,8 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <tuple>
+#include <vector>
 
 #include "ilm_fftcore.cuh"
 
@@ -609,41 +611,61 @@ __global__ void __launch_bounds__(256) k_ring_potential(int N, int n2, const dou
   }
 }
 
-// The mode tables in use, by (N, n2), and the last few beside them (a cache that
-// is made again finds its own): kKeptTables of up to 5 MB.
-using TabKey = std::pair<int, int>;
-constexpr size_t kKeptTables = 8;
-struct ModeTables {
+__global__ void k_copy_table(const double* __restrict__ src, int lds, int n, double* __restrict__ dst) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) dst[(size_t)blockIdx.y * n + i] = src[(size_t)blockIdx.y * lds + i];
+}
+
+// The tables in use -- mode tables by (N, n2), copies of G by size -- and the last
+// few beside them (a cache that is made again finds its own): kKeptBytes at most.
+// (G is copied because the library's table, as large as its largest user, spreads a
+// small one's rows over its long ones: 0.7 us of 48 at 105^2.)
+using TabKey = std::tuple<int, int, int>;
+enum { TAB_MODES, TAB_LGF };
+constexpr size_t kKeptBytes = 64 << 20;
+struct TableCache {
   std::mutex mu;
   std::map<TabKey, std::weak_ptr<const double>> all;
-  std::deque<DevTable> kept;
+  std::deque<std::pair<DevTable, size_t>> kept;
+  size_t bytes = 0;
 };
-ModeTables& mode_tables() {
-  static ModeTables* p = new ModeTables;  // (not destroyed: the driver may be gone by then)
+TableCache& table_cache() {
+  static TableCache* p = new TableCache;  // (not destroyed: the driver may be gone by then)
   return *p;
 }
 DevTable find_table(const TabKey& key) {
-  ModeTables& T = mode_tables();
+  TableCache& T = table_cache();
   std::lock_guard<std::mutex> lk(T.mu);
   auto it = T.all.find(key);
   return it == T.all.end() ? nullptr : it->second.lock();
 }
 // the first one added wins
-DevTable add_table(const TabKey& key, const DevTable& t) {
-  ModeTables& T = mode_tables();
-  DevTable out = t, old;  // (freed after the lock)
+DevTable add_table(const TabKey& key, const DevTable& t, size_t bytes) {
+  TableCache& T = table_cache();
+  std::vector<DevTable> old;  // (freed after the lock)
   std::lock_guard<std::mutex> lk(T.mu);
   for (auto it = T.all.begin(); it != T.all.end();) it = it->second.expired() ? T.all.erase(it) : std::next(it);
   auto it = T.all.find(key);
   if (it != T.all.end())
     if (DevTable first = it->second.lock()) return first;
-  T.all[key] = out;
-  T.kept.push_back(out);
-  if (T.kept.size() > kKeptTables) {
-    old = T.kept.front();
+  T.all[key] = t;
+  T.kept.emplace_back(t, bytes);
+  T.bytes += bytes;
+  while (T.bytes > kKeptBytes) {
+    old.push_back(T.kept.front().first);
+    T.bytes -= T.kept.front().second;
     T.kept.pop_front();
   }
-  return out;
+  return t;
+}
+int new_table(size_t bytes, double** d, DevTable* t) {
+  if (cudaMalloc(d, bytes) != cudaSuccess) {
+    (void)cudaGetLastError();
+    set_error("cudaMalloc of a sine-transform table (%zu bytes) failed", bytes);
+    return ILM_ERR_NO_MEMORY;
+  }
+  *t = dev_table(*d);
+  return ILM_OK;
 }
 
 }  // namespace
@@ -665,22 +687,36 @@ int sine_plan_init(SinePlan* p, int n1, int n2, const void* tw, cudaStream_t st)
   const int nch = chunks(p->MB);
   p->L = (n2 + nch - 1) / nch;
   const size_t ntab = (size_t)(TB_HEAD + 2 * nch) * N;
-  p->tab_own = find_table({N, n2});
+  const TabKey modes(TAB_MODES, N, n2);
+  p->tab_own = find_table(modes);
   if (!p->tab_own) {
+    const size_t bytes = (ntab + 2 * (size_t)N) * sizeof(double);
     double* d = nullptr;
-    if (cudaMalloc(&d, (ntab + 2 * (size_t)N) * sizeof(double)) != cudaSuccess) {
-      set_error("cudaMalloc sine-transform tables failed");
-      return ILM_ERR_NO_MEMORY;
-    }
-    const DevTable t = dev_table(d);
+    DevTable t;
+    ILM_TRY(new_table(bytes, &d, &t));
     k_mode_table<<<(2 * N + 127) / 128, 128, 0, st>>>(N, n2, nch, p->L, d, d + ntab);
     ILM_CHECK_LAUNCH();
     ILM_CHECK_CUDA(cudaStreamSynchronize(st));
-    p->tab_own = add_table({N, n2}, t);
+    p->tab_own = add_table(modes, t, bytes);
   }
   p->tab = p->tab_own.get();
   p->s2 = p->tab + ntab;
-  ILM_TRY(lgf_table_shared(std::max(N, n2 + 1), &p->lgf_own, &p->ldg, st));
+  const int M = std::max(N, n2 + 1);
+  const TabKey lgf(TAB_LGF, M, 0);
+  p->ldg = M + 1;
+  p->lgf_own = find_table(lgf);
+  if (!p->lgf_own) {
+    const size_t bytes = (size_t)(M + 1) * (M + 1) * sizeof(double);
+    double* d = nullptr;
+    DevTable t, G;  // (G stays while it is copied)
+    int ld = 0;
+    ILM_TRY(lgf_table_shared(M, &G, &ld, st));
+    ILM_TRY(new_table(bytes, &d, &t));
+    k_copy_table<<<dim3((M + 1 + 255) / 256, M + 1), 256, 0, st>>>(G.get(), ld, M + 1, d);
+    ILM_CHECK_LAUNCH();
+    ILM_CHECK_CUDA(cudaStreamSynchronize(st));
+    p->lgf_own = add_table(lgf, t, bytes);
+  }
   p->lgf = p->lgf_own.get();
   return p->work.alloc(((size_t)n2 * N + 4 * (size_t)N + 4 * (size_t)n2) * sizeof(double));
 }

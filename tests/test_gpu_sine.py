@@ -81,10 +81,10 @@ def test_inverse_laplacian_rows_of_zeros(cuda, nx, ny, rows):
 
 
 def test_tables_are_given_back(cuda):
-    """Grids of forty heights, one after the other, and the first one again:
+    """Grids of forty heights, one after the other, and the first ones again:
     what stays on the device is bounded (a copy of the lattice Green's function
-    per height was 8 MB here, 320 MB in all), and the results are the same.  At
-    most eight mode tables of 0.1 MB stay; 32 MB leaves room for the allocator."""
+    per height is 8 MB here, 320 MB in all), and the results are the same.  Tables
+    of 64 MB may stay; 32 MB more leaves room for the allocator."""
     def field(ny):
         grid = il.PhysicalGrid.from_cells(64, 0.5, ny=ny)
         c = il.SurfaceScalarCache(None, grid)
@@ -101,4 +101,4 @@ def test_tables_are_given_back(cuda):
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(first, again))
     torch.cuda.empty_cache()
-    assert free - torch.cuda.mem_get_info()[0] <= 32 << 20
+    assert free - torch.cuda.mem_get_info()[0] <= 96 << 20
