@@ -48,14 +48,15 @@ constexpr int C64_T = 256;             // threads per CTA
 constexpr int C64_CLUSTER = 16;        // CTAs of the cluster variant
 // dynamic shared memory beside the static scalars
 constexpr int C64_MAX_CLUSTER = 227 * 1024 - 512, C64_MAX_GRID = 227 * 1024 - 256;
-// matrix entries up to which the cluster variant is used: an iteration of a
+// matrix entries up to which the cluster variant is used without an FP32
+// inverse (no memory for it): an iteration of a
 // dense n takes 4.8 / 5.4 / 6.9 / 8.2 us with the cluster and 5.5 / 5.8 / 6.8 /
 // 6.9 us with the grid at n = 157 / 224 / 300 / 400
 constexpr long long C64_CLUSTER_ENTRIES = 256 * 256;
 // unknowns up to which it is used with an FP32 inverse, whose rows 16 SMs read
-// from L2 (us per solve, cluster and grid): dense n = 157 25 / 33, 300 39.6 /
+// from L2 (us per solve, cluster and grid: dense n = 157 25 / 33, 300 39.6 /
 // 41.2, 400 41.6 / 34.9; 19 entries a row, n = 157 29 / 39, 560 39.1 / 39.8,
-// 696 43.3 / 41.3
+// 696 43.3 / 41.3; both about 1 us more since the last correction is judged)
 constexpr int C64_CLUSTER_DENSE = 320, C64_CLUSTER_CSR = 560;
 constexpr unsigned C64_SPIN = 1u << 22;  // polls of the grid barrier before it gives up (seconds)
 
@@ -981,8 +982,8 @@ int launch_cg64(const CG64Problem& P, void* scratch, cudaStream_t st) {
   size_t smem = plan(P, false, C64_CLUSTER, &A);
   const bool few = P.inv ? n <= (csr ? C64_CLUSTER_CSR : C64_CLUSTER_DENSE) : entries <= C64_CLUSTER_ENTRIES;
   if (few && smem <= (size_t)C64_MAX_CLUSTER && (csr || A.resident)) {
-    ILM_CHECK_CUDA((csr ? kernel_attributes<true, false>() : kernel_attributes<false, false>()));
-    const cudaError_t e = csr ? run_cluster<true>(A, smem, st) : run_cluster<false>(A, smem, st);
+    cudaError_t e = csr ? kernel_attributes<true, false>() : kernel_attributes<false, false>();
+    if (e == cudaSuccess) e = csr ? run_cluster<true>(A, smem, st) : run_cluster<false>(A, smem, st);
     if (!no_room(e)) {
       ILM_CHECK_CUDA(e);
       return ILM_OK;

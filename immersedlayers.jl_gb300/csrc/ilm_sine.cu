@@ -1,5 +1,6 @@
 // FP64 unbounded-domain inverse Laplacian by sine transforms and discrete
-// potential theory: the same linear convolution with the lattice Green's
+// potential theory (R. A. James, The solution of Poisson's equation for isolated
+// source distributions, 1977): the same linear convolution with the lattice Green's
 // function G as the zero-padded FFTs of ilm_fft.cu, in a third of the FP64
 // operations.
 //

@@ -96,7 +96,8 @@ typedef void* ilm_stream_t; /* cudaStream_t */
 typedef struct {
   int iterations;          /* Krylov iterations taken                          */
   int converged;           /* 1 if rel. residual <= tol                        */
-  double rel_residual;     /* ||b - S s||_2 / ||b||_2, evaluated in FP64       */
+  double rel_residual;     /* ||b - S s||_2 / ||b||_2 of the s returned, in FP64
+                            * (NaN, not converged: data that are no numbers)   */
 } ilm_solve_info_t;
 
 /* ---- library ----------------------------------------------------------- */
